@@ -30,6 +30,7 @@ from .. import _lib
 from ..kv.paged import PagedKvCache
 from ..runtime.graph import GraphCache, bucket_for
 from ..ops import decode as D
+from ..ops import narrow
 from .transformer import TransformerModel
 
 
@@ -239,6 +240,14 @@ class CachedDecode(DecodeEngineBase):
             self.wts = torch.zeros(B, k, dtype=torch.float32, device=dev)
             self.act = torch.zeros(B * k, i_local, **bf)
             self.router_scratch = D.RouterScratch(B, moe.num_experts, dev)
+            # several rows on one GPU: every chosen expert's weights are read once for all rows (ops/narrow.py)
+            self.expert_scratch = None
+            routed = [l for l in model.w.layers if l.experts_gate_up is not None]
+            if B > 1 and model.layout.world == 1 and all(
+                    narrow.supported(l.experts_gate_up) and narrow.supported(l.experts_down) and
+                    l.experts_gate_up.n % 32 == 0 and l.experts_gate_up.experts == moe.num_experts for l in routed):
+                l = max(routed, key=lambda l: l.experts_gate_up.n)
+                self.expert_scratch = narrow.ExpertScratch(B, k, l.experts_gate_up, l.experts_down)
         dense_i = [l.w_gate_up.n // 2 for l in model.w.layers if l.w_gate_up is not None]
         if dense_i:
             self.dense_act = torch.zeros(B, max(dense_i), **bf)
@@ -281,7 +290,7 @@ class CachedDecode(DecodeEngineBase):
         h, h2 = self.h[:nb], self.h2[:nb]
         # several rows on 4-bit weights: the projection runs on the tensor-core mat-vec (eight rows
         # per pass) and RoPE + the KV append follow as their own small kernel
-        fuse_rope = self.fuse_rope and not (nb >= 2 and w.layers[0].wqkv.kind == 1)
+        fuse_rope = self.fuse_rope and not (nb >= 2 and (w.layers[0].wqkv.kind == 1 or D._several(nb, w.layers[0].wqkv, h)))
         for li, lw in enumerate(w.layers):
             if fuse_rope:
                 D.rms_qkv_rope(h, lw.wqkv, lw.norm1, eps, q, self.cache.k[li], self.cache.v[li],
@@ -306,6 +315,11 @@ class CachedDecode(DecodeEngineBase):
                 idx, wts, act = self.idx[:nb], self.wts[:nb], self.act[:nb * k]
                 D.moe_router(h2, lw.router, lw.norm2, eps, k, lw.expert_bias,
                              self.router_scratch, idx, wts, pdl=pdl)
+                if self.expert_scratch is not None and narrow.pays_shared(lw.experts_gate_up, nb, k) and \
+                        D._several(nb, lw.experts_gate_up, h2):
+                    narrow.expert_ffn(h2, idx, wts, lw.experts_gate_up, lw.experts_down, lw.norm2, eps, residual=h2,
+                                      out=h, scratch=self.expert_scratch, pdl=pdl)
+                    continue
                 D.moe_gate_up(h2, lw.experts_gate_up, lw.norm2, eps, idx, out=act,
                               expert_base=lw.expert_base, pdl=pdl)
                 if tp:

@@ -23,6 +23,7 @@ import torch
 from .. import _lib
 from ..kv.paged import PagedKvCache
 from ..ops import decode as D
+from ..ops import narrow
 from ..runtime.graph import GraphCache, bucket_for
 from ..ops.attention import flash_prefill_paged
 from ..ops.gemm import GemmStatus, gemm_bf16
@@ -31,8 +32,15 @@ from ..ops.quantized import qmm, xgemm
 from ..ops.weights import LinearWeight, W_BF16, W_Q4
 
 
+def _narrow(x: torch.Tensor, w: LinearWeight) -> bool:
+    """Whether these few rows go through the weight-streaming kernel (``ops/narrow.py``)."""
+    return x.shape[0] <= 64 and narrow.pays(w, x.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+
+
 def _mm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     if w.kind == W_BF16:
+        if _narrow(x, w):
+            return narrow.narrow_gemm(x, w, residual=residual)
         return gemm_bf16(x, w.w, residual=residual)
     return qmm(x, w, residual=residual)
 
@@ -40,6 +48,8 @@ def _mm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = Non
 def _gate_up_act(x: torch.Tensor, w: LinearWeight) -> torch.Tensor:
     """silu(x W_gate^T) * (x W_up^T) for W = [gate; up]: SwiGLU runs in the GEMM epilogue when the
     shape allows, else GEMM then the element-wise kernel."""
+    if w.n % 32 == 0 and _narrow(x, w):
+        return narrow.narrow_gemm(x, w, swiglu=True)
     q4_ok = w.kind == W_BF16 or (w.kind == W_Q4 and not w.scales_f16 and
                                  bool(_lib.cuda().rmlx_qgemm_supported(w.k)))
     if w.n % 256 == 0 and w.k % 8 == 0 and q4_ok:
@@ -112,7 +122,7 @@ class _Layers:
         m = self.m
         cfg, w = m.cfg, m.w
         r = rows.shape[0]
-        if r <= 4:
+        if r <= 4 or narrow.pays(w.lm_head, r):
             out = D.rms_gemv(rows.contiguous(), w.lm_head, w.final_norm, cfg.rms_norm_eps,
                              out=torch.empty(r, w.lm_head.n, dtype=torch.float32, device=m.device))
         else:

@@ -1,0 +1,138 @@
+"""Projections of a few rows on csrc/kernels/narrow_gemm.cu: decode batches, short prompts and verification. The weights
+(bf16, 4-bit or 8-bit) are streamed once through registers, eight rows of x per tensor-core instruction; the grouped form
+takes (row, slot) pairs by expert. Counterpart of the reference's small-M qmm / gather_qmm kernels
+(crates/rmlx-core/src/ops/quantized.rs:2755,9634)."""
+from __future__ import annotations
+
+from typing import Optional
+
+import torch
+
+from .. import _lib
+from .weights import LinearWeight, W_BF16, W_Q4, W_Q8
+
+_lib.register_cuda_sigs({
+    "rmlx_narrow_supported": ("iii", "i"),
+    "rmlx_narrow_gemm": ("ippppiippipfpipiiiiiiiiip", "i"),
+    "rmlx_narrow_group": ("piippip", "i"),
+    "rmlx_narrow_combine": ("pppipiiiiip", "i"),
+})
+
+
+def supported(w: LinearWeight) -> bool:
+    """Whether the kernel takes this weight: bf16 scales, whole 16-row tiles, K a multiple of
+    512 (bf16 weights: 64), up to 256 experts."""
+    return not w.scales_f16 and max(1, w.experts) <= 256 and bool(_lib.cuda().rmlx_narrow_supported(w.kind, w.n, w.k))
+
+
+def pays(w: LinearWeight, rows: int) -> bool:
+    """Whether a plain projection of ``rows`` rows is faster here than on the 128-row tensor-core tiles (and takes this weight).
+
+    Measured (us, this kernel / the tiles). 4-bit, 9216 x 4096: 16 / 32 at 16 rows, 30 / 32 at 32, 40 / 32 at 64; 28672 x 4096:
+    31 / 73, 55 / 73, 106 / 74; 4096 x 14336: 34 / 96, 83 / 96, 90 / 96: up to 32 rows, and up to 64 where a few rows of W leave
+    the tiles less than half of the SMs. 8-bit weights would be expanded first (53 us for 28672 x 4096). bf16, 9216 x 4096:
+    20 / 28 at 16 rows; 28672 x 4096: 46 / 45: eight rows, and 16 for up to 16384 rows of W. Weights of less than a million
+    entries take a tile's time anyway."""
+    if rows < 1 or rows > 64 or w.n * w.k < 1 << 20:
+        return False
+    if w.kind == W_BF16:
+        ok = rows <= 8 or (rows <= 16 and w.n <= 16384)
+    elif w.kind == W_Q4:
+        ok = rows <= 32 or w.n <= 4096
+    else:
+        ok = rows <= 16 or (rows <= 32 and w.n >= 8192)
+    return ok and supported(w)
+
+
+def pays_grouped(gate_up: LinearWeight, down: LinearWeight, pairs: int) -> bool:
+    """Whether an expert feed-forward of ``pairs`` (row, slot) pairs is faster here: up to eight pairs per expert (128 experts
+    of 4096 x 1536, us: 4-bit 378 against 1046 on the tiles at 512 pairs, 492 against 778 at 1024; 8-bit 551 against 799 on
+    expanded weights, 627 against 766). bf16 experts are as fast on the tiles (523 + 275 against 549 + 305 at 512 pairs)."""
+    return (gate_up.kind in (W_Q4, W_Q8) and down.kind == gate_up.kind and 0 < pairs <= 8 * gate_up.experts and
+            gate_up.n * gate_up.k >= 1 << 20 and supported(gate_up) and supported(down))
+
+
+def narrow_gemm(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6,
+                residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, out_dtype=torch.bfloat16,
+                swiglu: bool = False, offsets: Optional[torch.Tensor] = None, order: Optional[torch.Tensor] = None,
+                x_div: int = 1, rows: Optional[int] = None, tiles: int = 0, shares: int = 0, pdl: bool = False) -> torch.Tensor:
+    """out = residual + rmsnorm(x; norm_w) W^T, or silu(gate) * up of a stacked [gate; up] weight with ``swiglu``.
+
+    Grouped: w is [E, N, K], ``offsets`` int32 [E + 1] the positions of every expert's rows, ``order`` the output row of each
+    position (None: the position itself), whose input is row ``output row // x_div`` of x; ``rows``: positions in all.
+    ``tiles`` (eight rows of x each per pass: 1, 2, 4) and ``shares`` (of K) are chosen from the sizes when 0."""
+    _lib.require_cuda_tensor(x, w.w)
+    assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] == w.k
+    m = x.shape[0] if rows is None else rows
+    n = w.n // 2 if swiglu else w.n
+    if out is None:
+        out = torch.empty(m, n, dtype=out_dtype, device=x.device)
+    rc = _lib.cuda().rmlx_narrow_gemm(
+        w.kind, w.w.data_ptr(), _lib.ptr(w.scales), _lib.ptr(w.biases), x.data_ptr(), x.stride(0), x_div, _lib.ptr(order),
+        _lib.ptr(offsets), 1 if offsets is None else w.experts, _lib.ptr(norm_w), eps, _lib.ptr(residual),
+        0 if residual is None else residual.stride(0), out.data_ptr(), out.stride(0), int(out.dtype == torch.float32), m, w.n, w.k,
+        int(swiglu), tiles, shares, int(pdl), _lib.stream_ptr())
+    _lib.check(rc, "narrow_gemm")
+    return out
+
+
+def group_pairs(idx: torch.Tensor, experts: int, offsets: Optional[torch.Tensor] = None, order: Optional[torch.Tensor] = None,
+                pdl: bool = False):
+    """Pairs (row * k + slot) by chosen expert: (offsets [E + 1], order [rows * k]), int32."""
+    n = idx.numel()
+    if offsets is None:
+        offsets = torch.empty(experts + 1, dtype=torch.int32, device=idx.device)
+    if order is None:
+        order = torch.empty(n, dtype=torch.int32, device=idx.device)
+    _lib.check(_lib.cuda().rmlx_narrow_group(idx.data_ptr(), n, experts, offsets.data_ptr(), order.data_ptr(), int(pdl),
+                                             _lib.stream_ptr()), "narrow_group")
+    return offsets, order
+
+
+def combine(y: torch.Tensor, wts: torch.Tensor, residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+            pdl: bool = False) -> torch.Tensor:
+    """out[t] = residual[t] + sum over slots of wts[t, slot] * y[t k + slot], y fp32."""
+    t, k = wts.shape
+    d = y.shape[1]
+    if out is None:
+        out = torch.empty(t, d, dtype=torch.bfloat16, device=y.device)
+    _lib.check(_lib.cuda().rmlx_narrow_combine(y.data_ptr(), wts.data_ptr(), _lib.ptr(residual),
+                                               0 if residual is None else residual.stride(0), out.data_ptr(), out.stride(0), t, k,
+                                               d, int(pdl), _lib.stream_ptr()), "narrow_combine")
+    return out
+
+
+def pays_shared(gate_up: LinearWeight, rows: int, top_k: int) -> bool:
+    """Whether a decode step of ``rows`` rows should read every chosen expert once for all rows (four launches) rather than once
+    per (row, slot) pair on the streaming kernels (two). Measured on whole two-layer steps (us, here / there), 128 experts of
+    4096 x 1536 and 32 of 2048 x 2048: 4-bit 371 / 386 at 2 rows of the larger, 251 / 243 at 5 of the smaller and 277 / 313 at 8;
+    8-bit 470 / 544 and 183 / 182 at 2; bf16 691 / 582 at 2 rows of the larger, 732 / 731 at 3, 877 / 930 at 4: there only the
+    sharing itself helps, as pairs already stream at the copy bandwidth."""
+    if gate_up.kind == W_BF16:
+        return rows >= 4
+    return rows >= 2 and rows * top_k * gate_up.n * gate_up.k >= (200e6 if gate_up.kind == W_Q4 else 60e6)
+
+
+class ExpertScratch:
+    """Buffers of ``expert_ffn`` for up to ``rows`` rows, for callers whose launches may not allocate."""
+
+    def __init__(self, rows: int, top_k: int, gate_up: LinearWeight, down: LinearWeight):
+        dev, pairs = gate_up.device, rows * top_k
+        self.offsets = torch.empty(gate_up.experts + 1, dtype=torch.int32, device=dev)
+        self.order = torch.empty(pairs, dtype=torch.int32, device=dev)
+        self.act = torch.empty(pairs, gate_up.n // 2, dtype=torch.bfloat16, device=dev)
+        self.y = torch.empty(pairs, down.n, dtype=torch.float32, device=dev)
+
+
+def expert_ffn(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, gate_up: LinearWeight, down: LinearWeight,
+               norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6, residual: Optional[torch.Tensor] = None,
+               out: Optional[torch.Tensor] = None, scratch: Optional[ExpertScratch] = None, pdl: bool = False) -> torch.Tensor:
+    """residual + sum over slots of wts * down_e(silu(gate_e xn) * up_e xn), e = idx[row, slot], xn = rmsnorm(x; norm_w):
+    every expert's weights are read once for all rows that chose it."""
+    t, k = idx.shape
+    pairs = t * k
+    s = scratch or ExpertScratch(t, k, gate_up, down)
+    offsets, order = group_pairs(idx, gate_up.experts, s.offsets, s.order[:pairs], pdl=pdl)
+    act = narrow_gemm(x, gate_up, norm_w, eps, out=s.act[:pairs], swiglu=True, offsets=offsets, order=order, x_div=k, rows=pairs, pdl=pdl)
+    y = narrow_gemm(act, down, out=s.y[:pairs], offsets=offsets, order=order, rows=pairs, pdl=pdl)
+    return combine(y, wts, residual, out, pdl=pdl)

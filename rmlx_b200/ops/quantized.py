@@ -11,6 +11,7 @@ from typing import Optional
 import torch
 
 from .. import _lib
+from . import narrow
 from .gemm import GemmStatus, gemm_bf16
 from .weights import LinearWeight, W_Q4
 
@@ -50,11 +51,13 @@ def xgemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = N
 
 def qmm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = None,
         out: Optional[torch.Tensor] = None, pdl: bool = False) -> torch.Tensor:
-    """x @ W^T for affine-quantised W: 4-bit weights are expanded inside the tensor-core GEMM's main
+    """x @ W^T for affine-quantised W: a few rows go through the weight-streaming kernel (``ops/narrow.py``); otherwise 4-bit weights are expanded inside the tensor-core GEMM's main
     loop; 8-bit weights, weights with fp16 scales and 4-bit shapes the fused kernel does not take are
     expanded to bf16 by the
     dequantisation kernel first and go through the bf16 tensor-core GEMM."""
     assert w.kind != 0
+    if x.shape[0] <= 64 and narrow.pays(w, x.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+        return narrow.narrow_gemm(x, w, residual=residual, out=out, pdl=pdl)
     if w.kind == W_Q4 and not w.scales_f16 and _lib.cuda().rmlx_qgemm_supported(w.k):
         return xgemm(x, w, residual, out, pdl=pdl)
     return gemm_bf16(x, w.dense_bf16(), residual=residual, out=out, pdl=pdl)

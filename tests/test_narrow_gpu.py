@@ -1,0 +1,117 @@
+"""Projections of a few rows (csrc/kernels/narrow_gemm.cu) against 64-bit products of the same weights.
+
+Tolerances. fp32 results: codes and bf16 inputs enter the products exactly, so what is left is the fp32 summation, 2e-5 of the
+result's norm. With a norm, 4-bit and 8-bit kernels round x times its weight to fp16 (2^-12 relative, independent per term):
+3e-4; bf16 ones keep it in two terms. bf16 results add 2^-9."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    return torch.device("cuda")
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+def _case(dev, kind, n, k, rows, experts=0, seed=0):
+    from rmlx_b200.ops.weights import LinearWeight
+    g = torch.Generator(device=dev).manual_seed(seed)
+    w = LinearWeight.random(n, k, kind, dev, experts=experts, generator=g)
+    return w, w.dequantized().double(), torch.randn(rows, k, device=dev, generator=g).to(torch.bfloat16), g
+
+
+# one slab and several (K), one row tile and ragged runs of them (N), every tile count of rows and its edges
+@pytest.mark.parametrize("kind", ["q4", "q8", None])
+@pytest.mark.parametrize("n,k", [(16, 512), (48, 1024), (1056, 2560), (544, 4608), (64, 14336)])
+@pytest.mark.parametrize("rows", [1, 8, 9, 17, 33, 64])
+def test_plain(dev, kind, n, k, rows):
+    from rmlx_b200.ops import narrow
+    w, wd, x, g = _case(dev, kind, n, k, rows)
+    assert narrow.supported(w)
+    want = x.double() @ wd.t()
+    for shares in (0, 1, 2, 4, 8):
+        assert _rel(narrow.narrow_gemm(x, w, out_dtype=torch.float32, shares=shares), want) < 2e-5
+    res = torch.randn(rows, n, device=dev, generator=g).to(torch.bfloat16)
+    assert _rel(narrow.narrow_gemm(x, w, residual=res), want + res.double()) < 4e-3
+
+
+@pytest.mark.parametrize("kind", ["q4", "q8", None])
+@pytest.mark.parametrize("k", [512, 4096, 8192])
+@pytest.mark.parametrize("rows", [1, 5, 8, 16])
+def test_norm_and_swiglu(dev, kind, k, rows):
+    from rmlx_b200.ops import narrow
+    w, wd, x, g = _case(dev, kind, 96, k, rows, seed=1)
+    nw = torch.rand(k, device=dev, generator=g).to(torch.bfloat16) + 0.5
+    xd = x.double()
+    up = (xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double()) @ wd.t()
+    assert _rel(narrow.narrow_gemm(x, w, nw, 1e-6, out_dtype=torch.float32), up) < (3e-4 if kind else 2e-5)
+    want = torch.nn.functional.silu(up[:, :48]) * up[:, 48:]
+    # a relative error e of gate and up is at most about 3 e of the activation at these sizes
+    assert _rel(narrow.narrow_gemm(x, w, nw, 1e-6, out_dtype=torch.float32, swiglu=True), want) < (1e-3 if kind else 6e-5)
+
+
+@pytest.mark.parametrize("kind", ["q4", "q8", None])
+@pytest.mark.parametrize("rows", [1, 3, 40])
+def test_expert_feed_forward(dev, kind, rows):
+    """Experts without rows, with one, and with more rows than a pass holds (every row of the largest batch chooses expert 3)."""
+    from rmlx_b200.ops import narrow
+    e, d, inner, k = 12, 1024, 512, 4
+    gu, gud, x, g = _case(dev, kind, 2 * inner, d, rows, experts=e, seed=2)
+    dn, dnd, _, _ = _case(dev, kind, d, inner, 1, experts=e, seed=3)
+    idx = torch.stack([torch.randperm(e - 1, device=dev, generator=g)[:k] for _ in range(rows)]).to(torch.int32)
+    if rows == 40:
+        idx[:, 1] = torch.where((idx == 3).any(1), idx[:, 1], torch.full_like(idx[:, 1], 3))
+    wts = torch.rand(rows, k, device=dev, generator=g)
+    res = torch.randn(rows, d, device=dev, generator=g).to(torch.bfloat16)
+    up = torch.einsum("tsnk,tk->tsn", gud[idx.long()], x.double())
+    act = torch.nn.functional.silu(up[..., :inner]) * up[..., inner:]
+    y = torch.einsum("tsnk,tsk->tsn", dnd[idx.long()], act)
+    want = res.double() + (y * wts.double()[..., None]).sum(1)
+    # the activation is rounded to bf16 (2^-9) in between, the result at the end
+    assert _rel(narrow.expert_ffn(x, idx, wts, gu, dn, residual=res), want) < 8e-3
+    offsets, order = narrow.group_pairs(idx, e)
+    assert torch.equal(torch.sort(order).values, torch.arange(rows * k, device=dev, dtype=torch.int32))
+    flat = idx.flatten()[order.long()]
+    counts = torch.bincount(flat.long(), minlength=e)
+    assert torch.equal(offsets[1:].long(), counts.cumsum(0)) and bool((flat[1:] >= flat[:-1]).all())
+    for tiles in (0, 1, 2, 4):
+        got = narrow.narrow_gemm(x, gu, offsets=offsets, order=order, x_div=k, rows=rows * k, out_dtype=torch.float32, tiles=tiles)
+        assert _rel(got, up.view(rows * k, -1)) < 2e-5
+
+
+@pytest.mark.parametrize("kind", ["q4", "q8"])
+def test_extreme_inputs(dev, kind):
+    """Zero groups, the smallest and largest magnitudes the activations' scaling covers, one huge value beside small ones, and
+    an infinity, which stays in its own row."""
+    from rmlx_b200.ops import narrow
+    w, wd, x, _ = _case(dev, kind, 64, 512, 6, seed=4)
+    x[0, :] = 0
+    x[1, 64:128] = 0
+    x[2] *= 2.0 ** -70
+    x[3] *= 2.0 ** 80
+    x[4, 7] = 2.0 ** 20
+    want = x.double() @ wd.t()
+    x[5, 3] = float("inf")
+    got = narrow.narrow_gemm(x, w, out_dtype=torch.float32)
+    assert float(got[0].abs().max()) == 0.0
+    for r in range(1, 5):
+        assert _rel(got[r], want[r]) < 2e-5
+    assert not torch.isfinite(got[5]).any()
+
+
+def test_refusals(dev):
+    from rmlx_b200 import _lib
+    from rmlx_b200.ops import narrow
+    from rmlx_b200.ops.weights import LinearWeight
+    for n, k in ((24, 512), (64, 320)):
+        w = LinearWeight.random(n, k, "q4", dev)
+        assert not narrow.supported(w)
+        with pytest.raises(_lib.NativeError):
+            narrow.narrow_gemm(torch.zeros(2, k, dtype=torch.bfloat16, device=dev), w)
