@@ -32,7 +32,7 @@ constexpr int kXMaxExperts = 256;
 constexpr int kXMaxRanks = 8;
 constexpr int kCommNone = 0, kCommReduce = 1, kCommGather = 2;
 constexpr int kGatherChunkRows = 8;
-constexpr int kDqWarps = 8;          // dequant warps of the Q4 main loop (two per SM sub-partition)
+constexpr int kDqWarps = 8;          // dequant warps of one group of the Q4 main loop (two per SM sub-partition)
 constexpr int kCommThreads = 160;   // collective modes: four reducer/pusher warps + one signalling warp
 
 struct XComm {
@@ -53,20 +53,32 @@ struct XComm {
   unsigned long long* trace = nullptr;       // optional [grid][8] timestamps (see x_trace)
 };
 
+// Single-GPU Q4 form: a warp of its own asks for the packed weights, as far ahead as their ring is deep (behind the rows of A
+// it was five 4 KB stages, too little under way to stream the experts of a decode batch), and two groups of dequant warps take
+// the k-blocks in turn, so that one expands while the other waits for its block, its slot or its stores. The collective modes
+// keep the narrower block (their five warps need the registers).
+template <bool WQ4, int COMM>
+struct XRoles {
+  static constexpr bool kDeep = WQ4 && COMM == kCommNone;
+  static constexpr int kGroups = kDeep ? 2 : 1;
+  static constexpr int kRawWarp = 6 + kDqWarps * kGroups;            // kDeep only
+  static constexpr int kThreads = 192 + (WQ4 ? 32 * kDqWarps * kGroups : 0) + (kDeep ? 32 : 0) + (COMM != kCommNone ? kCommThreads : 0);
+};
+
 // MT = 2: a tile is two stacked 128-row blocks of A against ONE staged block of W, i.e. two
 // accumulators per dequantised operand stage — the dequant warps' work per multiply-add halves.
-template <int BN, bool WQ4, int MT = 1>
+template <int BN, bool WQ4, int MT = 1, bool DEEP = false>
 struct XSmem {
   static constexpr int kStages = MT == 2 ? 3 : (WQ4 ? ((BN >= 256) ? 3 : 5) : ((BN >= 256) ? 4 : 6));
-  static constexpr int kRawStages = 4;
+  static constexpr int kRawStages = !DEEP ? 4 : BN >= 256 ? 7 : BN == 128 ? 12 : 16;
   static constexpr int kStageA = MT * kXBM * kXBK * 2;
   static constexpr int kStageB = BN * kXBK * 2;
   static constexpr int kStageRaw = BN * 32;          // 64 nibbles per row
   static constexpr int kScaleSlot = 2 * BN * 16;     // scales + biases for 8 k-blocks
+  static constexpr int kBarBytes = 768;              // 3 kStages + 2 kRawStages + 13 barriers of 8 bytes, three words
   static constexpr int kBytes = kStages * (kStageA + kStageB) +
-                                (WQ4 ? kRawStages * kStageRaw + 2 * kScaleSlot : 0) + 1024 + 512 +
+                                (WQ4 ? kRawStages * kStageRaw + 2 * kScaleSlot : 0) + 1024 + kBarBytes +
                                 (kXMaxExperts + 2) * 8;
-  static constexpr int kThreads = WQ4 ? 192 + 32 * kDqWarps : 192;
 };
 
 struct XTile {
@@ -185,7 +197,7 @@ __device__ __forceinline__ void x_reduce_tile(const XComm& cm, const __nv_bfloat
 }
 
 template <int BN, bool WQ4, bool GROUPED, bool RESIDUAL, int COMM, int MT>
-__global__ void __launch_bounds__((XSmem<BN, WQ4>::kThreads + (COMM != kCommNone ? kCommThreads : 0)), 1)
+__global__ void __launch_bounds__((XRoles<WQ4, COMM>::kThreads), 1)
 xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a2,
              const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
              const __grid_constant__ CUtensorMap tmap_b, __nv_bfloat16* __restrict__ C,
@@ -193,11 +205,12 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
              int N, int K, int ldc, int* __restrict__ status, const XComm cm, int swiglu, float gate_limit) {
   static_assert(COMM == kCommNone || !GROUPED, "collective modes are for plain GEMMs");
   static_assert(MT == 1 || (COMM == kCommNone && 2 * BN * MT <= 512), "stacked tiles: no collective modes");
-  using S = XSmem<BN, WQ4, MT>;
+  using Ro = XRoles<WQ4, COMM>;
+  using S = XSmem<BN, WQ4, MT, Ro::kDeep>;
   constexpr int STAGES = S::kStages, RAW = S::kRawStages;
   // a role may be waiting, through the pipeline, on a peer that started late: be more patient then
   constexpr uint32_t LIM = (COMM == kCommNone) ? kMbarPollLimit : (kMbarPollLimit << 4);
-  constexpr int kCommWarp0 = S::kThreads / 32;          // first of the five collective-mode warps
+  constexpr int kCommWarp0 = 6 + (WQ4 ? kDqWarps : 0);   // first of the five collective-mode warps
   constexpr uint32_t TMEM_COLS = (2 * BN * MT <= 32) ? 32 : 2 * BN * MT;
   extern __shared__ char smem_raw[];
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -222,7 +235,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(comm_mb + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* peer_fail = tmem_slot + 2;
-  int* s_off = reinterpret_cast<int*>(after + 512);          // [E+1]
+  int* s_off = reinterpret_cast<int*>(after + S::kBarBytes);          // [E+1]
   int* s_tprefix = s_off + kXMaxExperts + 1;                 // [E+1]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -234,7 +247,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     for (int i = 0; i < STAGES; ++i) { mbar_init(full + i, 1); mbar_init(empty + i, 1); mbar_init(bq_full + i, kDqWarps); }
     for (int i = 0; i < RAW; ++i) { mbar_init(raw_full + i, 1); mbar_init(raw_empty + i, kDqWarps); }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(sc_full + i, 1); mbar_init(sc_empty + i, kDqWarps);
+      mbar_init(sc_full + i, 1); mbar_init(sc_empty + i, kDqWarps * Ro::kGroups);
       mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 4);
     }
     for (int i = 0; i < 2; ++i) { mbar_init(sig_full + i, 128); mbar_init(sig_free + i, 1); }
@@ -295,7 +308,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           }
         }
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (WQ4) {
+          if (WQ4 && !Ro::kDeep) {
             if ((kb & 7) == 0) {
               if (!mbar_wait(sc_empty + sslot, sphase ^ 1u, abort_flag, LIM)) { ok = false; break; }
               mbar_arrive_expect_tx(sc_full + sslot, S::kScaleSlot);
@@ -578,10 +591,43 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         }
       }
     }
-  } else if (WQ4 && warp < 6 + kDqWarps) {
-    // ------------------------------------------------------------------ dequant (warps 6..13)
-    const int dt = threadIdx.x - 192;   // 0 .. 32*kDqWarps-1
-    int stage = 0, rstage = 0, sslot = 0;
+  } else if (Ro::kDeep && warp == Ro::kRawWarp) {
+    // ------------------------------------------------------------------ packed weights, scales and biases
+    // Weights are no other kernel's result: asked for before the wait on the previous one (grouped: its offsets were needed).
+    if (elect_one()) {
+      tma_prefetch_desc(&tmap_w);
+      int rstage = 0, sslot = 0;
+      uint32_t rphase = 0, sphase = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        const XTile t = x_tile<BN, GROUPED, COMM == kCommGather, MT>(tile, M, N, tiles_m, tiles_n, s_off, s_tprefix, E, rot, swiglu);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if ((kb & 7) == 0) {
+            if (!mbar_wait(sc_empty + sslot, sphase ^ 1u, abort_flag, LIM)) { ok = false; break; }
+            mbar_arrive_expect_tx(sc_full + sslot, S::kScaleSlot);
+            char* sd = sScale + sslot * S::kScaleSlot;
+            tma_load_2d(sd, &tmap_s, sc_full + sslot, kb, t.w_row0);
+            tma_load_2d(sd + BN * 16, &tmap_b, sc_full + sslot, kb, t.w_row0);
+            if (swiglu) {
+              tma_load_2d(sd + BN * 8, &tmap_s, sc_full + sslot, kb, t.w_row0 + N / 2);
+              tma_load_2d(sd + BN * 16 + BN * 8, &tmap_b, sc_full + sslot, kb, t.w_row0 + N / 2);
+            }
+            if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
+          }
+          if (!mbar_wait(raw_empty + rstage, rphase ^ 1u, abort_flag, LIM)) { ok = false; break; }
+          mbar_arrive_expect_tx(raw_full + rstage, S::kStageRaw);
+          tma_load_2d(sRaw + rstage * S::kStageRaw, &tmap_w, raw_full + rstage, kb * 32, t.w_row0);
+          if (swiglu)
+            tma_load_2d(sRaw + rstage * S::kStageRaw + BN * 16, &tmap_w, raw_full + rstage, kb * 32, t.w_row0 + N / 2);
+          if (++rstage == RAW) { rstage = 0; rphase ^= 1u; }
+        }
+      }
+    }
+  } else if (WQ4 && warp < 6 + kDqWarps * Ro::kGroups) {
+    // ------------------------------------------------------------------ dequant (from warp 6)
+    const int dt = (threadIdx.x - 192) % (32 * kDqWarps);          // 0 .. 32*kDqWarps-1 within the group
+    const int group = (threadIdx.x - 192) / (32 * kDqWarps);       // takes k-blocks group, group + kGroups, ..
+    int stage = group, rstage = group, sslot = 0;
     uint32_t phase = 0, rphase = 0, sphase = 0;
     bool ok = true;
     // Static work split: item = (row of the W tile, which 32-element half of the 64-wide k-block);
@@ -589,6 +635,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // and a row's 8 group scales/biases stay in registers for 8 k-blocks.
     constexpr int ITEMS = (BN * 2 + 32 * kDqWarps - 1) / (32 * kDqWarps);
     const __nv_bfloat162 k128 = __float2bfloat162_rn(128.f);
+    const uint32_t half_sel = group ? 0x3232u : 0x1010u;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       for (int kb8 = 0; kb8 < num_kb && ok; kb8 += 8) {     // K % 512 == 0: whole groups of 8
         if (!mbar_wait(sc_full + sslot, sphase, abort_flag, LIM)) { ok = false; break; }
@@ -606,7 +653,8 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         if (lane == 0) mbar_arrive(sc_empty + sslot);       // the slot can be refilled already
         if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
+        for (int k2 = 0; k2 < 8 / Ro::kGroups; ++k2) {
+          const int kk = k2 * Ro::kGroups + group;
           if (!mbar_wait(raw_full + rstage, rphase, abort_flag, LIM)) { ok = false; break; }
           if (!mbar_wait(empty + stage, phase ^ 1u, abort_flag, LIM)) { ok = false; break; }  // B slot free
           const char* raw = sRaw + rstage * S::kStageRaw;
@@ -617,10 +665,11 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             if (item < BN * 2) {
               const int r = item >> 1, h = item & 1;
               const uint4 wv = *reinterpret_cast<const uint4*>(raw + item * 16);
-              const uint32_t sw = (kk >> 1) == 0 ? sv[it].x : (kk >> 1) == 1 ? sv[it].y : (kk >> 1) == 2 ? sv[it].z : sv[it].w;
-              const uint32_t bw = (kk >> 1) == 0 ? bv[it].x : (kk >> 1) == 1 ? bv[it].y : (kk >> 1) == 2 ? bv[it].z : bv[it].w;
-              const uint32_t s2u = __byte_perm(sw, 0u, (kk & 1) ? 0x3232u : 0x1010u);
-              const uint32_t b2u = __byte_perm(bw, 0u, (kk & 1) ? 0x3232u : 0x1010u);
+              // two groups: word k2 of the row's scales, the group's half of it
+              const uint32_t sws[4] = {sv[it].x, sv[it].y, sv[it].z, sv[it].w}, bws[4] = {bv[it].x, bv[it].y, bv[it].z, bv[it].w};
+              const int wi = Ro::kGroups == 2 ? k2 : k2 >> 1;
+              const uint32_t odd = Ro::kGroups == 2 ? half_sel : (k2 & 1) ? 0x3232u : 0x1010u;
+              const uint32_t s2u = __byte_perm(sws[wi], 0u, odd), b2u = __byte_perm(bws[wi], 0u, odd);
               const __nv_bfloat162 s2 = *reinterpret_cast<const __nv_bfloat162*>(&s2u);
               const __nv_bfloat162 b2 = *reinterpret_cast<const __nv_bfloat162*>(&b2u);
               const uint32_t words[4] = {wv.x, wv.y, wv.z, wv.w};
@@ -652,8 +701,10 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             mbar_arrive(bq_full + stage);
             mbar_arrive(raw_empty + rstage);
           }
-          if (++rstage == RAW) { rstage = 0; rphase ^= 1u; }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          rstage += Ro::kGroups;
+          if (rstage >= RAW) { rstage -= RAW; rphase ^= 1u; }
+          stage += Ro::kGroups;
+          if (stage >= STAGES) { stage -= STAGES; phase ^= 1u; }
         }
       }
     }
@@ -679,13 +730,15 @@ static int launch_x(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtenso
                     const CUtensorMap& ts, const CUtensorMap& tb, void* C, const void* residual,
                     const int* offsets, int E, int M, int N, int K, int ldc, int* status, int pdl,
                     cudaStream_t st, const XComm& cm = XComm(), int swiglu = 0, float gate_limit = 0.f) {
-  using S = XSmem<BN, WQ4, MT>;
+  using Ro = XRoles<WQ4, COMM>;
+  using S = XSmem<BN, WQ4, MT, Ro::kDeep>;
+  static_assert(S::kBytes <= 227 * 1024, "shared memory");
   auto kern = xgemm_kernel<BN, WQ4, GROUPED, RESIDUAL, COMM, MT>;
   RB_CHECK(set_max_smem(kern, S::kBytes));
   int tiles = ((M + kXBM * MT - 1) / (kXBM * MT)) * ((N + BN - 1) / BN);
   if (GROUPED) tiles += E * ((N + BN - 1) / BN);   // upper bound: every group may add a ragged tile
   const int grid = tiles < sm_count() ? (tiles > 0 ? tiles : 1) : sm_count();
-  return launch(kern, dim3(grid), dim3(S::kThreads + (COMM != kCommNone ? kCommThreads : 0)), size_t(S::kBytes), st, pdl != 0, ta, ta2, tw, ts, tb,
+  return launch(kern, dim3(grid), dim3(Ro::kThreads), size_t(S::kBytes), st, pdl != 0, ta, ta2, tw, ts, tb,
                 static_cast<__nv_bfloat16*>(C), static_cast<const __nv_bfloat16*>(residual), offsets, E,
                 M, N, K, ldc, status, cm, swiglu, gate_limit);
 }

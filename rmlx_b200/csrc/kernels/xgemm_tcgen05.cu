@@ -45,15 +45,17 @@ extern "C" int rmlx_xgemm(int w_kind, const void* A, const void* W, const void* 
   if (bn < 0) { mt = 2; bn = -bn; }
   if (mt == 2 && (bn != 128 || (grouped && residual))) return -2;
   if (bn == 0) {
-    bn = (grouped || w_kind == 1) ? ((N % 256 == 0 && M >= 1024) ? 256 : 128) : 128;
-    // Q4, many rows: the dequant warps are the limit, so share each dequantised block of W
-    // between two row blocks
-    if (w_kind == 1 && !grouped && ((M + 255) / 256) * ((N + 127) / 128) >= 120) { bn = 128; mt = 2; }
-    // grouped: experts with more than 128 rows share their dequantised blocks too (M is the total
-    // row count; below ~256 rows per expert the wider single-block tile measures faster)
-    if (w_kind == 1 && grouped && !residual && M >= 256 * E && N % 128 == 0) { bn = 128; mt = 2; }
-    // few rows: the work is streaming W, so spread it over more SMs with narrower tiles
-    if (!grouped && ((M + kXBM - 1) / kXBM) * ((N + 127) / 128) < 100) bn = 64;
+    // What bounds a full tile is shared-memory traffic (per 64 of K, 128 x 256: the products read 48 KB, A and the expanded W
+    // are written, the packed W written and read: 112 KB at 128 bytes a cycle), so the widest tile is the best where there are
+    // tiles enough: bf16 8192 x 28672 x 4096 with SwiGLU 1685 us with 128 columns, 1366 with 256; 4-bit 2048 x 28672 x 4096
+    // 615 / 477 (two stacked row blocks of 128 columns: 478), 128 experts of 3072 x 4096 at 128 rows each 835 / 665.
+    const int tiles256 = ((M + kXBM - 1) / kXBM) * ((N + 255) / 256), tiles128 = ((M + kXBM - 1) / kXBM) * ((N + 127) / 128);
+    const bool whole = (!grouped && !swiglu) || N % 256 == 0;
+    if (grouped) bn = whole && M >= 1024 ? 256 : 128;
+    // few rows are a stream of W: 64 x 28672 x 4096 in 4 bits 45 us with 256 columns (112 tiles), 61 with 128, 81 stacked;
+    // 64 x 9216 x 4096 28 us with 64 columns (144 tiles), 40 with 256 (36)
+    else if (whole && (w_kind == 1 ? tiles256 >= 100 : tiles256 >= 100 && M >= 1024)) bn = 256;
+    else bn = tiles128 < 100 ? 64 : 128;
   }
   if (bn != 64 && bn != 128 && bn != 256) return -2;
   if (grouped && N % bn) return -2;

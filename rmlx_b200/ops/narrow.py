@@ -28,8 +28,8 @@ def supported(w: LinearWeight) -> bool:
 def pays(w: LinearWeight, rows: int) -> bool:
     """Whether a plain projection of ``rows`` rows is faster here than on the 128-row tensor-core tiles (and takes this weight).
 
-    Measured (us, this kernel / the tiles). 4-bit, 9216 x 4096: 16 / 32 at 16 rows, 30 / 32 at 32, 40 / 32 at 64; 28672 x 4096:
-    31 / 73, 55 / 73, 106 / 74; 4096 x 14336: 34 / 96, 83 / 96, 90 / 96: up to 32 rows, and up to 64 where a few rows of W leave
+    Measured (us, this kernel / the tiles). 4-bit, 9216 x 4096: 16 / 28 at 16 rows, 30 / 28 at 32, 40 / 29 at 64; 28672 x 4096:
+    31 / 47, 55 / 47, 106 / 45; 4096 x 8192: 21 / 53, 48 / 54, 62 / 57: up to 16 rows, and up to 32 where a few rows of W leave
     the tiles less than half of the SMs. 8-bit weights would be expanded first (53 us for 28672 x 4096). bf16, 9216 x 4096:
     20 / 28 at 16 rows; 28672 x 4096: 46 / 45: eight rows, and 16 for up to 16384 rows of W. Weights of less than a million
     entries take a tile's time anyway."""
@@ -38,7 +38,7 @@ def pays(w: LinearWeight, rows: int) -> bool:
     if w.kind == W_BF16:
         ok = rows <= 8 or (rows <= 16 and w.n <= 16384)
     elif w.kind == W_Q4:
-        ok = rows <= 32 or w.n <= 4096
+        ok = rows <= 16 or (rows <= 32 and w.n <= 4096)
     else:
         ok = rows <= 16 or (rows <= 32 and w.n >= 8192)
     return ok and supported(w)
