@@ -156,7 +156,13 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream_ptr(stream: Optional[torch.cuda.Stream] = None) -> int:
-    return (stream or torch.cuda.current_stream()).cuda_stream
+    """The raw handle of ``stream`` or of the current device's current stream. Asked for at every launch: the handle itself
+    costs 0.3 us, a ``torch.cuda.current_stream()`` object 4 (a third of a short prompt's host time)."""
+    if stream is not None:
+        return stream.cuda_stream
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _launch_count = 0

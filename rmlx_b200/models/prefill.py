@@ -45,6 +45,24 @@ def _mm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = Non
     return qmm(x, w, residual=residual)
 
 
+def _norm_fits(x: torch.Tensor, w: LinearWeight, norm: torch.Tensor) -> bool:
+    """Whether ``_narrow`` rows can take their norm along (16-bit weights then use twice the tiles of rows)."""
+    return _narrow(x, w) and norm.data_ptr() % 16 == 0 and (w.kind != W_BF16 or x.shape[0] <= 8)
+
+
+def _norm_mm(h: torch.Tensor, norm: torch.Tensor, eps: float, w: LinearWeight) -> torch.Tensor:
+    """rmsnorm(h) W^T; one launch where the weight-streaming kernel takes the rows."""
+    if _norm_fits(h, w, norm):
+        return narrow.narrow_gemm(h, w, norm, eps)
+    return _mm(D.rms_norm(h, norm, eps), w)
+
+
+def _norm_gate_up_act(h: torch.Tensor, norm: torch.Tensor, eps: float, w: LinearWeight) -> torch.Tensor:
+    if w.n % 32 == 0 and _norm_fits(h, w, norm):
+        return narrow.narrow_gemm(h, w, norm, eps, swiglu=True)
+    return _gate_up_act(D.rms_norm(h, norm, eps), w)
+
+
 def _gate_up_act(x: torch.Tensor, w: LinearWeight) -> torch.Tensor:
     """silu(x W_gate^T) * (x W_up^T) for W = [gate; up]: SwiGLU runs in the GEMM epilogue when the
     shape allows, else GEMM then the element-wise kernel."""
@@ -97,13 +115,12 @@ class _Layers:
         t = h.shape[0]
         hd, hq = cfg.head_dim, m.hq
         for li, lw in enumerate(w.layers):
-            xn = D.rms_norm(h, lw.norm1, cfg.rms_norm_eps)
-            qkv = _mm(xn, lw.wqkv)
+            qkv = _norm_mm(h, lw.norm1, cfg.rms_norm_eps, lw.wqkv)
             attn = attend(li, qkv)
             h = self._row_parallel(attn.view(t, hq * hd), lw.wo, h)
-            xn = D.rms_norm(h, lw.norm2, cfg.rms_norm_eps)
             if lw.router is not None:
                 moe = cfg.ff_type.moe
+                xn = D.rms_norm(h, lw.norm2, cfg.rms_norm_eps)
                 logits = _router_logits(xn, lw.router)
                 idx, wts, _, offsets = D.topk_route(logits, moe.num_experts_per_token, lw.expert_bias)
                 single = m.layout.world == 1 and lw.shared_gate_up is None
@@ -113,7 +130,7 @@ class _Layers:
                     y = y + _mm(_gate_up_act(xn, lw.shared_gate_up), lw.shared_down)
                 h = y if single else h + m._sum(y)
             else:
-                act = _gate_up_act(xn, lw.w_gate_up)
+                act = _norm_gate_up_act(h, lw.norm2, cfg.rms_norm_eps, lw.w_gate_up)
                 h = self._row_parallel(act, lw.w_down, h)
         return h
 
