@@ -32,7 +32,7 @@ constexpr int kXMaxExperts = 256;
 constexpr int kXMaxRanks = 8;
 constexpr int kCommNone = 0, kCommReduce = 1, kCommGather = 2;
 constexpr int kGatherChunkRows = 8;
-constexpr int kDqWarps = 8;          // dequant warps of one group of the Q4 main loop (two per SM sub-partition)
+constexpr int kDqWarps = 8;          // dequant warps of the collective modes' Q4 main loop (two per SM sub-partition)
 constexpr int kCommThreads = 160;   // collective modes: four reducer/pusher warps + one signalling warp
 
 struct XComm {
@@ -53,16 +53,19 @@ struct XComm {
   unsigned long long* trace = nullptr;       // optional [grid][8] timestamps (see x_trace)
 };
 
-// Single-GPU Q4 form: a warp of its own asks for the packed weights, as far ahead as their ring is deep (behind the rows of A
-// it was five 4 KB stages, too little under way to stream the experts of a decode batch), and two groups of dequant warps take
-// the k-blocks in turn, so that one expands while the other waits for its block, its slot or its stores. The collective modes
-// keep the narrower block (their five warps need the registers).
+// Single-GPU Q4 form. A warp of its own asks for the packed weights, as far ahead as their ring is deep (behind the rows of A it was
+// four 4 KB stages, too little under way to stream the experts of a decode batch), 64 or 128 bytes of a row at a time, since the copy
+// engine spends its time per row. A k-block's expansion is a chain of some 200 dependent instructions, two waits and a fence,
+// so four groups of four warps take the k-blocks in turn (one group of eight warps: 815 cycles a k-block of 128 rows). Four groups
+// need four operand stages: a group that has finished its k-block waits for a slot whose last use but one must be over, or the
+// barrier's parity would tell it nothing; with three stages there are two groups of eight. The collective modes keep the
+// narrower block (their five warps need the registers).
 template <bool WQ4, int COMM>
 struct XRoles {
   static constexpr bool kDeep = WQ4 && COMM == kCommNone;
-  static constexpr int kGroups = kDeep ? 2 : 1;
-  static constexpr int kRawWarp = 6 + kDqWarps * kGroups;            // kDeep only
-  static constexpr int kThreads = 192 + (WQ4 ? 32 * kDqWarps * kGroups : 0) + (kDeep ? 32 : 0) + (COMM != kCommNone ? kCommThreads : 0);
+  static constexpr int kDq = kDeep ? 16 : kDqWarps;
+  static constexpr int kRawWarp = 6 + kDq;                           // kDeep only
+  static constexpr int kThreads = 192 + (WQ4 ? 32 * kDq : 0) + (kDeep ? 32 : 0) + (COMM != kCommNone ? kCommThreads : 0);
 };
 
 // MT = 2: a tile is two stacked 128-row blocks of A against ONE staged block of W, i.e. two
@@ -70,16 +73,46 @@ struct XRoles {
 template <int BN, bool WQ4, int MT = 1, bool DEEP = false>
 struct XSmem {
   static constexpr int kStages = MT == 2 ? 3 : (WQ4 ? ((BN >= 256) ? 3 : 5) : ((BN >= 256) ? 4 : 6));
-  static constexpr int kRawStages = !DEEP ? 4 : BN >= 256 ? 7 : BN == 128 ? 12 : 16;
+  static constexpr int kRawBlocks = !DEEP ? 1 : BN >= 256 ? 2 : 4;     // k-blocks per stage of packed weights
+  static constexpr int kRawStages = !DEEP ? 4 : BN == 64 ? 6 : 3;
   static constexpr int kStageA = MT * kXBM * kXBK * 2;
   static constexpr int kStageB = BN * kXBK * 2;
-  static constexpr int kStageRaw = BN * 32;          // 64 nibbles per row
+  static constexpr int kStageRaw = BN * 32 * kRawBlocks;             // 64 nibbles per row and k-block
   static constexpr int kScaleSlot = 2 * BN * 16;     // scales + biases for 8 k-blocks
   static constexpr int kBarBytes = 768;              // 3 kStages + 2 kRawStages + 13 barriers of 8 bytes, three words
   static constexpr int kBytes = kStages * (kStageA + kStageB) +
                                 (WQ4 ? kRawStages * kStageRaw + 2 * kScaleSlot : 0) + 1024 + kBarBytes +
                                 (kXMaxExperts + 2) * 8;
 };
+
+// Plain shared-memory accesses: through a pointer whose address space the compiler has lost they would be generic ones.
+__device__ __forceinline__ uint4 x_lds(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t x_lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void x_sts(uint32_t a, const uint32_t (&v)[4]) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+// Eight 4-bit codes of a word in order, as s q + b rounded once to bf16.
+__device__ __forceinline__ void x_expand(uint32_t w, __nv_bfloat162 s2, __nv_bfloat162 b2, uint32_t (&o)[4]) {
+  // byte b of the word holds elements 2b (low nibble) and 2b + 1 (high nibble): pick the byte from w and from w >> 4 into the two
+  // halves, keep the low nibbles, and drop them into the mantissa of 128.0 (128 + q is exact in bf16)
+  const uint32_t w4 = w >> 4;
+  const uint32_t p[4] = {(__byte_perm(w, w4, 0x0400u) & 0x000f000fu) | 0x43004300u, (__byte_perm(w, w4, 0x0501u) & 0x000f000fu) | 0x43004300u,
+                         (__byte_perm(w, w4, 0x0602u) & 0x000f000fu) | 0x43004300u, (__byte_perm(w, w4, 0x0703u) & 0x000f000fu) | 0x43004300u};
+  const __nv_bfloat162 k128 = __float2bfloat162_rn(128.f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 v = __hfma2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&p[i]), k128), s2, b2);
+    o[i] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
 
 struct XTile {
   int a_row0;     // first row of the A/C tile
@@ -208,6 +241,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   using Ro = XRoles<WQ4, COMM>;
   using S = XSmem<BN, WQ4, MT, Ro::kDeep>;
   constexpr int STAGES = S::kStages, RAW = S::kRawStages;
+  constexpr int GROUPS = !Ro::kDeep ? 1 : STAGES >= 4 ? 4 : 2, GROUP_WARPS = Ro::kDq / GROUPS;
   // a role may be waiting, through the pipeline, on a peer that started late: be more patient then
   constexpr uint32_t LIM = (COMM == kCommNone) ? kMbarPollLimit : (kMbarPollLimit << 4);
   constexpr int kCommWarp0 = 6 + (WQ4 ? kDqWarps : 0);   // first of the five collective-mode warps
@@ -244,10 +278,10 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const int num_kb = (K + kXBK - 1) / kXBK;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < STAGES; ++i) { mbar_init(full + i, 1); mbar_init(empty + i, 1); mbar_init(bq_full + i, kDqWarps); }
-    for (int i = 0; i < RAW; ++i) { mbar_init(raw_full + i, 1); mbar_init(raw_empty + i, kDqWarps); }
+    for (int i = 0; i < STAGES; ++i) { mbar_init(full + i, 1); mbar_init(empty + i, 1); mbar_init(bq_full + i, GROUP_WARPS); }
+    for (int i = 0; i < RAW; ++i) { mbar_init(raw_full + i, 1); mbar_init(raw_empty + i, S::kRawBlocks * GROUP_WARPS); }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(sc_full + i, 1); mbar_init(sc_empty + i, kDqWarps * Ro::kGroups);
+      mbar_init(sc_full + i, 1); mbar_init(sc_empty + i, Ro::kDq);
       mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 4);
     }
     for (int i = 0; i < 2; ++i) { mbar_init(sig_full + i, 128); mbar_init(sig_free + i, 1); }
@@ -614,28 +648,97 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             }
             if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
           }
-          if (!mbar_wait(raw_empty + rstage, rphase ^ 1u, abort_flag, LIM)) { ok = false; break; }
-          mbar_arrive_expect_tx(raw_full + rstage, S::kStageRaw);
-          tma_load_2d(sRaw + rstage * S::kStageRaw, &tmap_w, raw_full + rstage, kb * 32, t.w_row0);
-          if (swiglu)
-            tma_load_2d(sRaw + rstage * S::kStageRaw + BN * 16, &tmap_w, raw_full + rstage, kb * 32, t.w_row0 + N / 2);
-          if (++rstage == RAW) { rstage = 0; rphase ^= 1u; }
+          if (kb % S::kRawBlocks == 0) {
+            if (!mbar_wait(raw_empty + rstage, rphase ^ 1u, abort_flag, LIM)) { ok = false; break; }
+            mbar_arrive_expect_tx(raw_full + rstage, S::kStageRaw);
+            tma_load_2d(sRaw + rstage * S::kStageRaw, &tmap_w, raw_full + rstage, kb * 32, t.w_row0);
+            if (swiglu)
+              tma_load_2d(sRaw + rstage * S::kStageRaw + S::kStageRaw / 2, &tmap_w, raw_full + rstage, kb * 32, t.w_row0 + N / 2);
+            if (++rstage == RAW) { rstage = 0; rphase ^= 1u; }
+          }
         }
       }
     }
-  } else if (WQ4 && warp < 6 + kDqWarps * Ro::kGroups) {
-    // ------------------------------------------------------------------ dequant (from warp 6)
-    const int dt = (threadIdx.x - 192) % (32 * kDqWarps);          // 0 .. 32*kDqWarps-1 within the group
-    const int group = (threadIdx.x - 192) / (32 * kDqWarps);       // takes k-blocks group, group + kGroups, ..
-    int stage = group, rstage = group, sslot = 0;
+  } else if (Ro::kDeep && warp < 6 + Ro::kDq) {
+    // ------------------------------------------------------------------ dequant, single GPU (from warp 6)
+    // group g takes k-blocks g, g + GROUPS, ..; a thread expands a row (or two, or half a row) of its k-block
+    constexpr int GT = 32 * GROUP_WARPS, ROWS = BN >= GT ? BN / GT : 1, WORDS = BN >= GT ? 8 : 4, RB = S::kRawBlocks;
+    static_assert(!Ro::kDeep || BN >= GT || 2 * BN == GT, "half a row at least");
+    const int dt = (threadIdx.x - 192) % GT, group = (threadIdx.x - 192) / GT;
+    const int row0 = BN >= GT ? dt : dt % BN, part = BN >= GT ? 0 : dt / BN;     // part: which half of the row's 64
+    const uint32_t half_sel = (group & 1) ? 0x3232u : 0x1010u;
+    int stage = group, rstage = group / RB, sslot = 0;
+    uint32_t phase = 0, rphase = 0, sphase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int kb8 = 0; kb8 < num_kb && ok; kb8 += 8) {     // K % 512 == 0: whole groups of 8
+        if (!mbar_wait(sc_full + sslot, sphase, abort_flag, LIM)) { ok = false; break; }
+        uint32_t sws[ROWS][8 / GROUPS], bws[ROWS][8 / GROUPS];       // k-blocks kb8 + GROUPS i + group, the half_sel half of each
+#pragma unroll
+        for (int it = 0; it < ROWS; ++it) {
+          const uint32_t scb = smem_u32(sScale) + sslot * S::kScaleSlot + (row0 + it * GT) * 16 + (group >> 1) * 4;
+#pragma unroll
+          for (int i = 0; i < 8 / GROUPS; ++i) {
+            sws[it][i] = x_lds32(scb + i * (2 * GROUPS));
+            bws[it][i] = x_lds32(scb + BN * 16 + i * (2 * GROUPS));
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sc_empty + sslot);       // the slot can be refilled already
+        if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
+#pragma unroll
+        for (int i = 0; i < 8 / GROUPS; ++i) {
+          if (!mbar_wait(raw_full + rstage, rphase, abort_flag, LIM)) { ok = false; break; }
+          if (!mbar_wait(empty + stage, phase ^ 1u, abort_flag, LIM)) { ok = false; break; }  // B slot free
+          const int piece = (GROUPS * i + group) % RB * 2 + part;    // 16 bytes of the row's 32 RB
+#pragma unroll
+          for (int it = 0; it < ROWS; ++it) {
+            const int r = row0 + it * GT;
+            // eight lanes read the same piece of eight rows: with the copy's swizzle that is every bank once
+            const uint32_t raw = smem_u32(sRaw) + rstage * S::kStageRaw + r * (32 * RB);
+            const int sw = RB == 4 ? r & 7 : (r >> 1) & 3;
+            const uint4 w0 = x_lds(raw + ((piece ^ sw) << 4));
+            const uint32_t s2u = __byte_perm(sws[it][i], 0u, half_sel), b2u = __byte_perm(bws[it][i], 0u, half_sel);
+            const __nv_bfloat162 s2 = *reinterpret_cast<const __nv_bfloat162*>(&s2u);
+            const __nv_bfloat162 b2 = *reinterpret_cast<const __nv_bfloat162*>(&b2u);
+            uint32_t words[8] = {w0.x, w0.y, w0.z, w0.w};
+            if (WORDS == 8) {
+              const uint4 w1 = x_lds(raw + (((piece + 1) ^ sw) << 4));
+              words[4] = w1.x; words[5] = w1.y; words[6] = w1.z; words[7] = w1.w;
+            }
+            const uint32_t bst = smem_u32(sB) + stage * S::kStageB + r * 128;
+#pragma unroll
+            for (int j = 0; j < WORDS; ++j) {
+              uint32_t o[4];
+              x_expand(words[j], s2, b2, o);
+              x_sts(bst + (((part * 4 + j) ^ (r & 7)) << 4), o);
+            }
+          }
+          fence_proxy_async_smem();     // generic-proxy stores -> visible to the tensor core's reads
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(bq_full + stage);
+            mbar_arrive(raw_empty + rstage);
+          }
+          if (GROUPS >= RB || i % (RB / (GROUPS < RB ? GROUPS : RB)) == RB / (GROUPS < RB ? GROUPS : RB) - 1) {
+            rstage += GROUPS >= RB ? GROUPS / RB : 1;
+            if (rstage >= RAW) { rstage -= RAW; rphase ^= 1u; }
+          }
+          stage += GROUPS;
+          if (stage >= STAGES) { stage -= STAGES; phase ^= 1u; }
+        }
+      }
+    }
+  } else if (WQ4 && !Ro::kDeep && warp < 6 + kDqWarps) {
+    // ------------------------------------------------------------------ dequant (warps 6..13)
+    const int dt = threadIdx.x - 192;   // 0 .. 32*kDqWarps-1
+    int stage = 0, rstage = 0, sslot = 0;
     uint32_t phase = 0, rphase = 0, sphase = 0;
     bool ok = true;
     // Static work split: item = (row of the W tile, which 32-element half of the 64-wide k-block);
     // consecutive threads take consecutive 16-byte pieces of the packed tile (conflict-free loads),
     // and a row's 8 group scales/biases stay in registers for 8 k-blocks.
     constexpr int ITEMS = (BN * 2 + 32 * kDqWarps - 1) / (32 * kDqWarps);
-    const __nv_bfloat162 k128 = __float2bfloat162_rn(128.f);
-    const uint32_t half_sel = group ? 0x3232u : 0x1010u;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       for (int kb8 = 0; kb8 < num_kb && ok; kb8 += 8) {     // K % 512 == 0: whole groups of 8
         if (!mbar_wait(sc_full + sslot, sphase, abort_flag, LIM)) { ok = false; break; }
@@ -653,8 +756,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         if (lane == 0) mbar_arrive(sc_empty + sslot);       // the slot can be refilled already
         if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
 #pragma unroll
-        for (int k2 = 0; k2 < 8 / Ro::kGroups; ++k2) {
-          const int kk = k2 * Ro::kGroups + group;
+        for (int kk = 0; kk < 8; ++kk) {
           if (!mbar_wait(raw_full + rstage, rphase, abort_flag, LIM)) { ok = false; break; }
           if (!mbar_wait(empty + stage, phase ^ 1u, abort_flag, LIM)) { ok = false; break; }  // B slot free
           const char* raw = sRaw + rstage * S::kStageRaw;
@@ -665,33 +767,19 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             if (item < BN * 2) {
               const int r = item >> 1, h = item & 1;
               const uint4 wv = *reinterpret_cast<const uint4*>(raw + item * 16);
-              // two groups: word k2 of the row's scales, the group's half of it
-              const uint32_t sws[4] = {sv[it].x, sv[it].y, sv[it].z, sv[it].w}, bws[4] = {bv[it].x, bv[it].y, bv[it].z, bv[it].w};
-              const int wi = Ro::kGroups == 2 ? k2 : k2 >> 1;
-              const uint32_t odd = Ro::kGroups == 2 ? half_sel : (k2 & 1) ? 0x3232u : 0x1010u;
-              const uint32_t s2u = __byte_perm(sws[wi], 0u, odd), b2u = __byte_perm(bws[wi], 0u, odd);
+              const uint32_t sw = (kk >> 1) == 0 ? sv[it].x : (kk >> 1) == 1 ? sv[it].y : (kk >> 1) == 2 ? sv[it].z : sv[it].w;
+              const uint32_t bw = (kk >> 1) == 0 ? bv[it].x : (kk >> 1) == 1 ? bv[it].y : (kk >> 1) == 2 ? bv[it].z : bv[it].w;
+              const uint32_t s2u = __byte_perm(sw, 0u, (kk & 1) ? 0x3232u : 0x1010u);
+              const uint32_t b2u = __byte_perm(bw, 0u, (kk & 1) ? 0x3232u : 0x1010u);
               const __nv_bfloat162 s2 = *reinterpret_cast<const __nv_bfloat162*>(&s2u);
               const __nv_bfloat162 b2 = *reinterpret_cast<const __nv_bfloat162*>(&b2u);
               const uint32_t words[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const uint32_t w = words[j], w4 = w >> 4;
-                // byte b of the word holds elements 2b (low nibble) and 2b+1 (high nibble): pick the
-                // byte from w and from w>>4 into the two halves, keep the low nibbles, and drop them
-                // into the mantissa of 128.0 (128 + q is exact in bf16)
-                uint32_t p0 = (__byte_perm(w, w4, 0x0400u) & 0x000f000fu) | 0x43004300u;
-                uint32_t p1 = (__byte_perm(w, w4, 0x0501u) & 0x000f000fu) | 0x43004300u;
-                uint32_t p2 = (__byte_perm(w, w4, 0x0602u) & 0x000f000fu) | 0x43004300u;
-                uint32_t p3 = (__byte_perm(w, w4, 0x0703u) & 0x000f000fu) | 0x43004300u;
-                __nv_bfloat162 v0 = __hfma2(__hsub2(*reinterpret_cast<__nv_bfloat162*>(&p0), k128), s2, b2);
-                __nv_bfloat162 v1 = __hfma2(__hsub2(*reinterpret_cast<__nv_bfloat162*>(&p1), k128), s2, b2);
-                __nv_bfloat162 v2 = __hfma2(__hsub2(*reinterpret_cast<__nv_bfloat162*>(&p2), k128), s2, b2);
-                __nv_bfloat162 v3 = __hfma2(__hsub2(*reinterpret_cast<__nv_bfloat162*>(&p3), k128), s2, b2);
-                uint4 o;   // natural k order: (k0,k1) (k2,k3) (k4,k5) (k6,k7)
-                o.x = *reinterpret_cast<uint32_t*>(&v0); o.y = *reinterpret_cast<uint32_t*>(&v1);
-                o.z = *reinterpret_cast<uint32_t*>(&v2); o.w = *reinterpret_cast<uint32_t*>(&v3);
+                uint32_t ov[4];      // natural k order: (k0,k1) (k2,k3) (k4,k5) (k6,k7)
+                x_expand(words[j], s2, b2, ov);
                 const int c = h * 4 + j;                 // 16-byte chunk of the 128-byte row
-                *reinterpret_cast<uint4*>(bst + r * 128 + ((c ^ (r & 7)) << 4)) = o;
+                *reinterpret_cast<uint4*>(bst + r * 128 + ((c ^ (r & 7)) << 4)) = make_uint4(ov[0], ov[1], ov[2], ov[3]);
               }
             }
           }
@@ -701,10 +789,8 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             mbar_arrive(bq_full + stage);
             mbar_arrive(raw_empty + rstage);
           }
-          rstage += Ro::kGroups;
-          if (rstage >= RAW) { rstage -= RAW; rphase ^= 1u; }
-          stage += Ro::kGroups;
-          if (stage >= STAGES) { stage -= STAGES; phase ^= 1u; }
+          if (++rstage == RAW) { rstage = 0; rphase ^= 1u; }
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
     }
@@ -746,7 +832,7 @@ static int launch_x(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtenso
 // Tensor maps of the weight operand (and of its scales/biases for Q4).
 static inline int x_weight_maps(int w_kind, const void* W, const void* scales, const void* biases,
                                 uint64_t rowsW, int K, int bn, CUtensorMap* tw, CUtensorMap* ts,
-                                CUtensorMap* tb) {
+                                CUtensorMap* tb, int raw_blocks = 1) {
   int rc;
   if (w_kind == 0) {
     rc = make_tmap_2d_bf16(tw, W, uint64_t(K), rowsW, uint64_t(K) * 2, kXBK, bn);
@@ -755,7 +841,8 @@ static inline int x_weight_maps(int w_kind, const void* W, const void* scales, c
     return 0;
   }
   rc = make_tmap_2d(tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, W, uint64_t(K) / 2, rowsW, uint64_t(K) / 2,
-                    32, bn, CU_TENSOR_MAP_SWIZZLE_NONE);
+                    32 * raw_blocks, bn, raw_blocks == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : raw_blocks == 2 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                                                         : CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc) return rc;
   rc = make_tmap_2d(ts, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, scales, uint64_t(K) / 64, rowsW,
                     uint64_t(K) / 64 * 2, 8, bn, CU_TENSOR_MAP_SWIZZLE_NONE);

@@ -1,6 +1,6 @@
 // Generalised tcgen05 GEMM, single-GPU entry points: C = A · W^T with
 //   * W either bf16 (TMA-fed) or MLX-affine Q4 (group 64) dequantised INSIDE the main loop:
-//     packed nibbles and per-group scales/biases arrive by TMA, four dequant warps expand them to
+//     packed nibbles and per-group scales/biases arrive by TMA, four groups of dequant warps expand them to
 //     bf16 (exactly s*q+b, rounded once) straight into the 128-byte-swizzled operand stage that
 //     tcgen05.mma reads, so quantised weights never exist in memory in expanded form;
 //   * an optional grouped mode for mixture-of-experts: rows of A are sorted by expert, a device
@@ -10,7 +10,7 @@
 //     crates/rmlx-core/src/ops/matmul.rs:8823-8950).
 //
 // Roles per CTA (persistent, one CTA per SM): warp 0 TMA producer, warp 1 MMA issuer (owns TMEM),
-// warps 2-5 epilogue (TMEM -> registers -> bf16 global, + residual), warps 6-13 dequant (Q4 only).
+// warps 2-5 epilogue (TMEM -> registers -> bf16 global, + residual), warps 6-21 dequant, warp 22 packed weights (Q4 only).
 // Accumulators are double-buffered in TMEM. All pipeline waits are bounded. The kernel itself is in
 // xgemm_kernel.cuh.
 //
@@ -64,7 +64,7 @@ extern "C" int rmlx_xgemm(int w_kind, const void* A, const void* W, const void* 
   CUtensorMap ta, tw, ts, tb;
   int rc = make_tmap_2d_bf16(&ta, A, uint64_t(K), uint64_t(M), uint64_t(lda) * 2, kXBK, kXBM);
   if (rc) return rc;
-  rc = x_weight_maps(w_kind, W, scales, biases, rowsW, K, swiglu ? bn / 2 : bn, &tw, &ts, &tb);
+  rc = x_weight_maps(w_kind, W, scales, biases, rowsW, K, swiglu ? bn / 2 : bn, &tw, &ts, &tb, bn == 256 ? XSmem<256, true, 1, true>::kRawBlocks : XSmem<128, true, 1, true>::kRawBlocks);
   if (rc) return rc;
 #define RB_X(BN_, Q_, G_)                                                                          \
   return residual ? launch_x<BN_, Q_, G_, true>(ta, ta, tw, ts, tb, C, residual, offsets, E, M, N, K, ldc, status, pdl, st) \

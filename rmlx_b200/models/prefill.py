@@ -28,7 +28,7 @@ from ..runtime.graph import GraphCache, bucket_for
 from ..ops.attention import flash_prefill_paged
 from ..ops.gemm import GemmStatus, gemm_bf16
 from ..ops.grouped import moe_prefill_ffn
-from ..ops.quantized import qmm, xgemm
+from ..ops.quantized import pair_pays, qmm, xgemm
 from ..ops.weights import LinearWeight, W_BF16, W_Q4
 
 
@@ -41,6 +41,8 @@ def _mm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = Non
     if w.kind == W_BF16:
         if _narrow(x, w):
             return narrow.narrow_gemm(x, w, residual=residual)
+        if x.shape[0] > 128 and pair_pays(W_BF16, x.shape[0], w.n, w.k):
+            return xgemm(x, w, residual=residual)         # SM pairs
         return gemm_bf16(x, w.w, residual=residual)
     return qmm(x, w, residual=residual)
 

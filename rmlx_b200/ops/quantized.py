@@ -18,6 +18,8 @@ from .weights import LinearWeight, W_Q4
 _lib.register_cuda_sigs({
     "rmlx_qgemm_supported": ("i", "i"),
     "rmlx_xgemm": ("ipppppppiiiiiiiifpip", "i"),
+    "rmlx_pair_gemm_supported": ("iiiiii", "i"),
+    "rmlx_pair_gemm": ("ipppppppiiiiiiifpip", "i"),
     "rmlx_moe_scatter_rows": ("pipppppiiiip", "i"),
     "rmlx_moe_combine": ("ppppipiiiip", "i"),
 })
@@ -40,12 +42,58 @@ def xgemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = N
         assert offsets.dtype == torch.int32 and offsets.numel() == e + 1
     if out is None:
         out = torch.empty(m, n // 2 if swiglu else n, dtype=torch.bfloat16, device=x.device)
+    if bn == 0 and m > 128 and pair_pays(w.kind, m, n, k, e) and (not swiglu or (n % 256 == 0 and residual is None)) and \
+            (residual is None or e == 0) and (w.kind != W_Q4 or not w.scales_f16) and (w.kind != W_Q4 or k % 512 == 0) and \
+            k % 8 == 0 and _pair_ready(x, out, residual) and out.dtype == torch.bfloat16:
+        return pair_gemm(x, w, residual, out, offsets, swiglu, gate_limit, pdl)
     rc = _lib.cuda().rmlx_xgemm(w.kind, x.data_ptr(), w.w.data_ptr(), _lib.ptr(w.scales),
                                 _lib.ptr(w.biases), out.data_ptr(), _lib.ptr(residual),
                                 _lib.ptr(offsets), e, m, n, k, x.stride(0), out.stride(0), bn, int(swiglu),
                                 gate_limit,
                                 GemmStatus.get(x.device).data_ptr(), int(pdl), _lib.stream_ptr())
     _lib.check(rc, "xgemm")
+    return out
+
+
+def pair_pays(kind: int, m: int, n: int, k: int, experts: int = 0) -> bool:
+    """Whether 256 x 256 tiles of SM pairs are faster than 128-row tiles of single SMs.
+
+    Measured (us, pairs / single SMs). 4-bit, 2048 rows: 28672 x 4096 346 / 455, 9216 x 4096 109 / 150, 4096 x 14336 176 / 243; 512
+    rows: 102 / 147, 34 / 44, 82 / 93, 4096 x 4096 (32 tiles) 31 / 31; 256 rows: 4096 x 4096 29 / 28. bf16, 8192 x 28672 x 4096 1232 /
+    1371, 1024 x 4096 x 4096 (64 tiles) 29 / 31, 512 x 9216 x 4096 (72) 32 / 39, 512 x 4096 x 8192 (32) 52 / 43. 4-bit experts (128 of
+    3072 x 4096 and 4096 x 1536): 930 + 560 / 1026 + 612 at 256 rows each, 622 + 369 / 626 + 376 at 128, where half of a pair's rows
+    are mostly empty."""
+    if experts:
+        return kind == W_Q4 and m >= 192 * experts and n % 256 == 0
+    tiles = -(-m // 256) * -(-n // 256)
+    return n % 32 == 0 and (m > 128 and tiles >= 32 if kind == W_Q4 else tiles >= 60 and m > 128)
+
+
+def _pair_ready(x: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
+    """16-byte rows, as the pair kernel loads and stores them."""
+    return x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and \
+        out.stride(1) == 1 and (residual is None or (residual.data_ptr() % 16 == 0 and residual.stride() == out.stride()))
+
+
+def pair_gemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+              offsets: Optional[torch.Tensor] = None, swiglu: bool = False, gate_limit: float = 0.0, pdl: bool = False) -> torch.Tensor:
+    """``xgemm`` on 256 x 256 tiles of SM pairs (csrc/kernels/pair_gemm.cu)."""
+    _lib.require_cuda_tensor(x, w.w)
+    assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1
+    m, k = x.shape
+    n = w.n
+    assert k == w.k
+    e = w.experts if offsets is not None else 0
+    if offsets is not None:
+        assert offsets.dtype == torch.int32 and offsets.numel() == e + 1
+    if out is None:
+        out = torch.empty(m, n // 2 if swiglu else n, dtype=torch.bfloat16, device=x.device)
+    if residual is not None:
+        assert residual.shape == out.shape and residual.stride() == out.stride()
+    rc = _lib.cuda().rmlx_pair_gemm(w.kind, x.data_ptr(), w.w.data_ptr(), _lib.ptr(w.scales), _lib.ptr(w.biases), out.data_ptr(),
+                                    _lib.ptr(residual), _lib.ptr(offsets), e, m, n, k, x.stride(0), out.stride(0), int(swiglu),
+                                    gate_limit, GemmStatus.get(x.device).data_ptr(), int(pdl), _lib.stream_ptr())
+    _lib.check(rc, "pair_gemm")
     return out
 
 

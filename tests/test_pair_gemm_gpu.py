@@ -1,0 +1,81 @@
+"""The tensor-core GEMM on SM pairs (csrc/kernels/pair_gemm.cu): the same products in the same order as the single-SM tiles, so
+plain results are equal bit for bit; against 64 bits the error is that of a bf16 result (and, for 4-bit weights, of weights
+rounded to bf16).
+
+Bounds: a rounding to bf16 is off by at most 2^-9 = 1.96e-3 of the value, so a result of bf16 weights by at most that of its norm
+(ROUND, with room for the fp32 sums); weights rounded to bf16 add at most as much again before anything averages out, and a
+gated activation, gate and up rounded each, at most three times that."""
+import pytest
+import torch
+
+ROUND = 2.0e-3
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    return torch.device("cuda")
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+def _case(dev, kind, m, n, k, experts=0, seed=0):
+    from rmlx_b200.ops.weights import LinearWeight
+    g = torch.Generator(device=dev).manual_seed(seed)
+    w = LinearWeight.random(n, k, kind, dev, experts=experts, generator=g)
+    return w, w.dequantized().double(), torch.randn(m, k, device=dev, generator=g).to(torch.bfloat16), g
+
+
+# one row, half a pair's rows and one more, more tiles than pairs, columns that end inside a tile
+@pytest.mark.parametrize("kind", [None, "q4"])
+@pytest.mark.parametrize("m,n,k", [(1, 256, 512), (129, 288, 1024), (256, 256, 4096), (300, 544, 1536), (2600, 2048, 512)])
+def test_plain(dev, kind, m, n, k):
+    from rmlx_b200.ops.gemm import GemmStatus
+    from rmlx_b200.ops.quantized import pair_gemm, xgemm
+    w, wd, x, g = _case(dev, kind, m, n, k)
+    want = x.double() @ wd.t()
+    got = pair_gemm(x, w)
+    assert torch.equal(got, xgemm(x, w, bn=128))
+    assert _rel(got, want) < (2 * ROUND if kind else ROUND)
+    res = torch.randn(m, n, device=dev, generator=g).to(torch.bfloat16)
+    assert _rel(pair_gemm(x, w, residual=res), want + res.double()) < 2 * ROUND
+    if n % 256 == 0:
+        act = torch.nn.functional.silu(want[:, :n // 2]) * want[:, n // 2:]
+        assert _rel(pair_gemm(x, w, swiglu=True), act) < (4 * ROUND if kind else ROUND)
+    GemmStatus.check(dev)
+
+
+@pytest.mark.parametrize("kind", [None, "q4"])
+def test_grouped(dev, kind):
+    """Experts without rows, with one, with a whole tile and with more."""
+    from rmlx_b200.ops.gemm import GemmStatus
+    from rmlx_b200.ops.quantized import pair_gemm
+    counts = [3, 0, 300, 256, 1, 130]
+    w, wd, x, _ = _case(dev, kind, sum(counts), 512, 1024, experts=len(counts), seed=1)
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=dev)
+    want = torch.cat([x[off[e]:off[e + 1]].double() @ wd[e].t() for e in range(len(counts))])
+    assert _rel(pair_gemm(x, w, offsets=off), want) < (2 * ROUND if kind else ROUND)
+    act = torch.nn.functional.silu(want[:, :256]) * want[:, 256:]
+    assert _rel(pair_gemm(x, w, offsets=off, swiglu=True), act) < (4 * ROUND if kind else ROUND)
+    GemmStatus.check(dev)
+
+
+@pytest.mark.parametrize("kind", [None, "q4"])
+@pytest.mark.parametrize("m", [128, 129, 700, 2048])
+def test_rule_changes_no_result(dev, kind, m):
+    """``xgemm`` on either side of the rule, with rows and outputs that are not 16-byte aligned: the same values."""
+    from rmlx_b200.ops.quantized import pair_pays, xgemm
+    w, _, x, g = _case(dev, kind, m, 4096, 512, seed=2)
+    assert pair_pays(w.kind, 2048, 4096, 512) and not pair_pays(w.kind, 128, 4096, 512)
+    want = xgemm(x, w, bn=128)
+    assert torch.equal(xgemm(x, w), want)
+    wide = torch.zeros(m, 4104, dtype=torch.bfloat16, device=dev)
+    assert torch.equal(xgemm(x, w, out=wide[:, :4096]), want)
+    x2 = torch.zeros(m, 520, dtype=torch.bfloat16, device=dev)
+    x2[:, :512] = x
+    assert torch.equal(xgemm(x2[:, :512], w), want)
