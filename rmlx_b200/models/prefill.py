@@ -41,7 +41,7 @@ def _mm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = Non
     if w.kind == W_BF16:
         if _narrow(x, w):
             return narrow.narrow_gemm(x, w, residual=residual)
-        if x.shape[0] > 128 and pair_pays(W_BF16, x.shape[0], w.n, w.k):
+        if x.shape[0] > 128 and w.w.is_contiguous() and pair_pays(W_BF16, x.shape[0], w.n, w.k):
             return xgemm(x, w, residual=residual)         # SM pairs
         return gemm_bf16(x, w.w, residual=residual)
     return qmm(x, w, residual=residual)

@@ -21,10 +21,10 @@ _lib.register_cuda_sigs({
 
 def supported(w: LinearWeight) -> bool:
     """Whether the kernel takes this weight (``rmlx_narrow_supported``, in Python because it is asked before every projection):
-    bf16 scales, whole 16-row tiles, K a multiple of 512 (bf16 weights: 64), up to 256 experts."""
+    bf16 scales, contiguous rows, whole 16-row tiles, K a multiple of 512 (bf16 weights: 64), up to 256 experts."""
     k = w.k
     return (w.n % 16 == 0 and k % (64 if w.kind == W_BF16 else 512) == 0 and k > 0 and w.experts <= 256 and not w.scales_f16 and
-            w.w.dtype in (torch.bfloat16, torch.int32))
+            w.w.dtype in (torch.bfloat16, torch.int32) and w.w.is_contiguous())
 
 
 def pays(w: LinearWeight, rows: int) -> bool:

@@ -115,3 +115,17 @@ def test_refusals(dev):
         assert not narrow.supported(w)
         with pytest.raises(_lib.NativeError):
             narrow.narrow_gemm(torch.zeros(2, k, dtype=torch.bfloat16, device=dev), w)
+
+
+def test_weights_that_are_views(dev):
+    """A weight whose rows are not next to each other keeps the kernels that take a row stride."""
+    from rmlx_b200.models.prefill import _mm
+    from rmlx_b200.ops import narrow
+    from rmlx_b200.ops.weights import LinearWeight, W_BF16
+    g = torch.Generator(device=dev).manual_seed(5)
+    wide = torch.randn(4096, 1024, device=dev, generator=g).to(torch.bfloat16)
+    w = LinearWeight(W_BF16, wide[:, :512])
+    assert not narrow.supported(w)
+    for rows in (4, 1024):
+        x = torch.randn(rows, 512, device=dev, generator=g).to(torch.bfloat16)
+        assert _rel(_mm(x, w), x.double() @ w.w.double().t()) < 4e-3
