@@ -40,7 +40,7 @@ _CUDA_SIGS: Dict[str, tuple] = {
     "rmlx_flash_decode_part_ml_elems": ("iiii", "q"),
     "rmlx_flash_decode_ticket_elems": ("iii", "q"),
     "rmlx_flash_decode_paged": ("pppppppppiiiiiiifip", "i"),
-    "rmlx_rope_kv_write": ("pppppppppiiiiiiiip", "i"),
+    "rmlx_rope_kv_write": ("pippppppppiiiiiiiip", "i"),
     "rmlx_rope": ("pppppiiiiip", "i"),
     "rmlx_embedding": ("pppiiiip", "i"),
     "rmlx_rms_norm": ("pppppiifip", "i"),

@@ -1,6 +1,7 @@
 // RoPE on Q and K plus the paged KV-cache append, one launch for every head of every token.
 //
-// Input is the merged QKV projection output [T, (Hq + 2*Hkv) * HD]. Q heads are rotated and
+// Input is the merged QKV projection output [T, (Hq + 2*Hkv) * HD], bf16 or fp32 (decode rows: the
+// projection's sums reach the rotation unrounded and are rounded once, after it). Q heads are rotated and
 // written to q_out; K heads are rotated and written straight into their page slot; V heads are
 // copied into theirs. Positions, block tables and the token->sequence map are device buffers, so
 // the launch is shape-stable under CUDA graph replay while the cache grows.
@@ -15,7 +16,11 @@
 
 namespace rb {
 
-__global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv,
+__device__ __forceinline__ float rope_value(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float rope_value(float v) { return v; }
+
+template <class T>
+__global__ void rope_kv_write_kernel(const T* __restrict__ qkv,
                                      __nv_bfloat16* __restrict__ q_out,
                                      __nv_bfloat16* __restrict__ k_cache,
                                      __nv_bfloat16* __restrict__ v_cache,
@@ -35,8 +40,8 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv,
   // a block takes every gridDim.y-th head of its token (one head each for decode-sized launches,
   // a strip of heads for prompts, where one block per head would be mostly launch overhead)
   for (int head = blockIdx.y; head < Hq + 2 * Hkv; head += gridDim.y) {
-    const __nv_bfloat16* src = qkv + (size_t(tkn) * (Hq + 2 * Hkv) + head) * HD;
-    const float a = __bfloat162float(src[ia]), b = __bfloat162float(src[ib]);
+    const T* src = qkv + (size_t(tkn) * (Hq + 2 * Hkv) + head) * HD;
+    const float a = rope_value(src[ia]), b = rope_value(src[ib]);
     __nv_bfloat16* dst;
     if (head < Hq) {
       dst = q_out + (size_t(tkn) * Hq + head) * HD;
@@ -47,7 +52,7 @@ __global__ void rope_kv_write_kernel(const __nv_bfloat16* __restrict__ qkv,
       const bool is_k = head < Hq + Hkv;
       const int kvh = is_k ? head - Hq : head - Hq - Hkv;
       dst = (is_k ? k_cache : v_cache) + ((size_t(blk) * Hkv + kvh) * page + pos % page) * HD;
-      if (!is_k) { dst[ia] = src[ia]; dst[ib] = src[ib]; continue; }
+      if (!is_k) { dst[ia] = __float2bfloat16_rn(a); dst[ib] = __float2bfloat16_rn(b); continue; }
     }
     dst[ia] = __float2bfloat16_rn(a * c - b * s);
     dst[ib] = __float2bfloat16_rn(b * c + a * s);
@@ -78,19 +83,29 @@ using namespace rb;
 RB_BOUNDS_REGISTER("rope_kv.cu")
 
 
-extern "C" int rmlx_rope_kv_write(const void* qkv, void* q_out, void* k_cache, void* v_cache,
+template <class T>
+static int launch_rope_kv(const void* qkv, void* q_out, void* k_cache, void* v_cache, const int* block_table,
+                          const int* positions, const int* token_seq, const float* cos_t, const float* sin_t, int tokens,
+                          int Hq, int Hkv, int HD, int max_blocks, int page, int traditional, int pdl, cudaStream_t st) {
+  const int H = Hq + 2 * Hkv;
+  const int gy = tokens >= 128 ? (H + 17) / 18 : H;     // prompts: ~18 heads per block
+  return launch(rope_kv_write_kernel<T>, dim3(tokens, gy), dim3(HD / 2), 0, st, pdl != 0, static_cast<const T*>(qkv),
+                static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_cache),
+                static_cast<__nv_bfloat16*>(v_cache), block_table, positions, token_seq, cos_t, sin_t, Hq, Hkv, HD,
+                max_blocks, page, traditional);
+}
+
+// qkv bf16, or fp32 with qkv_f32.
+extern "C" int rmlx_rope_kv_write(const void* qkv, int qkv_f32, void* q_out, void* k_cache, void* v_cache,
                                   const int* block_table, const int* positions, const int* token_seq,
                                   const float* cos_t, const float* sin_t, int T, int Hq, int Hkv,
                                   int HD, int max_blocks, int page, int traditional, int pdl,
                                   cudaStream_t st) {
   if (T < 1 || HD % 2 || HD / 2 > 1024) return -2;
-  const int H = Hq + 2 * Hkv;
-  const int gy = T >= 128 ? (H + 17) / 18 : H;     // prompts: ~18 heads per block
-  return launch(rope_kv_write_kernel, dim3(T, gy), dim3(HD / 2), 0, st, pdl != 0,
-                static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out),
-                static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache),
-                block_table, positions, token_seq, cos_t, sin_t, Hq, Hkv, HD, max_blocks, page,
-                traditional);
+  return qkv_f32 ? launch_rope_kv<float>(qkv, q_out, k_cache, v_cache, block_table, positions, token_seq, cos_t, sin_t, T,
+                                         Hq, Hkv, HD, max_blocks, page, traditional, pdl, st)
+                 : launch_rope_kv<__nv_bfloat16>(qkv, q_out, k_cache, v_cache, block_table, positions, token_seq, cos_t,
+                                                 sin_t, T, Hq, Hkv, HD, max_blocks, page, traditional, pdl, st);
 }
 
 extern "C" int rmlx_rope(const void* x, void* out, const int* positions, const float* cos_t,

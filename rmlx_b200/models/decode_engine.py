@@ -31,6 +31,7 @@ from ..kv.paged import PagedKvCache
 from ..runtime.graph import GraphCache, bucket_for
 from ..ops import decode as D
 from ..ops import narrow
+from ..ops.weights import W_Q4
 from .transformer import TransformerModel
 
 
@@ -221,7 +222,8 @@ class CachedDecode(DecodeEngineBase):
         bf = dict(dtype=torch.bfloat16, device=dev)
         self.h = torch.zeros(B, D_, **bf)
         self.h2 = torch.zeros(B, D_, **bf)
-        self.qkv = torch.zeros(B, (hq + 2 * hkv) * hd, **bf)
+        # q, k and v stay in 32 bits until they are rotated (the 8-bit cache's append takes bf16)
+        self.qkv = torch.zeros(B, (hq + 2 * hkv) * hd, device=dev, dtype=torch.bfloat16 if cache.quantized else torch.float32)
         self.q = torch.zeros(B, hq, hd, **bf)
         self.attn = torch.zeros(B, hq, hd, **bf)
         lib = _lib.cuda()
@@ -288,11 +290,10 @@ class CachedDecode(DecodeEngineBase):
         block_table, q, attn = self.block_table[:nb], self.q[:nb], self.attn[:nb]
         D.embedding(w.embed, tokens, out=self.h[:nb], pdl=False)
         h, h2 = self.h[:nb], self.h2[:nb]
-        # several rows on 4-bit weights: the projection runs on the tensor-core mat-vec (eight rows
-        # per pass) and RoPE + the KV append follow as their own small kernel
-        fuse_rope = self.fuse_rope and not (nb >= 2 and (w.layers[0].wqkv.kind == 1 or D._several(nb, w.layers[0].wqkv, h)))
         for li, lw in enumerate(w.layers):
-            if fuse_rope:
+            # several rows: the projection runs on a kernel that takes eight rows per pass (ops/narrow.py, or the tensor-core
+            # mat-vec of 4-bit weights), and RoPE + the KV append follow as their own small kernel on its fp32 sums
+            if self.fuse_rope and not (nb >= 2 and (lw.wqkv.kind == W_Q4 or D._several(nb, lw.wqkv, h))):
                 D.rms_qkv_rope(h, lw.wqkv, lw.norm1, eps, q, self.cache.k[li], self.cache.v[li],
                                block_table, positions, m.cos, m.sin, m.hq, m.hkv,
                                traditional=cfg.rope_traditional, pdl=pdl)

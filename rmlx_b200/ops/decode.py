@@ -477,14 +477,15 @@ def rope_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor,
                   token_seq: Optional[torch.Tensor] = None, traditional: bool = False,
                   pdl: bool = False, k_sb: Optional[torch.Tensor] = None,
                   v_sb: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """RoPE(Q) -> q_out, RoPE(K) and V -> their page slots. qkv [T, (Hq+2Hkv)*D] bf16. With
-    ``k_sb`` / ``v_sb`` the caches are in the 8-bit format: K and V are quantised as they are
-    written."""
+    """RoPE(Q) -> q_out, RoPE(K) and V -> their page slots. qkv [T, (Hq+2Hkv)*D] bf16 or fp32 (rounded
+    once, after the rotation). With ``k_sb`` / ``v_sb`` the caches are in the 8-bit format: K and V are
+    quantised as they are written, from bf16."""
     _lib.require_cuda_tensor(qkv, q_out, k_cache, v_cache, block_table, positions, cos, sin)
     t = qkv.shape[0]
     d = k_cache.shape[3]
     assert qkv.is_contiguous() and qkv.shape[1] == (hq + 2 * hkv) * d
     assert positions.dtype == torch.int32 and cos.dtype == torch.float32
+    assert qkv.dtype == torch.bfloat16 or (qkv.dtype == torch.float32 and k_sb is None)
     if k_sb is not None:
         assert k_cache.dtype == torch.uint8 and v_sb is not None
         rc = _lib.cuda().rmlx_rope_kv_write_q8(
@@ -495,7 +496,7 @@ def rope_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor,
         _lib.check(rc, "rope_kv_write_q8")
         return q_out
     rc = _lib.cuda().rmlx_rope_kv_write(
-        qkv.data_ptr(), q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+        qkv.data_ptr(), int(qkv.dtype == torch.float32), q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
         block_table.data_ptr(), positions.data_ptr(), _lib.ptr(token_seq), cos.data_ptr(),
         sin.data_ptr(), t, hq, hkv, d, block_table.stride(0), k_cache.shape[2], int(traditional),
         int(pdl), _lib.stream_ptr())

@@ -319,3 +319,44 @@ def test_decode_with_8bit_kv_cache(dev, use_graph):
         assert rel < 6e-2, (i, rel)
         if i + 1 < steps:
             eng.set_next_tokens([toks[i + 1]])
+
+
+@pytest.mark.parametrize("quant", [None, "q8", "q4"])
+@pytest.mark.parametrize("traditional", [False, True])
+def test_several_rows_round_keys_once(dev, quant, traditional):
+    """Several rows project with one kernel and rotate with the next: keys and queries are rounded to bf16 once, after the
+    rotation. Per element: that rounding (2^-8 of the value at most) and the projection's own error, for 4-bit and 8-bit weights the
+    fp16 rounding of x times the norm's weight (2^-11 per term at most, so 2.1e-4 of the root mean square; five times that),
+    for bf16 weights fp32 sums (2e-5). A second rounding before the rotation moves an element by up to 2^-8 of its pair's other half."""
+    rows, at = 5, 3
+    cfg = TransformerConfig(hidden_size=512, num_heads=8, num_kv_heads=4, head_dim=64, num_layers=1, vocab_size=256,
+                            max_seq_len=64, rope_theta=1e4, rope_traditional=traditional,
+                            ff_type=FeedForwardType.gated(512), name="one-layer").validate()
+    model = TransformerModel(from_state_dict(cfg, random_state_dict(cfg, 0), device=dev, quant=quant))
+    cache = model.new_cache(16, max_seqs=rows)
+    for s in range(rows):
+        cache.add_sequence(s)
+        cache.reserve(s, at)
+        cache.commit(s, at)
+    eng = CachedDecode(model, cache, max_batch=rows)
+    tokens = [3, 50, 71, 9, 200]
+    eng.bind(range(rows), tokens)
+    eng.reserve(1)
+    eng.step()
+    torch.cuda.synchronize()
+    lw = model.w.layers[0]
+    x = model.w.embed[torch.tensor(tokens, device=dev)].double()
+    x = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + cfg.rms_norm_eps) * lw.norm1.double()
+    qkv = (x @ lw.wqkv.dequantized().double().t()).view(rows, -1, 64)
+    c, s = model.cos[at].double(), model.sin[at].double()
+
+    def rotate(v):
+        a, b = (v[..., 0::2], v[..., 1::2]) if traditional else (v[..., :32], v[..., 32:])
+        r = (a * c - b * s, b * c + a * s)
+        return torch.stack(r, -1).flatten(-2) if traditional else torch.cat(r, -1)
+
+    pages = [cache.manager.block_table(s)[0] for s in range(rows)]
+    k, v = cache.k[0][pages, :, at].double(), cache.v[0][pages, :, at].double()
+    for got, want in ((eng.q.double(), rotate(qkv[:, :8])), (k, rotate(qkv[:, 8:12])), (v, qkv[:, 12:])):
+        slack = (1.1e-3 if quant else 2e-5) * float(want.pow(2).mean().sqrt())
+        assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + slack).all())
