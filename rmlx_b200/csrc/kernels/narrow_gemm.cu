@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(NwShape<KIND, T>::THREADS, 1) narrow_gemm_kern
 }
 
 // Position list of the grouped form: order[offsets[e] ..] are the (row, slot) pairs that chose expert e. One block; pairs
-// of an expert in no particular order (every row of x is a column of its own, so results don't depend on it).
+// of an expert in no particular order (every row of x is a column of its own, so results don't depend on it). A choice outside
+// [0, E) (a row of NaN logits has no largest one: decode_moe.cu) is in no expert's list, and the combination skips it.
 __global__ void __launch_bounds__(1024) narrow_group_kernel(const int* __restrict__ idx, int pairs, int E,
                                                             int* __restrict__ offsets, int* __restrict__ order) {
   __shared__ int count[kNwMaxExperts], start[kNwMaxExperts + 1];
@@ -544,7 +545,8 @@ __global__ void __launch_bounds__(1024) narrow_group_kernel(const int* __restric
   for (int i = threadIdx.x; i < E; i += blockDim.x) count[i] = 0;
   __syncthreads();
   pdl_wait();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) atomicAdd(count + idx[i], 1);
+  for (int i = threadIdx.x; i < pairs; i += blockDim.x)
+    if (const int e = idx[i]; unsigned(e) < unsigned(E)) atomicAdd(count + e, 1);
   __syncthreads();
   if (threadIdx.x < 32) {
     int base = 0;
@@ -562,11 +564,14 @@ __global__ void __launch_bounds__(1024) narrow_group_kernel(const int* __restric
   __syncthreads();
   for (int i = threadIdx.x; i <= E; i += blockDim.x) offsets[i] = start[i];
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) order[atomicAdd(start + idx[i], 1)] = i;
+  for (int i = threadIdx.x; i < pairs; i += blockDim.x)
+    if (const int e = idx[i]; unsigned(e) < unsigned(E)) order[atomicAdd(start + e, 1)] = i;
 }
 
-// out[t] = residual[t] + sum_s w[t, s] y[t k + s], slots in order, y in fp32.
-__global__ void __launch_bounds__(256) narrow_combine_kernel(const float* __restrict__ y, const float* __restrict__ wts,
+// out[t] = residual[t] + sum_s w[t, s] y[t k + s], slots in order, y in fp32; slots whose choice idx[t, s] is no expert are
+// skipped (nobody has written their y).
+__global__ void __launch_bounds__(256) narrow_combine_kernel(const float* __restrict__ y, const int* __restrict__ idx, int E,
+                                                             const float* __restrict__ wts,
                                                              const __nv_bfloat16* __restrict__ residual, int res_stride,
                                                              __nv_bfloat16* __restrict__ out, int out_stride, int top_k, int D) {
   const int row = blockIdx.y, c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -580,6 +585,7 @@ __global__ void __launch_bounds__(256) narrow_combine_kernel(const float* __rest
   }
 #pragma unroll 8
   for (int s = 0; s < top_k; ++s) {
+    if (unsigned(idx[row * top_k + s]) >= unsigned(E)) continue;
     const float w = wts[row * top_k + s];
     const float4 v = *reinterpret_cast<const float4*>(y + size_t(row * top_k + s) * D + c);
     a[0] = fmaf(w, v.x, a[0]); a[1] = fmaf(w, v.y, a[1]); a[2] = fmaf(w, v.z, a[2]); a[3] = fmaf(w, v.w, a[3]);
@@ -693,9 +699,9 @@ extern "C" int rmlx_narrow_group(const int* idx, int pairs, int E, int* offsets,
   return launch(narrow_group_kernel, dim3(1), dim3(threads), 0, st, pdl != 0, idx, pairs, E, offsets, order);
 }
 
-extern "C" int rmlx_narrow_combine(const float* y, const float* wts, const void* residual, int res_stride, void* out,
+extern "C" int rmlx_narrow_combine(const float* y, const int* idx, int E, const float* wts, const void* residual, int res_stride, void* out,
                                    int out_stride, int rows, int top_k, int D, int pdl, cudaStream_t st) {
   if (rows < 1 || D % 4) return -2;
-  return launch(narrow_combine_kernel, dim3((D / 4 + 255) / 256, rows), dim3(256), 0, st, pdl != 0, y, wts,
+  return launch(narrow_combine_kernel, dim3((D / 4 + 255) / 256, rows), dim3(256), 0, st, pdl != 0, y, idx, E, wts,
                 static_cast<const __nv_bfloat16*>(residual), res_stride, static_cast<__nv_bfloat16*>(out), out_stride, top_k, D);
 }

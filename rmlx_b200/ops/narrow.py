@@ -15,7 +15,7 @@ _lib.register_cuda_sigs({
     "rmlx_narrow_supported": ("iii", "i"),
     "rmlx_narrow_gemm": ("ippppiippipfpipiiiiiiiiip", "i"),
     "rmlx_narrow_group": ("piippip", "i"),
-    "rmlx_narrow_combine": ("pppipiiiiip", "i"),
+    "rmlx_narrow_combine": ("ppippipiiiiip", "i"),
 })
 
 
@@ -80,7 +80,8 @@ def narrow_gemm(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor]
 
 def group_pairs(idx: torch.Tensor, experts: int, offsets: Optional[torch.Tensor] = None, order: Optional[torch.Tensor] = None,
                 pdl: bool = False):
-    """Pairs (row * k + slot) by chosen expert: (offsets [E + 1], order [rows * k]), int32."""
+    """Pairs (row * k + slot) by chosen expert: (offsets [E + 1], order [rows * k]), int32. Choices outside [0, experts) are in
+    no list: offsets[E] counts the others."""
     n = idx.numel()
     if offsets is None:
         offsets = torch.empty(experts + 1, dtype=torch.int32, device=idx.device)
@@ -91,14 +92,14 @@ def group_pairs(idx: torch.Tensor, experts: int, offsets: Optional[torch.Tensor]
     return offsets, order
 
 
-def combine(y: torch.Tensor, wts: torch.Tensor, residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-            pdl: bool = False) -> torch.Tensor:
-    """out[t] = residual[t] + sum over slots of wts[t, slot] * y[t k + slot], y fp32."""
+def combine(y: torch.Tensor, idx: torch.Tensor, experts: int, wts: torch.Tensor, residual: Optional[torch.Tensor] = None,
+            out: Optional[torch.Tensor] = None, pdl: bool = False) -> torch.Tensor:
+    """out[t] = residual[t] + sum over the slots whose choice idx[t, slot] is an expert of wts[t, slot] * y[t k + slot], y fp32."""
     t, k = wts.shape
     d = y.shape[1]
     if out is None:
         out = torch.empty(t, d, dtype=torch.bfloat16, device=y.device)
-    _lib.check(_lib.cuda().rmlx_narrow_combine(y.data_ptr(), wts.data_ptr(), _lib.ptr(residual),
+    _lib.check(_lib.cuda().rmlx_narrow_combine(y.data_ptr(), idx.data_ptr(), experts, wts.data_ptr(), _lib.ptr(residual),
                                                0 if residual is None else residual.stride(0), out.data_ptr(), out.stride(0), t, k,
                                                d, int(pdl), _lib.stream_ptr()), "narrow_combine")
     return out
@@ -130,11 +131,11 @@ def expert_ffn(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, gate_up: L
                norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6, residual: Optional[torch.Tensor] = None,
                out: Optional[torch.Tensor] = None, scratch: Optional[ExpertScratch] = None, pdl: bool = False) -> torch.Tensor:
     """residual + sum over slots of wts * down_e(silu(gate_e xn) * up_e xn), e = idx[row, slot], xn = rmsnorm(x; norm_w):
-    every expert's weights are read once for all rows that chose it."""
+    every expert's weights are read once for all rows that chose it. Slots whose choice is no expert add nothing."""
     t, k = idx.shape
     pairs = t * k
     s = scratch or ExpertScratch(t, k, gate_up, down)
     offsets, order = group_pairs(idx, gate_up.experts, s.offsets, s.order[:pairs], pdl=pdl)
     act = narrow_gemm(x, gate_up, norm_w, eps, out=s.act[:pairs], swiglu=True, offsets=offsets, order=order, x_div=k, rows=pairs, pdl=pdl)
     y = narrow_gemm(act, down, out=s.y[:pairs], offsets=offsets, order=order, rows=pairs, pdl=pdl)
-    return combine(y, wts, residual, out, pdl=pdl)
+    return combine(y, idx, gate_up.experts, wts, residual, out, pdl=pdl)

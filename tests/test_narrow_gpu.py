@@ -129,3 +129,30 @@ def test_weights_that_are_views(dev):
     for rows in (4, 1024):
         x = torch.randn(rows, 512, device=dev, generator=g).to(torch.bfloat16)
         assert _rel(_mm(x, w), x.double() @ w.w.double().t()) < 4e-3
+
+
+@pytest.mark.parametrize("experts", [12, 256])
+@pytest.mark.parametrize("bad", [-1, 0, 0x7fffffff])
+def test_choices_that_are_no_expert(dev, experts, bad):
+    """A slot whose choice is outside [0, E) (0 stands for E itself; a row of NaN logits gives E or the largest number) adds
+    nothing and changes no other row: results are equal bit for bit to those of a batch in which it carries no weight."""
+    from rmlx_b200.ops import narrow
+    d, inner, rows, k = 512, 512, 5, 4
+    gu, _, x, g = _case(dev, "q4", 2 * inner, d, rows, experts=experts, seed=6)
+    dn, _, _, _ = _case(dev, "q4", d, inner, 1, experts=experts, seed=7)
+    idx = torch.randint(0, experts, (rows, k), device=dev, generator=g).to(torch.int32)
+    wts = torch.rand(rows, k, device=dev, generator=g)
+    res = torch.randn(rows, d, device=dev, generator=g).to(torch.bfloat16)
+    scratch = narrow.ExpertScratch(rows, k, gu, dn)
+    scratch.act.fill_(float("nan")), scratch.y.fill_(float("nan"))
+    none = wts.clone()
+    none[1], none[3, 2] = 0.0, 0.0
+    want = narrow.expert_ffn(x, idx, none, gu, dn, residual=res)
+    out = idx.clone()
+    out[1], out[3, 2] = bad or experts, bad or experts
+    got = narrow.expert_ffn(x, out, wts, gu, dn, residual=res, scratch=scratch)
+    assert torch.equal(got, want) and torch.equal(got[1], res[1])
+    offsets, order = narrow.group_pairs(out, experts)
+    assert int(offsets[-1]) == rows * k - k - 1
+    flat = out.flatten()[order[:int(offsets[-1])].long()]
+    assert torch.equal(offsets[1:].long(), torch.bincount(flat.long(), minlength=experts).cumsum(0))
