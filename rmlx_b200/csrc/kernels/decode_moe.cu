@@ -22,7 +22,8 @@ constexpr int kMaxExperts = 256;
 constexpr int kMaxTopK = 8;
 
 // Softmax over E logits held 8-per-lane, then k rounds of warp arg-max (ties: lowest index wins),
-// weights renormalised to sum 1. Executed by one full warp for one token.
+// weights renormalised to sum 1. Executed by one full warp for one token. NaN logits have no largest one: such a row's choices
+// are numbers outside [0, E), which are not counted and which every user of the choices skips.
 __device__ __forceinline__ void warp_topk(const float* logits, const float* bias, int E, int k,
                                           int* out_idx, float* out_w, int* counts) {
   const int lane = threadIdx.x & 31;
@@ -69,7 +70,7 @@ __device__ __forceinline__ void warp_topk(const float* logits, const float* bias
   if (lane < k) {
     out_idx[lane] = sel_e;
     out_w[lane] = sel_w / wsum;
-    if (counts) atomicAdd(counts + sel_e, 1);
+    if (counts && unsigned(sel_e) < unsigned(E)) atomicAdd(counts + sel_e, 1);
   }
 }
 

@@ -11,21 +11,23 @@
 
 namespace rb {
 
-// One warp per (token, slot) pair. cursors[E] must be zero on entry.
+// One warp per (token, slot) pair. cursors[E] must be zero on entry. A pair whose choice is no expert (a row of NaN logits) gets
+// row -1 and no copy; the combine skips it.
 __global__ void __launch_bounds__(256)
 moe_scatter_rows_kernel(const __nv_bfloat16* __restrict__ x, int x_stride,
                         const int* __restrict__ topk_idx, const int* __restrict__ offsets,
                         int* __restrict__ cursors, __nv_bfloat16* __restrict__ xs,
-                        int* __restrict__ row_of_pair, int pairs, int top_k, int D) {
+                        int* __restrict__ row_of_pair, int pairs, int top_k, int D, int E) {
   const int p = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p >= pairs) return;
-  int pos = 0;
+  int pos = -1;
   if (lane == 0) {
     const int e = topk_idx[p];
-    pos = offsets[e] + atomicAdd(cursors + e, 1);
+    if (unsigned(e) < unsigned(E)) pos = offsets[e] + atomicAdd(cursors + e, 1);
     row_of_pair[p] = pos;
   }
   pos = __shfl_sync(0xffffffffu, pos, 0);
+  if (pos < 0) return;
   const uint4* src = reinterpret_cast<const uint4*>(x + size_t(p / top_k) * x_stride);
   uint4* dst = reinterpret_cast<uint4*>(xs + size_t(pos) * D);
   for (int i = lane; i < D / 8; i += 32) dst[i] = src[i];
@@ -73,7 +75,7 @@ extern "C" int rmlx_moe_scatter_rows(const void* x, int x_stride, const int* top
   const int pairs = T * top_k;
   moe_scatter_rows_kernel<<<(pairs + 7) / 8, 256, 0, st>>>(
       static_cast<const __nv_bfloat16*>(x), x_stride, topk_idx, offsets, cursors,
-      static_cast<__nv_bfloat16*>(xs), row_of_pair, pairs, top_k, D);
+      static_cast<__nv_bfloat16*>(xs), row_of_pair, pairs, top_k, D, E);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -297,3 +297,30 @@ def test_serving_engine_warm_up_and_logit_monitor_on_device(dev):
     assert int(eng._engine.block_table[len(eng._engine.seq_ids):].abs().sum()) == 0
     assert eng.guard.checks >= 3 and eng.guard_fallbacks == 0 and eng.guard.nan_events == 0
     GemmStatus.check(dev)
+
+
+@pytest.mark.parametrize("experts", [12, 256])
+@pytest.mark.parametrize("kind", [None, "q4"])
+def test_nan_row_has_no_expert(dev, experts, kind):
+    """A token of NaN logits is counted for no expert, and the other tokens' results stay as they are without it: the choice, the
+    rows sorted by expert and the combination."""
+    from rmlx_b200.ops import decode as D
+    from rmlx_b200.ops.grouped import moe_prefill_ffn
+    from rmlx_b200.ops.weights import LinearWeight
+    g = torch.Generator(device=dev).manual_seed(11)
+    t, k, d, inner, nan = 70, 4, 512, 512, 33
+    gu = LinearWeight.random(2 * inner, d, kind, dev, experts=experts, generator=g)
+    dn = LinearWeight.random(d, inner, kind, dev, experts=experts, generator=g)
+    x = torch.randn(t, d, device=dev, generator=g).to(torch.bfloat16)
+    logits = torch.randn(t, experts, device=dev, generator=g)
+    whole = D.topk_route(logits, k)
+    logits[nan] = float("nan")
+    idx, wts, counts, offsets = D.topk_route(logits, k)
+    kept = [i for i in range(t) if i != nan]
+    assert torch.equal(idx[kept], whole[0][kept]) and bool(((idx[nan] < 0) | (idx[nan] >= experts)).all())
+    assert torch.equal(counts.long(), torch.bincount(idx[kept].flatten().long(), minlength=experts))
+    assert torch.equal(offsets[1:].long(), counts.long().cumsum(0))
+    res = torch.randn(t, d, device=dev, generator=g).to(torch.bfloat16)
+    got = moe_prefill_ffn(x, idx, wts, offsets, gu, dn, residual=res)
+    want = moe_prefill_ffn(x, whole[0], whole[1], whole[3], gu, dn, residual=res)
+    assert torch.equal(got[kept], want[kept]) and torch.equal(got[nan], res[nan])
