@@ -661,6 +661,7 @@ extern "C" int rmlx_narrow_gemm(int w_kind, const void* w, const void* scales, c
   const int split = w_kind == 0 && norm != nullptr;      // twice the tiles for the same rows
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return -2;
   if (norm && (reinterpret_cast<uintptr_t>(norm) & 15)) return -2;
+  if (w_kind && (!scales || !biases || ((reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(biases)) & 15))) return -2;
   if (ks < 0 || ks > 8 || (ks & (ks - 1))) return -2;
   NwParams p = {};
   p.w = static_cast<const uint8_t*>(w);

@@ -483,6 +483,11 @@ extern "C" int rmlx_qmv_mma_supported(int K, int cols, int rows_per_block) {
   return smem <= 200 * 1024;
 }
 
+// The bulk copies read rows of the packed words, scales and biases from 16-byte addresses.
+static bool qmv_tables_ok(const void* w, const void* scales, const void* biases) {
+  return !((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(biases)) & 15);
+}
+
 template <int NCOLS, int TILES, bool F32>
 static int launch_rms_qmv(const void* w, const void* sc, const void* bi, const void* x, int x_stride,
                           const void* norm_w, float eps, const void* res, int res_stride, void* out,
@@ -505,7 +510,7 @@ extern "C" int rmlx_rms_qmv_mma(const void* w, const void* scales, const void* b
                                 int x_stride, const void* norm_w, float eps, const void* residual,
                                 int res_stride, void* out, int out_stride, int out_f32, int B, int N,
                                 int K, int pdl, cudaStream_t st) {
-  if (B < 1 || B > 8 || N < 1) return -2;
+  if (B < 1 || B > 8 || N < 1 || !qmv_tables_ok(w, scales, biases)) return -2;
   const bool big = N > 16384 && rmlx_qmv_mma_supported(K, B, 32);
   if (!rmlx_qmv_mma_supported(K, B, big ? 32 : 16)) return -2;
 #define RB_QMV(NC)                                                                                   \
@@ -527,7 +532,7 @@ extern "C" int rmlx_moe_gate_up_q4_mma(const void* w, const void* scales, const 
                                        int top_k, int I, int K, int expert_base, int experts_local,
                                        int pdl, cudaStream_t st) {
   constexpr int TILES = 2;
-  if (B < 1 || top_k < 1 || top_k > kQMaxTopK || I < 1) return -2;
+  if (B < 1 || top_k < 1 || top_k > kQMaxTopK || I < 1 || !qmv_tables_ok(w, scales, biases)) return -2;
   if (!rmlx_qmv_mma_supported(K, 1, 16 * TILES)) return -2;
   const WTile wt{K};
   const size_t smem = ((wt.bytes(16 * TILES) + 127) & ~size_t(127)) + QStage::col_bytes(K);
@@ -555,7 +560,7 @@ extern "C" int rmlx_moe_down_q4_mma(const void* w, const void* scales, const voi
                                     void* out, int out_stride, int out_f32, int B, int top_k, int N,
                                     int I, int expert_base, int experts_local, int pdl,
                                     cudaStream_t st) {
-  if (B < 1 || N < 1 || !rmlx_moe_down_q4_mma_supported(I, top_k)) return -2;
+  if (B < 1 || N < 1 || !rmlx_moe_down_q4_mma_supported(I, top_k) || !qmv_tables_ok(w, scales, biases)) return -2;
   const WTile wt{I};
   const size_t smem = (((wt.bytes(16) + 127) & ~size_t(127)) + QStage::col_bytes(I)) * top_k;
   const int gx = (N + 15) / 16;

@@ -119,6 +119,11 @@ def _several(b: int, w: LinearWeight, x: torch.Tensor) -> bool:
             x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
 
 
+def _copied_whole(w: LinearWeight) -> bool:
+    """Whether the bulk copies of the tensor-core mat-vec can read this weight's tables (16-byte addresses)."""
+    return (w.w.data_ptr() | w.scales.data_ptr() | w.biases.data_ptr()) % 16 == 0
+
+
 def _wargs(w: LinearWeight):
     return (w.kernel_kind, w.w.data_ptr(), _lib.ptr(w.scales), _lib.ptr(w.biases))
 
@@ -142,7 +147,7 @@ def rms_gemv(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor] = 
     # MMA's columns for the price of one, while the CUDA-core kernels pay their unpacking FMAs per
     # row (measured on B200, 9216x4096: four rows 29.5 us streaming; the weights are read once
     # either way).
-    mma_rows = (w.kind == W_Q4 and not w.scales_f16 and b >= 2 and q4_path() != "scalar" and
+    mma_rows = (w.kind == W_Q4 and not w.scales_f16 and b >= 2 and q4_path() != "scalar" and _copied_whole(w) and
                 bool(lib.rmlx_qmv_mma_supported(k, min(8, b), 16)))
     if _stream("gemv", w) and not mma_rows:
         done = True
@@ -160,7 +165,7 @@ def rms_gemv(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor] = 
             _lib.check(rc, "sg_rms_gemv")
         if done:
             return out
-    if mma_rows or (w.kind == W_Q4 and not w.scales_f16 and q4_path() == "mma" and
+    if mma_rows or (w.kind == W_Q4 and not w.scales_f16 and q4_path() == "mma" and _copied_whole(w) and
                     lib.rmlx_qmv_mma_supported(k, min(8, b), 16)):
         for b0 in range(0, b, 8):
             bb = min(8, b - b0)

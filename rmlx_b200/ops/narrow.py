@@ -21,10 +21,17 @@ _lib.register_cuda_sigs({
 
 def supported(w: LinearWeight) -> bool:
     """Whether the kernel takes this weight (``rmlx_narrow_supported``, in Python because it is asked before every projection):
-    bf16 scales, contiguous rows, whole 16-row tiles, K a multiple of 512 (bf16 weights: 64), up to 256 experts."""
-    k = w.k
-    return (w.n % 16 == 0 and k % (64 if w.kind == W_BF16 else 512) == 0 and k > 0 and w.experts <= 256 and not w.scales_f16 and
-            w.w.dtype in (torch.bfloat16, torch.int32) and w.w.is_contiguous())
+    whole 16-row tiles, K a multiple of 512 (bf16 weights: 64), up to 256 experts, and every table contiguous and at a 16-byte
+    address, as the copies of 16 bytes need it (views that are not keep the kernels that take them)."""
+    t, s, b = w.w, w.scales, w.biases
+    shape = t.shape
+    if shape[-2] % 16 or (len(shape) == 3 and shape[0] > 256) or not t.is_contiguous():
+        return False
+    if w.kind == W_BF16:
+        return t.dtype == torch.bfloat16 and shape[-1] % 64 == 0 and shape[-1] > 0 and t.data_ptr() % 16 == 0
+    return (t.dtype == torch.int32 and shape[-1] % (64 if w.kind == W_Q4 else 128) == 0 and shape[-1] > 0 and s is not None and
+            b is not None and s.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and s.is_contiguous() and
+            b.is_contiguous() and (t.data_ptr() | s.data_ptr() | b.data_ptr()) % 16 == 0)
 
 
 def pays(w: LinearWeight, rows: int) -> bool:

@@ -156,3 +156,21 @@ def test_choices_that_are_no_expert(dev, experts, bad):
     assert int(offsets[-1]) == rows * k - k - 1
     flat = out.flatten()[order[:int(offsets[-1])].long()]
     assert torch.equal(offsets[1:].long(), torch.bincount(flat.long(), minlength=experts).cumsum(0))
+
+
+@pytest.mark.parametrize("kind", ["q4", "q8"])
+def test_scales_at_odd_addresses(dev, kind):
+    """Several rows against weights whose scales and biases are views at an odd offset take the kernels that read those."""
+    from rmlx_b200.ops import decode as D
+    from rmlx_b200.ops import narrow
+    from rmlx_b200.ops.weights import LinearWeight
+    w, wd, x, _ = _case(dev, kind, 2048, 1024, 4, seed=8)
+
+    def shifted(t):
+        room = torch.zeros(t.numel() + 8, dtype=t.dtype, device=dev)
+        return room[3:3 + t.numel()].view(t.shape).copy_(t)
+
+    odd = LinearWeight(w.kind, w.w, shifted(w.scales), shifted(w.biases))
+    assert narrow.supported(w) and not narrow.supported(odd)
+    # the per-row kernels multiply in fp16 (2^-11 per product)
+    assert _rel(D.rms_gemv(x, odd, out_dtype=torch.float32), x.double() @ wd.t()) < 2e-3
