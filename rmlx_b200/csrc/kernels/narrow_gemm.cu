@@ -158,13 +158,17 @@ __global__ void __launch_bounds__(NwShape<KIND, T>::THREADS, 1) narrow_gemm_kern
 
   if (p.offsets) {
     pdl_wait();
-    for (int i = threadIdx.x; i <= p.E; i += S::THREADS) s_off[i] = p.offsets[i];
+    for (int i = threadIdx.x; i <= p.E; i += S::THREADS) {
+      const int o = p.offsets[i];
+      s_off[i] = RB_BOUNDS(o, p.M + 1) ? o : 0;
+    }
     __syncthreads();
     if (warp == 0) {       // items before every expert: a scan over 32 experts at a time
       int base = 0;
       for (int e0 = 0; e0 < p.E; e0 += 32) {
         const int e = e0 + lane;
-        const int mine = e < p.E ? (s_off[e + 1] - s_off[e] + rows - 1) / rows * blocks_n : 0;
+        const int n = e < p.E ? s_off[e + 1] - s_off[e] : 0;
+        const int mine = RB_BOUNDS(n, p.M + 1) ? (n + rows - 1) / rows * blocks_n : 0;
         int sum = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
@@ -250,7 +254,9 @@ __global__ void __launch_bounds__(NwShape<KIND, T>::THREADS, 1) narrow_gemm_kern
   auto out_row = [&](int e, int mt, int i) {
     const int pos = s_off[e] + mt * rows + i;
     if (i >= rows || pos >= s_off[e + 1]) return -1;
-    return p.order ? __ldg(p.order + pos) : pos;
+    if (!p.order) return pos;
+    const int row = __ldg(p.order + pos);
+    return RB_BOUNDS(row, p.M) ? row : -1;
   };
   // unit u of the buffer: tile u / SLG of the rows of x (split: the second half of the tiles repeats the first half's rows),
   // group u % SLG of the slab. A lane holds the 16 values that its fragments need: row g, share t.
@@ -643,6 +649,7 @@ static int launch_narrow_t(const NwParams& p, int T, int passes, int ks, int pdl
 }  // namespace rb
 
 using namespace rb;
+RB_BOUNDS_REGISTER("narrow_gemm.cu")
 
 // Whether the kernel takes a weight of this kind, N rows (stacked gate and up rows included) and K columns: whole ring
 // stages, 16-byte rows of scales, whole 16-row tiles.

@@ -119,7 +119,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
   pdl_wait();
   if (GROUPED)
-    for (int i = threadIdx.x; i <= E; i += blockDim.x) s_off[i] = offsets[i];
+    for (int i = threadIdx.x; i <= E; i += blockDim.x) {
+      const int o = offsets[i];
+      s_off[i] = RB_BOUNDS(o, M + 1) ? o : 0;
+    }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -128,7 +131,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       int acc = 0;
       for (int e = 0; e < E; ++e) {
         s_tprefix[e] = acc;
-        acc += ((s_off[e + 1] - s_off[e] + 2 * kPairRows - 1) / (2 * kPairRows)) * tiles_n;
+        const int n = s_off[e + 1] - s_off[e];
+        if (RB_BOUNDS(n, M + 1)) acc += ((n + 2 * kPairRows - 1) / (2 * kPairRows)) * tiles_n;
       }
       s_tprefix[E] = acc;
     }
@@ -387,6 +391,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUten
 }  // namespace rb
 
 using namespace rb;
+RB_BOUNDS_REGISTER("pair_gemm.cu")
 
 // Shapes of the pair kernel: whole 32-column pieces (SwiGLU, grouped: whole tiles), 16-byte rows.
 extern "C" int rmlx_pair_gemm_supported(int w_kind, int N, int K, int ldc, int grouped, int swiglu) {

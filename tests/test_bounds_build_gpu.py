@@ -76,6 +76,36 @@ torch.cuda.synchronize()
 rec = _lib.bounds_status()
 assert rec is not None and rec[0] == "misc.cu" and rec[2:] == (40, 32), rec
 
+# grouped products: an offset past the rows ends its expert early, a position past them has no row
+from rmlx_b200.ops import narrow
+from rmlx_b200.ops.quantized import pair_gemm
+we = LinearWeight.random(256, 512, "q4", dev, experts=3, generator=g)
+xe = torch.randn(6, 512, device=dev, generator=g).to(torch.bfloat16)
+good = torch.tensor([0, 2, 3, 6], dtype=torch.int32, device=dev)
+want = narrow.narrow_gemm(xe, we, offsets=good)
+pairs = pair_gemm(xe, we, offsets=good)
+torch.cuda.synchronize()
+assert _lib.bounds_status() is None
+out = torch.zeros_like(want)
+narrow.narrow_gemm(xe, we, out=out, offsets=torch.tensor([0, 2, 3, 9], dtype=torch.int32, device=dev))
+torch.cuda.synchronize()
+rec = _lib.bounds_status()
+assert rec is not None and rec[0] == "narrow_gemm.cu" and rec[3] == 7, rec
+assert torch.equal(out[:3], want[:3]) and float(out[3:].abs().sum()) == 0
+order = torch.tensor([0, 1, 6, 3, 4, 5], dtype=torch.int32, device=dev)
+out.zero_()
+narrow.narrow_gemm(xe, we, out=out, offsets=good, order=order, rows=6)
+torch.cuda.synchronize()
+rec = _lib.bounds_status()
+assert rec is not None and rec[0] == "narrow_gemm.cu" and rec[2:] == (6, 6), rec
+assert torch.equal(out[:2], want[:2]) and float(out[2].abs().sum()) == 0
+out.zero_()
+pair_gemm(xe, we, out=out, offsets=torch.tensor([0, 2, 3, 9], dtype=torch.int32, device=dev))
+torch.cuda.synchronize()
+rec = _lib.bounds_status()
+assert rec is not None and rec[0] == "pair_gemm.cu" and rec[3] == 7, rec
+assert torch.equal(out[:3], pairs[:3]) and float(out[3:].abs().sum()) == 0
+
 # and a clean call leaves no record
 qkv(pos_ok)
 assert _lib.bounds_status() is None
