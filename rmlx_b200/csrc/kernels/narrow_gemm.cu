@@ -205,9 +205,11 @@ __global__ void __launch_bounds__(NwShape<KIND, T>::THREADS, 1) narrow_gemm_kern
       const int tile = locate(p_item, p_e).y * p.RT + rt;
       if (tile < tiles) {
         // the first two lines of the rows of the next row block, whose stages are asked for only when this item's have run
-        if (tile + p.RT < tiles)
-          nw_prefetch(p.w + (size_t(p_e) * p.N + (tile + p.RT) * per + (lane & 7) + ((lane >> 3) & 1) * half) * row_bytes +
-                      (ks + (lane >> 4) * p.KS) * kNwCB);
+        // (a row may have fewer)
+        if (const int c = ks + (lane >> 4) * p.KS; tile + p.RT < tiles && c < chunks) {
+          const size_t at = (size_t(p_e) * p.N + (tile + p.RT) * per + (lane & 7) + ((lane >> 3) & 1) * half) * row_bytes + c * kNwCB;
+          if (RB_BOUNDS(at, size_t(p.E) * p.N * row_bytes)) nw_prefetch(p.w + at);
+        }
         const size_t row = size_t(p_e) * p.N + tile * per;
         p_w = p.w + (row + (lane >> 3)) * row_bytes + (lane & 7) * 16;
         if (KIND)

@@ -106,6 +106,15 @@ rec = _lib.bounds_status()
 assert rec is not None and rec[0] == "pair_gemm.cu" and rec[3] == 7, rec
 assert torch.equal(out[:3], pairs[:3]) and float(out[3:].abs().sum()) == 0
 
+# rows of W shorter than what is asked for ahead (one ring stage), and more row blocks than one: no address past the weight
+for kind, k in (("q4", 512), ("q4", 1024), ("q8", 512), (None, 64)):
+    for shares in (0, 1, 2):
+        ws = LinearWeight.random(16 * 24 * 148 * 2 + 16, k, kind, dev, generator=g)
+        narrow.narrow_gemm(torch.randn(3, k, device=dev, generator=g).to(torch.bfloat16), ws, shares=shares)
+        torch.cuda.synchronize()
+        rec = _lib.bounds_status()
+        assert rec is None, (kind, k, shares, rec)
+
 # and a clean call leaves no record
 qkv(pos_ok)
 assert _lib.bounds_status() is None
