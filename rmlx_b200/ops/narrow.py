@@ -61,6 +61,17 @@ def pays_grouped(gate_up: LinearWeight, down: LinearWeight, pairs: int) -> bool:
             gate_up.n * gate_up.k >= 1 << 20 and supported(gate_up) and supported(down))
 
 
+def _holds(t: torch.Tensor, rows: int, columns: int) -> bool:
+    """At least so many rows and columns, columns side by side."""
+    return t.dim() == 2 and t.shape[0] >= rows and t.shape[1] >= columns and t.stride(1) == 1
+
+
+def same_layout(residual: Optional[torch.Tensor], out: Optional[torch.Tensor], rows: int, columns: int) -> bool:
+    """Whether a residual is laid out as the result is (a new one without ``out``), which the tensor-core GEMMs ask for."""
+    return residual is None or (residual.shape == (rows, columns) and
+                                residual.stride() == ((columns, 1) if out is None else out.stride()))
+
+
 def narrow_gemm(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6,
                 residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, out_dtype=torch.bfloat16,
                 swiglu: bool = False, offsets: Optional[torch.Tensor] = None, order: Optional[torch.Tensor] = None,
@@ -76,6 +87,8 @@ def narrow_gemm(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor]
     n = w.n // 2 if swiglu else w.n
     if out is None:
         out = torch.empty(m, n, dtype=out_dtype, device=x.device)
+    assert out.dtype in (torch.bfloat16, torch.float32) and _holds(out, m, n)
+    assert residual is None or (residual.dtype == torch.bfloat16 and _holds(residual, m, n))
     rc = _lib.cuda().rmlx_narrow_gemm(
         w.kind, w.w.data_ptr(), _lib.ptr(w.scales), _lib.ptr(w.biases), x.data_ptr(), x.stride(0), x_div, _lib.ptr(order),
         _lib.ptr(offsets), 1 if offsets is None else w.experts, _lib.ptr(norm_w), eps, _lib.ptr(residual),

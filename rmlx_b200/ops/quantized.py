@@ -99,12 +99,12 @@ def pair_gemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor]
 
 def qmm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = None,
         out: Optional[torch.Tensor] = None, pdl: bool = False) -> torch.Tensor:
-    """x @ W^T for affine-quantised W: a few rows go through the weight-streaming kernel (``ops/narrow.py``); otherwise 4-bit weights are expanded inside the tensor-core GEMM's main
-    loop; 8-bit weights, weights with fp16 scales and 4-bit shapes the fused kernel does not take are
-    expanded to bf16 by the
-    dequantisation kernel first and go through the bf16 tensor-core GEMM."""
+    """x @ W^T for affine-quantised W: a few rows go through the weight-streaming kernel (``ops/narrow.py``); otherwise 4-bit
+    weights are expanded inside the tensor-core GEMM's main loop; 8-bit weights, weights with fp16 scales and 4-bit shapes the
+    fused kernel does not take are expanded to bf16 by the dequantisation kernel first and go through the bf16 tensor-core GEMM."""
     assert w.kind != 0
-    if x.shape[0] <= 64 and narrow.pays(w, x.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+    if x.shape[0] <= 64 and narrow.pays(w, x.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and \
+            narrow.same_layout(residual, out, x.shape[0], w.n):
         return narrow.narrow_gemm(x, w, residual=residual, out=out, pdl=pdl)
     if w.kind == W_Q4 and not w.scales_f16 and _lib.cuda().rmlx_qgemm_supported(w.k):
         return xgemm(x, w, residual, out, pdl=pdl)

@@ -174,3 +174,29 @@ def test_scales_at_odd_addresses(dev, kind):
     assert narrow.supported(w) and not narrow.supported(odd)
     # the per-row kernels multiply in fp16 (2^-11 per product)
     assert _rel(D.rms_gemv(x, odd, out_dtype=torch.float32), x.double() @ wd.t()) < 2e-3
+
+
+@pytest.mark.parametrize("kind", ["q4", "q8", None])
+def test_residuals_of_another_shape(dev, kind):
+    """A residual with too few rows is refused for every kind of weight; one whose rows lie apart is refused where the tensor-core
+    GEMM of the same weight refuses it (bf16, 8-bit)."""
+    from rmlx_b200.models.prefill import _mm
+    from rmlx_b200.ops import decode as D
+    from rmlx_b200.ops import narrow
+    w, wd, x, g = _case(dev, kind, 2048, 1024, 6, seed=9)
+    assert narrow.pays(w, 6)
+    res = torch.randn(6, 2048, device=dev, generator=g).to(torch.bfloat16)
+    for bad in (res[:1], res[:5], res[:, :2032].contiguous(), res.float(), res[0]):
+        with pytest.raises(AssertionError):
+            narrow.narrow_gemm(x, w, residual=bad)
+        with pytest.raises(AssertionError):
+            D.rms_gemv(x, w, residual=bad)
+    wide = torch.zeros(6, 2056, dtype=torch.bfloat16, device=dev)
+    wide[:, :2048] = res
+    if kind != "q4":
+        for bad in (res[:1], wide[:, :2048]):
+            with pytest.raises(AssertionError):
+                _mm(x, w, residual=bad)
+    want = x.double() @ wd.t() + res.double()
+    assert _rel(_mm(x, w, residual=res), want) < 4e-3
+    assert _rel(narrow.narrow_gemm(x, w, residual=wide[:, :2048]), want) < 4e-3
