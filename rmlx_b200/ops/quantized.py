@@ -42,6 +42,9 @@ def xgemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = N
         assert offsets.dtype == torch.int32 and offsets.numel() == e + 1
     if out is None:
         out = torch.empty(m, n // 2 if swiglu else n, dtype=torch.bfloat16, device=x.device)
+    # the epilogue reads the residual with the result's row stride
+    assert residual is None or (residual.dim() == 2 and residual.shape[0] >= m and residual.shape[1] >= n and
+                                residual.stride(1) == 1 and (m == 1 or residual.stride(0) == out.stride(0)))
     if bn == 0 and m > 128 and pair_pays(w.kind, m, n, k, e) and (not swiglu or (n % 256 == 0 and residual is None)) and \
             (residual is None or e == 0) and (w.kind != W_Q4 or not w.scales_f16) and (w.kind != W_Q4 or k % 512 == 0) and \
             k % 8 == 0 and _pair_ready(x, out, residual) and out.dtype == torch.bfloat16:
@@ -72,7 +75,7 @@ def pair_pays(kind: int, m: int, n: int, k: int, experts: int = 0) -> bool:
 def _pair_ready(x: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
     """16-byte rows, as the pair kernel loads and stores them."""
     return x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and \
-        out.stride(1) == 1 and (residual is None or (residual.data_ptr() % 16 == 0 and residual.stride() == out.stride()))
+        out.stride(1) == 1 and (residual is None or (residual.data_ptr() % 16 == 0 and residual.shape == out.shape))
 
 
 def pair_gemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,

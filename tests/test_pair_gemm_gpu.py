@@ -79,3 +79,19 @@ def test_rule_changes_no_result(dev, kind, m):
     x2 = torch.zeros(m, 520, dtype=torch.bfloat16, device=dev)
     x2[:, :512] = x
     assert torch.equal(xgemm(x2[:, :512], w), want)
+
+
+@pytest.mark.parametrize("kind", [None, "q4"])
+def test_residual_with_more_rows(dev, kind):
+    """``xgemm`` takes the first rows of a longer residual on either side of the rule, and refuses one that is too short or has
+    another row stride."""
+    from rmlx_b200.ops.quantized import pair_pays, xgemm
+    w, _, x, g = _case(dev, kind, 2048, 4096, 512, seed=3)
+    assert pair_pays(w.kind, 2048, 4096, 512)
+    res = torch.randn(2050, 4096, device=dev, generator=g).to(torch.bfloat16)
+    for m in (100, 2048):
+        assert torch.equal(xgemm(x[:m], w, residual=res), xgemm(x[:m], w, residual=res[:m]))
+        wide = torch.zeros(m, 4104, dtype=torch.bfloat16, device=dev)
+        for bad in (res[:m - 1], wide[:, :4096]):
+            with pytest.raises(AssertionError):
+                xgemm(x[:m], w, residual=bad)
