@@ -141,11 +141,13 @@ class _Layers:
         m = self.m
         cfg, w = m.cfg, m.w
         r = rows.shape[0]
-        if r <= 4 or narrow.pays(w.lm_head, r):
-            out = D.rms_gemv(rows.contiguous(), w.lm_head, w.final_norm, cfg.rms_norm_eps,
+        rows = rows.contiguous()
+        # more rows than the per-row kernels are for only if rms_gemv will take the weight-streaming kernel
+        if r <= 4 or (narrow.pays(w.lm_head, r) and D._several(r, w.lm_head, rows, w.final_norm)):
+            out = D.rms_gemv(rows, w.lm_head, w.final_norm, cfg.rms_norm_eps,
                              out=torch.empty(r, w.lm_head.n, dtype=torch.float32, device=m.device))
         else:
-            xn = D.rms_norm(rows.contiguous(), w.final_norm, cfg.rms_norm_eps)
+            xn = D.rms_norm(rows, w.final_norm, cfg.rms_norm_eps)
             if w.lm_head.kind == W_BF16 and w.lm_head.k % 8 == 0:
                 from ..ops.gemm import gemm_bf16_f32       # accumulator stored unrounded
                 out = gemm_bf16_f32(xn, w.lm_head.w)

@@ -108,7 +108,7 @@ def set_q4_path(path: str) -> None:
     _Q4_PATH = path
 
 
-def _several(b: int, w: LinearWeight, x: torch.Tensor) -> bool:
+def _several(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[torch.Tensor] = None) -> bool:
     """Several rows: the weight-streaming kernel of ``ops/narrow.py``, which multiplies eight rows for the price of one
     (4-bit 9216 x 4096 at 8 rows: 11 us, 39 on the tensor-core mat-vec, 30 on the streaming kernel), unless the weight is so
     small that its fixed part exceeds two or three passes of the per-row kernels. ``q4_path`` and the streaming switch away
@@ -116,7 +116,7 @@ def _several(b: int, w: LinearWeight, x: torch.Tensor) -> bool:
     # two rows of 4-bit weights: a 16384 x 2048 projection 9 us against 11, a 3072 x 2048 one 6 against 5
     least = 0 if b >= 4 else 1 << 24 if b == 2 and w.kind == W_Q4 else 1 << 20
     return (b >= 2 and _STREAM and q4_path() == "auto" and w.n * w.k >= least and narrow.supported(w) and
-            x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+            x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and (norm_w is None or norm_w.data_ptr() % 16 == 0))
 
 
 def _copied_whole(w: LinearWeight) -> bool:
@@ -140,7 +140,7 @@ def rms_gemv(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor] = 
     assert k == w.k, f"K mismatch {k} vs {w.k}"
     if out is None:
         out = torch.empty(b, n, dtype=out_dtype, device=x.device)
-    if _several(b, w, x) and (norm_w is None or norm_w.data_ptr() % 16 == 0):
+    if _several(b, w, x, norm_w):
         return narrow.narrow_gemm(x, w, norm_w, eps, residual=residual, out=out, pdl=pdl)
     lib, st = _lib.cuda(), _lib.stream_ptr()
     # Several rows against 4-bit weights: the tensor-core mat-vec carries up to eight rows in the
@@ -197,7 +197,7 @@ def rms_gate_up_swiglu(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.
     i = w.n // 2
     if out is None:
         out = torch.empty(b, i, dtype=torch.bfloat16, device=x.device)
-    if _several(b, w, x) and w.n % 32 == 0 and (norm_w is None or norm_w.data_ptr() % 16 == 0):
+    if w.n % 32 == 0 and _several(b, w, x, norm_w):
         return narrow.narrow_gemm(x, w, norm_w, eps, out=out, swiglu=True, pdl=pdl)
     lib, st = _lib.cuda(), _lib.stream_ptr()
     if _stream("gate_up", w):

@@ -324,3 +324,36 @@ def test_nan_row_has_no_expert(dev, experts, kind):
     got = moe_prefill_ffn(x, idx, wts, offsets, gu, dn, residual=res)
     want = moe_prefill_ffn(x, whole[0], whole[1], whole[3], gu, dn, residual=res)
     assert torch.equal(got[kept], want[kept]) and torch.equal(got[nan], res[nan])
+
+
+@pytest.mark.parametrize("quant", [None, "q4", "q8"])
+def test_logits_of_some_rows_without_the_streaming_kernels(dev, quant, monkeypatch):
+    """The LM head on 5 to 32 rows with the streaming kernels off, another 4-bit path, or a norm at an odd address: the tensor-core
+    projection of the normalised rows, as for more rows, whatever the weight's kind. It rounds the norm's result to bf16 and, for
+    quantised weights, expanded weights and logits: 1.7e-3 each in the mean over a binade, so 3e-3 of the whole."""
+    from rmlx_b200.models.prefill import _Layers
+    from rmlx_b200.ops import decode as D
+    cfg = _dense_cfg().replace(hidden_size=512, vocab_size=4096)
+    model = TransformerModel(from_state_dict(cfg, random_state_dict(cfg, 0), device=dev, quant=quant))
+    layers, w = _Layers(model), model.w
+    g = torch.Generator(device=dev).manual_seed(12)
+    rows = torch.randn(32, 512, device=dev, generator=g).to(torch.bfloat16)
+    want = rows.double() * torch.rsqrt(rows.double().pow(2).mean(-1, keepdim=True) + cfg.rms_norm_eps) * w.final_norm.double()
+    want = want @ w.lm_head.dequantized().double().t()
+
+    def check():
+        for r in (5, 8, 16, 32):
+            got = layers.logits(rows[:r])
+            assert float((got.double() - want[:r]).norm() / want[:r].norm()) < 4e-3
+
+    check()
+    monkeypatch.setattr(D, "_STREAM", False)
+    check()
+    monkeypatch.setattr(D, "_STREAM", True)
+    monkeypatch.setattr(D, "_Q4_PATH", "mma")
+    check()
+    monkeypatch.setattr(D, "_Q4_PATH", "auto")
+    odd = torch.zeros(520, dtype=torch.bfloat16, device=dev)
+    odd[1:513] = w.final_norm
+    w.final_norm = odd[1:513]
+    check()
