@@ -417,6 +417,8 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    // 16-byte stores (and loads of the residual) where the rows allow them: any result may be a view, and N any number
+    const bool vec = (ldc & 7) == 0 && ((reinterpret_cast<uintptr_t>(C) | (RESIDUAL ? reinterpret_cast<uintptr_t>(residual) : 0)) & 15) == 0;
     if (RESIDUAL && !GROUPED) pdl_wait();
 
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -475,7 +477,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             for (int j = 0; j < 32; ++j) {
               f[j] = gated_act_fast(__uint_as_float(rg[j]), __uint_as_float(ru[j]), gate_limit);
             }
-            if (col0 + 32 <= n_out) {
+            if (vec && col0 + 32 <= n_out) {
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
                 uint4 o;
@@ -500,7 +502,7 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           if (row < t.row_end && col0 < N) {
             __nv_bfloat16* dst = C + size_t(row) * ldc + col0;
             const __nv_bfloat16* res = RESIDUAL ? residual + size_t(row) * ldc + col0 : nullptr;
-            if (col0 + 32 <= N) {
+            if (vec && col0 + 32 <= N) {
 #pragma unroll
               for (int v = 0; v < 4; ++v) {
                 float f[8];

@@ -68,17 +68,38 @@ def test_grouped(dev, kind):
 @pytest.mark.parametrize("kind", [None, "q4"])
 @pytest.mark.parametrize("m", [128, 129, 700, 2048])
 def test_rule_changes_no_result(dev, kind, m):
-    """``xgemm`` on either side of the rule, with rows and outputs that are not 16-byte aligned: the same values."""
+    """``xgemm`` on either side of the rule, with rows of x apart and results that are views, 16-byte aligned (SM pairs) and not
+    (single SMs, stored element by element): the same values, and nothing beside them is written."""
     from rmlx_b200.ops.quantized import pair_pays, xgemm
     w, _, x, g = _case(dev, kind, m, 4096, 512, seed=2)
     assert pair_pays(w.kind, 2048, 4096, 512) and not pair_pays(w.kind, 128, 4096, 512)
-    want = xgemm(x, w, bn=128)
+    res = torch.randn(m, 4096, device=dev, generator=g).to(torch.bfloat16)
+    want, more, act = xgemm(x, w, bn=128), xgemm(x, w, residual=res, bn=128), xgemm(x, w, bn=128, swiglu=True)
     assert torch.equal(xgemm(x, w), want)
-    wide = torch.zeros(m, 4104, dtype=torch.bfloat16, device=dev)
-    assert torch.equal(xgemm(x, w, out=wide[:, :4096]), want)
+    for stride, at in ((4104, 0), (4104, 8), (4100, 0), (4104, 1), (4101, 3)):
+        room = torch.zeros(m * stride + 8, dtype=torch.bfloat16, device=dev)
+        wide = torch.zeros(m * stride + 8, dtype=torch.bfloat16, device=dev)
+        out = room[at:at + m * stride].view(m, stride)[:, :4096]
+        r = wide[at:at + m * stride].view(m, stride)[:, :4096]
+        r.copy_(res)
+        assert torch.equal(xgemm(x, w, out=out), want)
+        assert torch.equal(xgemm(x, w, residual=r, out=out), more)
+        out.zero_()
+        assert torch.equal(xgemm(x, w, out=out[:, :2048], swiglu=True), act)
+        out[:, :2048].zero_()
+        assert not bool(room.any())
     x2 = torch.zeros(m, 520, dtype=torch.bfloat16, device=dev)
     x2[:, :512] = x
     assert torch.equal(xgemm(x2[:, :512], w), want)
+
+
+@pytest.mark.parametrize("kind", [None, "q4"])
+@pytest.mark.parametrize("n", [33, 100, 1001])
+def test_any_number_of_columns(dev, kind, n):
+    """Rows of a result of any number of columns start at any address: more than one piece of 32 columns, ends inside a piece."""
+    from rmlx_b200.ops.quantized import xgemm
+    w, wd, x, _ = _case(dev, kind, 150, n, 512, seed=4)
+    assert _rel(xgemm(x, w), x.double() @ wd.t()) < (2 * ROUND if kind else ROUND)
 
 
 @pytest.mark.parametrize("kind", [None, "q4"])
