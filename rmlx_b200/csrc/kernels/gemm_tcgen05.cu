@@ -164,6 +164,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    // plain and residual results: 16-byte accesses where the rows allow them
+    const bool vec = (ldc & 7) == 0 && ((reinterpret_cast<uintptr_t>(Cv) | (RESIDUAL ? reinterpret_cast<uintptr_t>(residual) : 0)) & 15) == 0;
     if (RESIDUAL || DUAL) pdl_wait();
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const int tm = tile % tiles_m, tn = tile / tiles_m;
@@ -246,7 +248,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         } else if (row < M && col0 < N) {
           __nv_bfloat16* dst = C + size_t(row) * ldc + col0;
           const __nv_bfloat16* res = RESIDUAL ? residual + size_t(row) * ldc + col0 : nullptr;
-          if (col0 + 32 <= N) {
+          if (vec && col0 + 32 <= N) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
               float f[8];

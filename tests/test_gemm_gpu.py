@@ -51,3 +51,23 @@ def test_many_tiles_per_cta_phases():
     # > 148 tiles so every CTA walks several tiles and both accumulators wrap their phases
     _check(4096, 4096, 512, bn=128)
     _check(8192, 4096, 256, bn=256, residual=True)
+
+
+@pytest.mark.parametrize("residual", [False, True])
+def test_rows_at_any_address(residual):
+    """Any number of columns, and results and residuals that are views at odd strides and offsets."""
+    for n in (33, 100, 1001):
+        _check(150, n, 128, residual=residual, seed=2)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(150, 128, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(256, 128, device="cuda", generator=g).to(torch.bfloat16)
+    r = torch.randn(150, 256, device="cuda", generator=g).to(torch.bfloat16) if residual else None
+    want = gemm_bf16(x, w, residual=r)
+    for stride, at in ((264, 8), (260, 0), (264, 1), (259, 3)):
+        room, wide = (torch.zeros(150 * stride + 8, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        out, res = (t[at:at + 150 * stride].view(150, stride)[:, :256] for t in (room, wide))
+        if residual:
+            res.copy_(r)
+        assert torch.equal(gemm_bf16(x, w, residual=res if residual else None, out=out), want)
+        out.zero_()
+        assert not bool(room.any())
