@@ -14,7 +14,9 @@
 //     are never rounded;
 //   * x is staged in shared memory in the order in which the fragments read it, as fp16 with one power of two per (row,
 //     group) chosen from the group's maximum (exact for bf16 inputs), with the group's sum beside it. bf16 weights take x
-//     as bf16, and x times a norm's weight (16 significant bits) as two bf16 terms, in two tiles that share the weights;
+//     as bf16, and x times a norm's weight (16 significant bits) as two bf16 terms, in two tiles that share the weights, and are
+//     summed 64 of K at a time in the tensor cores, which cut what they add, and from there in fp32 (error of the fp32 result
+//     at K = 14336 1.4e-7 of it, 2.0e-6 as one sum in the tensor cores; a step of 5 rows 626 -> 634 us);
 //   * a norm's 1 / rms multiplies the sums.
 // The loop is a chain of short dependent instructions: what hides it is warps, so the quantised kernels are held to 80
 // registers for 24 of them (16 warps of 128: 332 us for 128 experts of 3072 x 4096 in 4 bits, where 24 take 222).
@@ -106,11 +108,17 @@ __device__ __forceinline__ void nw_mma(float (&d)[4], uint32_t a0, uint32_t a1, 
 }
 
 // The first product of a sum: nothing to add to.
+template <bool F16>
 __device__ __forceinline__ void nw_mma0(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                         uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+  if constexpr (F16)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ void nw_mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                             uint32_t b1) {
@@ -439,14 +447,17 @@ __global__ void __launch_bounds__(NwShape<KIND, T>::THREADS, 1) narrow_gemm_kern
         const uint32_t un = n * S::SLG + j;
         const uint4 x0 = nw_lds128(xa + un * 1024), x1 = nw_lds128(xa + un * 1024 + 512);
         if constexpr (KIND == 0) {
-          nw_mma<false>(acc[n], a[0][0], a[1][0], a[0][1], a[1][1], x0.x, x0.y);
-          nw_mma<false>(acc[n], a[0][2], a[1][2], a[0][3], a[1][3], x0.z, x0.w);
-          nw_mma<false>(acc[n], a[0][4], a[1][4], a[0][5], a[1][5], x1.x, x1.y);
-          nw_mma<false>(acc[n], a[0][6], a[1][6], a[0][7], a[1][7], x1.z, x1.w);
+          float c[4];
+          nw_mma0<false>(c, a[0][0], a[1][0], a[0][1], a[1][1], x0.x, x0.y);
+          nw_mma<false>(c, a[0][2], a[1][2], a[0][3], a[1][3], x0.z, x0.w);
+          nw_mma<false>(c, a[0][4], a[1][4], a[0][5], a[1][5], x1.x, x1.y);
+          nw_mma<false>(c, a[0][6], a[1][6], a[0][7], a[1][7], x1.z, x1.w);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[n][i] += c[i];
         } else {
           const uint2 xq = nw_lds64(qa + un * 32);        // scales of rows 2t and 2t + 1
           float c[4];
-          nw_mma0(c, a[0][0], a[1][0], a[0][1], a[1][1], x0.x, x0.y);
+          nw_mma0<true>(c, a[0][0], a[1][0], a[0][1], a[1][1], x0.x, x0.y);
           nw_mma<true>(c, a[0][2], a[1][2], a[0][3], a[1][3], x0.z, x0.w);
           nw_mma<true>(c, a[0][4], a[1][4], a[0][5], a[1][5], x1.x, x1.y);
           nw_mma<true>(c, a[0][6], a[1][6], a[0][7], a[1][7], x1.z, x1.w);

@@ -200,3 +200,17 @@ def test_residuals_of_another_shape(dev, kind):
     want = x.double() @ wd.t() + res.double()
     assert _rel(_mm(x, w, residual=res), want) < 4e-3
     assert _rel(narrow.narrow_gemm(x, w, residual=wide[:, :2048]), want) < 4e-3
+
+
+@pytest.mark.parametrize("k", [2048, 14336])
+@pytest.mark.parametrize("norm", [False, True])
+def test_sums_of_bf16_weights(dev, k, norm):
+    """Products of bf16 are exact in fp32, so the error is that of adding them up: K / 64 rounded additions of 2^-24 each (in a
+    random walk 4e-7 for the longest K), and what the tensor cores cut inside 64 of K. With one sum in the tensor cores it is 2e-6."""
+    from rmlx_b200.ops import narrow
+    w, wd, x, g = _case(dev, None, 512, k, 5, seed=10)
+    nw = (torch.rand(k, device=dev, generator=g) + 0.5).to(torch.bfloat16) if norm else None
+    xd = x.double()
+    want = (xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double() if norm else xd) @ wd.t()
+    for shares in (0, 1):
+        assert _rel(narrow.narrow_gemm(x, w, nw, 1e-6, out_dtype=torch.float32, shares=shares), want) < 5e-7
