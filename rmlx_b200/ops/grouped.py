@@ -6,6 +6,7 @@ down -> routing-weighted combine + residual). The reference's counterpart is
 crates/rmlx-nn/src/moe.rs:1391-1508)."""
 from __future__ import annotations
 
+import os
 from typing import Optional
 
 import torch
@@ -15,6 +16,14 @@ from . import narrow
 from .quantized import xgemm
 from .weights import LinearWeight, W_BF16, W_Q4
 
+# RMLX_MOE_NARROW_ROWS=n: up to n rows per expert on average, 4-bit experts that ``narrow.pays_grouped`` leaves to the tensor-core
+# tiles (a rank's slice of the experts, more rows) take the weight-streaming kernel too. Off by default (0).
+_NARROW_MAX_AVG_ROWS = float(os.environ.get("RMLX_MOE_NARROW_ROWS", "0"))
+
+
+def narrow_ok(gate_up: LinearWeight, down: LinearWeight, rows: int, experts: int) -> bool:
+    """Whether ``moe_prefill_ffn`` sends this many sorted rows through ``narrow_expert_ffn``."""
+    return 0 < rows <= _NARROW_MAX_AVG_ROWS * experts and narrow_supported(gate_up, down)
 
 
 def narrow_supported(gate_up: LinearWeight, down: LinearWeight, variant: Optional[int] = None) -> bool:
@@ -91,10 +100,11 @@ def moe_prefill_ffn(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, offse
     _lib.check(lib.rmlx_moe_scatter_rows(x.data_ptr(), x.stride(0), idx.data_ptr(), offsets.data_ptr(),
                                          cursors.data_ptr(), xs.data_ptr(), row_of_pair.data_ptr(),
                                          t, k, d, e, st), "moe_scatter_rows")
+    ffn = narrow_expert_ffn if narrow_ok(gate_up, down, t * k, e) else grouped_expert_ffn
     if e_local == e:
-        y = grouped_expert_ffn(xs, offsets, gate_up, down)
+        y = ffn(xs, offsets, gate_up, down)
     else:
-        y = grouped_expert_ffn(xs, offsets[expert_base:expert_base + e_local + 1], gate_up, down, zero_rest=True)
+        y = ffn(xs, offsets[expert_base:expert_base + e_local + 1], gate_up, down, zero_rest=True)
     out = torch.empty(t, d, dtype=torch.bfloat16, device=x.device)
     _lib.check(lib.rmlx_moe_combine(y.data_ptr(), row_of_pair.data_ptr(), wts.data_ptr(),
                                     _lib.ptr(residual), 0 if residual is None else residual.stride(0),

@@ -138,6 +138,30 @@ def test_narrow_grouped_expert_ffn(dev, variant):
     lo, hi = int(off[2]), int(off[5])
     _close(part[lo:hi], want[lo:hi])
     assert float(part[:lo].abs().sum()) == 0.0 and float(part[hi:].abs().sum()) == 0.0
-    torch.cuda.synchronize()
-    from rmlx_b200 import _lib
-    assert _lib.cuda().rmlx_qmv_status() == 0
+
+
+def test_narrow_rows_switch_on_a_slice_of_the_experts(dev, monkeypatch):
+    """RMLX_MOE_NARROW_ROWS: ranks that hold a slice of the experts each take the few-row kernel, and their results add up to the
+    whole layer's. Both sides are bf16 results, 5e-3 from the exact one each, so 7e-3 from each other."""
+    from rmlx_b200.ops import decode as D
+    from rmlx_b200.ops import grouped
+    e, d, i, t, k = 8, 1024, 512, 12, 2
+    wgu, wdn = _w(2 * i, d, "q4", dev, experts=e, seed=21), _w(d, i, "q4", dev, experts=e, seed=22)
+    torch.manual_seed(23)
+    x = torch.randn(t, d, device=dev).to(torch.bfloat16)
+    idx, wts, _, offsets = D.topk_route(torch.randn(t, e, device=dev), k)
+    taken = []
+    plain = grouped.narrow_expert_ffn
+    monkeypatch.setattr(grouped, "narrow_expert_ffn", lambda *a, **kw: taken.append(1) or plain(*a, **kw))
+
+    def parts():
+        return sum(grouped.moe_prefill_ffn(x, idx, wts, offsets, wgu.experts_slice(b, b + 4), wdn.experts_slice(b, b + 4),
+                                           expert_base=b).float() for b in (0, 4))
+
+    whole = parts()
+    assert not taken
+    monkeypatch.setattr(grouped, "_NARROW_MAX_AVG_ROWS", 3.0)
+    _close(parts(), whole, fro=7e-3)
+    assert len(taken) == 2
+    monkeypatch.setattr(grouped, "_NARROW_MAX_AVG_ROWS", 2.9)
+    assert torch.equal(parts(), whole) and len(taken) == 2
