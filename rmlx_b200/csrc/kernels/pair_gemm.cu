@@ -8,11 +8,11 @@
 // once for both: 64 KB (bf16) or 72 KB (4-bit) per SM, and each SM expands half as many weights per product.
 //
 // Roles per block (persistent, one pair per two SMs): warp 0 TMA producer of A (and bf16 W), warp 1 issues the products in the first
-// block of the pair (in both it owns the tensor memory), warps 2-5 epilogue of the block's 128 rows; 4-bit weights: two groups of
-// eight dequant warps that take the k-blocks in turn, and a warp that asks for packed weights and scales. Packed weights come 128
-// bytes of a row at a time, four k-blocks: the copy engine spends its time per row (32-byte pieces: 1300 cycles a k-block). Loads of both blocks count
-// on the first one's barriers; the products' completion is committed to both. Every wait is bounded; both blocks meet before they
-// leave, since each reads or signals the other's shared memory. Loads carry no cluster-broadcast qualifier.
+// block of the pair (in both it owns the tensor memory), warps 2-5 epilogue of the block's 128 rows; 4-bit weights: four groups of
+// four dequant warps that take the k-blocks in turn, and a warp that asks for packed weights and scales. Packed weights come 128
+// bytes of a row at a time, four k-blocks: the copy engine spends its time per row (32-byte pieces: 1300 cycles a k-block). Loads of
+// both blocks count on the first one's barriers; the products' completion is committed to both. Every wait is bounded; both blocks
+// meet before they leave, since each reads or signals the other's shared memory. Loads carry no cluster-broadcast qualifier.
 #include "xgemm_kernel.cuh"
 
 namespace rb {
@@ -47,9 +47,12 @@ __device__ __forceinline__ uint32_t pair_first(const void* p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
   return a;
 }
-// Signals and waits order accesses of the tensor cores and the copy engine, which the fences in front of them cover, and none of
-// the threads' own to the other block's memory: the default scope is enough (the cluster scope costs a memory barrier per signal and
-// an L1 invalidation per poll, 880 cycles a k-block instead of 600).
+// Signals and waits between the blocks have the default scope, the block's. That is a reliance, not something that the memory model
+// gives: two of them order more than one block's accesses. What they order is what the tensor cores and the copy engine read or write
+// (expanded weights behind each thread's proxy fence, accumulators behind the tcgen05 fences), in the memory of the SM whose threads
+// wrote it, and no thread reads what the other block's threads stored; the pair tests compare every result bit for bit with the
+// single-SM tiles over many runs. Release and acquire of cluster scope on the expanded weights' barrier alone cost a memory barrier
+// per signal and an L1 invalidation per poll: 2048 rows of 28672 x 4096 336 -> 395 us, 4096 x 14336 173 -> 220.
 __device__ __forceinline__ void pair_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }

@@ -1,6 +1,6 @@
 // The generalised tcgen05 GEMM kernel (see xgemm_tcgen05.cu for the plain entry points and
 // ../comm/tp_gemm.cu for the tensor-parallel ones). C = A · W^T with
-//   * W bf16 (TMA-fed) or MLX-affine Q4 dequantised inside the main loop by eight dequant warps;
+//   * W bf16 (TMA-fed) or MLX-affine Q4 dequantised inside the main loop by sixteen dequant warps in groups (collective modes: eight);
 //   * GROUPED: rows of A sorted by expert, tile table derived on the device from offsets[E+1];
 //   * swiglu: a tile holds BN/2 gate rows and the matching BN/2 up rows of W; the epilogue writes
 //     the gated activation (gated.cuh) straight from the fp32 accumulators;

@@ -86,6 +86,32 @@ def test_expert_feed_forward(dev, kind, rows):
         assert _rel(got, up.view(rows * k, -1)) < 2e-5
 
 
+@pytest.mark.parametrize("kind", ["q4", "q8", None])
+@pytest.mark.parametrize("experts,rows", [(12, 3), (256, 9)])
+def test_expert_feed_forward_with_norm(dev, kind, experts, rows):
+    """The form of a decode step: the norm of x inside the first projection, buffers that the caller keeps, and, at most, 256
+    experts. Errors: the norm's product rounded to fp16 (4-bit, 8-bit: 3e-4), activations and the result to bf16."""
+    from rmlx_b200.ops import narrow
+    d, inner, k = 1024, 512, 4
+    gu, gud, x, g = _case(dev, kind, 2 * inner, d, rows, experts=experts, seed=11)
+    dn, dnd, _, _ = _case(dev, kind, d, inner, 1, experts=experts, seed=12)
+    nw = (torch.rand(d, device=dev, generator=g) + 0.5).to(torch.bfloat16)
+    idx = torch.stack([torch.randperm(experts, device=dev, generator=g)[:k] for _ in range(rows)]).to(torch.int32)
+    idx[0, 0] = experts - 1
+    wts = torch.rand(rows, k, device=dev, generator=g)
+    res = torch.randn(rows, d, device=dev, generator=g).to(torch.bfloat16)
+    xd = x.double()
+    xn = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    up = torch.einsum("tsnk,tk->tsn", gud[idx.long()], xn)
+    act = torch.nn.functional.silu(up[..., :inner]) * up[..., inner:]
+    y = torch.einsum("tsnk,tsk->tsn", dnd[idx.long()], act)
+    want = res.double() + (y * wts.double()[..., None]).sum(1)
+    scratch, out = narrow.ExpertScratch(rows + 3, k, gu, dn), torch.empty_like(res)
+    for _ in range(2):
+        assert narrow.expert_ffn(x, idx, wts, gu, dn, nw, 1e-6, residual=res, out=out, scratch=scratch) is out
+        assert _rel(out, want) < 8e-3
+
+
 @pytest.mark.parametrize("kind", ["q4", "q8"])
 def test_extreme_inputs(dev, kind):
     """Zero groups, the smallest and largest magnitudes the activations' scaling covers, one huge value beside small ones, and

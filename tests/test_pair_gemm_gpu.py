@@ -51,6 +51,46 @@ def test_plain(dev, kind, m, n, k):
 
 
 @pytest.mark.parametrize("kind", [None, "q4"])
+@pytest.mark.parametrize("k", [512, 520, 1000, 4096])
+def test_many_runs_and_tiles(dev, kind, k):
+    """More tiles than pairs of SMs (162 for 74), K that ends inside a block of 64 (bf16), run after run: bit for bit the
+    single-SM tiles. The blocks of a pair rely on each other's signals (see the kernel); a signal that came too early would show."""
+    from rmlx_b200.ops.gemm import GemmStatus
+    from rmlx_b200.ops.quantized import pair_gemm, xgemm
+    if kind and k % 512:
+        pytest.skip("4-bit weights come 512 of K at a time")
+    w, wd, x, g = _case(dev, kind, 2304, 4608, k, seed=5)
+    want, act = xgemm(x, w, bn=128), xgemm(x, w, bn=128, swiglu=True)
+    assert _rel(want, x.double() @ wd.t()) < (2 * ROUND if kind else ROUND)
+    out, half = torch.empty_like(want), torch.empty_like(act)
+    for _ in range(60):
+        out.zero_(), half.zero_()
+        assert torch.equal(pair_gemm(x, w, out=out), want)
+        assert torch.equal(pair_gemm(x, w, out=half, swiglu=True), act)
+    GemmStatus.check(dev)
+
+
+@pytest.mark.parametrize("kind", [None, "q4"])
+@pytest.mark.parametrize("m,n,k", [(40, 256, 512), (300, 544, 1024), (700, 512, 2048)])
+def test_stacked_tiles(dev, kind, m, n, k):
+    """``bn=-128``, two row blocks per staged block of W, against the tiles of 128 columns: plain, residual, SwiGLU, grouped."""
+    from rmlx_b200.ops.gemm import GemmStatus
+    from rmlx_b200.ops.quantized import xgemm
+    w, _, x, g = _case(dev, kind, m, n, k, seed=6)
+    res = torch.randn(m, n, device=dev, generator=g).to(torch.bfloat16)
+    assert torch.equal(xgemm(x, w, bn=-128), xgemm(x, w, bn=128))
+    assert torch.equal(xgemm(x, w, residual=res, bn=-128), xgemm(x, w, residual=res, bn=128))
+    if n % 256 == 0:
+        assert torch.equal(xgemm(x, w, bn=-128, swiglu=True), xgemm(x, w, bn=128, swiglu=True))
+        counts = [m // 2, 0, 1, m - m // 2 - 1]
+        we, _, _, _ = _case(dev, kind, 1, n, k, experts=4, seed=7)
+        off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=dev)
+        for swiglu in (False, True):
+            assert torch.equal(xgemm(x, we, offsets=off, bn=-128, swiglu=swiglu), xgemm(x, we, offsets=off, bn=128, swiglu=swiglu))
+    GemmStatus.check(dev)
+
+
+@pytest.mark.parametrize("kind", [None, "q4"])
 def test_grouped(dev, kind):
     """Experts without rows, with one, with a whole tile and with more."""
     from rmlx_b200.ops.gemm import GemmStatus
