@@ -39,7 +39,7 @@ def _narrow(x: torch.Tensor, w: LinearWeight) -> bool:
 
 def _mm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     if w.kind == W_BF16:
-        if _narrow(x, w) and narrow.same_layout(residual, None, x.shape[0], w.n):
+        if _narrow(x, w) and (residual is None or narrow.same_layout(residual, None, x.shape[0], w.n)):
             return narrow.narrow_gemm(x, w, residual=residual)
         if x.shape[0] > 128 and w.w.is_contiguous() and pair_pays(W_BF16, x.shape[0], w.n, w.k):
             return xgemm(x, w, residual=residual)         # SM pairs

@@ -42,14 +42,15 @@ def pays(w: LinearWeight, rows: int) -> bool:
     the tiles less than half of the SMs. 8-bit weights would be expanded first (53 us for 28672 x 4096). bf16, 9216 x 4096:
     20 / 28 at 16 rows; 28672 x 4096: 46 / 45: eight rows, and 16 for up to 16384 rows of W. Weights of less than a million
     entries take a tile's time anyway."""
-    if rows < 1 or rows > 64 or w.n * w.k < 1 << 20:
+    n = w.n
+    if rows < 1 or rows > 64 or n * w.k < 1 << 20:
         return False
     if w.kind == W_BF16:
-        ok = rows <= 8 or (rows <= 16 and w.n <= 16384)
+        ok = rows <= 8 or (rows <= 16 and n <= 16384)
     elif w.kind == W_Q4:
-        ok = rows <= 16 or (rows <= 32 and w.n <= 4096)
+        ok = rows <= 16 or (rows <= 32 and n <= 4096)
     else:
-        ok = rows <= 16 or (rows <= 32 and w.n >= 8192)
+        ok = rows <= 16 or (rows <= 32 and n >= 8192)
     return ok and supported(w)
 
 
@@ -63,13 +64,13 @@ def pays_grouped(gate_up: LinearWeight, down: LinearWeight, pairs: int) -> bool:
 
 def _holds(t: torch.Tensor, rows: int, columns: int) -> bool:
     """At least so many rows and columns, columns side by side."""
-    return t.dim() == 2 and t.shape[0] >= rows and t.shape[1] >= columns and t.stride(1) == 1
+    shape = t.shape
+    return len(shape) == 2 and shape[0] >= rows and shape[1] >= columns and t.stride(1) == 1
 
 
-def same_layout(residual: Optional[torch.Tensor], out: Optional[torch.Tensor], rows: int, columns: int) -> bool:
+def same_layout(residual: torch.Tensor, out: Optional[torch.Tensor], rows: int, columns: int) -> bool:
     """Whether a residual is laid out as the result is (a new one without ``out``), which the tensor-core GEMMs ask for."""
-    return residual is None or (residual.shape == (rows, columns) and
-                                residual.stride() == ((columns, 1) if out is None else out.stride()))
+    return residual.shape == (rows, columns) and residual.stride() == ((columns, 1) if out is None else out.stride())
 
 
 def narrow_gemm(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6,
@@ -82,18 +83,25 @@ def narrow_gemm(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.Tensor]
     position (None: the position itself), whose input is row ``output row // x_div`` of x; ``rows``: positions in all.
     ``tiles`` (eight rows of x each per pass: 1, 2, 4) and ``shares`` (of K) are chosen from the sizes when 0."""
     _lib.require_cuda_tensor(x, w.w)
-    assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] == w.k
-    m = x.shape[0] if rows is None else rows
-    n = w.n // 2 if swiglu else w.n
+    n_all, k = w.n, w.k
+    shape, stride = x.shape, x.stride()
+    assert x.dtype == torch.bfloat16 and len(shape) == 2 and stride[1] == 1 and shape[1] == k
+    m = shape[0] if rows is None else rows
+    n = n_all // 2 if swiglu else n_all
     if out is None:
         out = torch.empty(m, n, dtype=out_dtype, device=x.device)
-    assert out.dtype in (torch.bfloat16, torch.float32) and _holds(out, m, n)
+    else:
+        assert _holds(out, m, n)
+    assert out.dtype in (torch.bfloat16, torch.float32)
     assert residual is None or (residual.dtype == torch.bfloat16 and _holds(residual, m, n))
+    scales, biases = w.scales, w.biases
     rc = _lib.cuda().rmlx_narrow_gemm(
-        w.kind, w.w.data_ptr(), _lib.ptr(w.scales), _lib.ptr(w.biases), x.data_ptr(), x.stride(0), x_div, _lib.ptr(order),
-        _lib.ptr(offsets), 1 if offsets is None else w.experts, _lib.ptr(norm_w), eps, _lib.ptr(residual),
-        0 if residual is None else residual.stride(0), out.data_ptr(), out.stride(0), int(out.dtype == torch.float32), m, w.n, w.k,
-        int(swiglu), tiles, shares, int(pdl), _lib.stream_ptr())
+        w.kind, w.w.data_ptr(), scales if scales is None else scales.data_ptr(), biases if biases is None else biases.data_ptr(),
+        x.data_ptr(), stride[0], x_div, order if order is None else order.data_ptr(),
+        offsets if offsets is None else offsets.data_ptr(), 1 if offsets is None else w.experts,
+        norm_w if norm_w is None else norm_w.data_ptr(), eps, residual if residual is None else residual.data_ptr(),
+        0 if residual is None else residual.stride(0), out.data_ptr(), out.stride(0), out.dtype == torch.float32, m, n_all, k,
+        swiglu, tiles, shares, pdl, _lib.stream_ptr())
     _lib.check(rc, "narrow_gemm")
     return out
 

@@ -107,7 +107,7 @@ def qmm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = Non
     fused kernel does not take are expanded to bf16 by the dequantisation kernel first and go through the bf16 tensor-core GEMM."""
     assert w.kind != 0
     if x.shape[0] <= 64 and narrow.pays(w, x.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and \
-            narrow.same_layout(residual, out, x.shape[0], w.n):
+            (residual is None or narrow.same_layout(residual, out, x.shape[0], w.n)):
         return narrow.narrow_gemm(x, w, residual=residual, out=out, pdl=pdl)
     if w.kind == W_Q4 and not w.scales_f16 and _lib.cuda().rmlx_qgemm_supported(w.k):
         return xgemm(x, w, residual, out, pdl=pdl)
