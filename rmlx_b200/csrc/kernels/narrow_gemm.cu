@@ -16,7 +16,8 @@
 //     group) chosen from the group's maximum (exact for bf16 inputs), with the group's sum beside it. bf16 weights take x
 //     as bf16, and x times a norm's weight (16 significant bits) as two bf16 terms, in two tiles that share the weights, and are
 //     summed 64 of K at a time in the tensor cores, which cut what they add, and from there in fp32 (error of the fp32 result
-//     at K = 14336 1.4e-7 of it, 2.0e-6 as one sum in the tensor cores; a step of 5 rows 626 -> 634 us);
+//     at K = 14336 1.4e-7 of it, 2.0e-6 as one sum in the tensor cores; 28672 x 4096 at 8 rows 45.4 -> 44.9 us, with a norm
+//     49.0 -> 50.2; adding the second terms up in the tensor cores: 50.9);
 //   * a norm's 1 / rms multiplies the sums.
 // The loop is a chain of short dependent instructions: what hides it is warps, so the quantised kernels are held to 80
 // registers for 24 of them (16 warps of 128: 332 us for 128 experts of 3072 x 4096 in 4 bits, where 24 take 222).
@@ -142,6 +143,12 @@ __device__ __forceinline__ uint64_t nw_fma2(uint64_t a, uint64_t b, uint64_t c) 
 __device__ __forceinline__ uint64_t nw_mul2(uint64_t a, uint64_t b) {
   uint64_t v;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+
+__device__ __forceinline__ uint64_t nw_add2(uint64_t a, uint64_t b) {
+  uint64_t v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
   return v;
 }
 
@@ -453,7 +460,9 @@ __global__ void __launch_bounds__(NwShape<KIND, T>::THREADS, 1) narrow_gemm_kern
           nw_mma<false>(c, a[0][4], a[1][4], a[0][5], a[1][5], x1.x, x1.y);
           nw_mma<false>(c, a[0][6], a[1][6], a[0][7], a[1][7], x1.z, x1.w);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) acc[n][i] += c[i];
+          for (int r = 0; r < 2; ++r)
+            nw_unpair(nw_add2(nw_pair(__float_as_uint(acc[n][2 * r]), __float_as_uint(acc[n][2 * r + 1])),
+                              nw_pair(__float_as_uint(c[2 * r]), __float_as_uint(c[2 * r + 1]))), acc[n][2 * r], acc[n][2 * r + 1]);
         } else {
           const uint2 xq = nw_lds64(qa + un * 32);        // scales of rows 2t and 2t + 1
           float c[4];

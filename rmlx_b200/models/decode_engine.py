@@ -31,7 +31,6 @@ from ..kv.paged import PagedKvCache
 from ..runtime.graph import GraphCache, bucket_for
 from ..ops import decode as D
 from ..ops import narrow
-from ..ops.weights import W_Q4
 from .transformer import TransformerModel
 
 
@@ -291,9 +290,8 @@ class CachedDecode(DecodeEngineBase):
         D.embedding(w.embed, tokens, out=self.h[:nb], pdl=False)
         h, h2 = self.h[:nb], self.h2[:nb]
         for li, lw in enumerate(w.layers):
-            # several rows: the projection runs on a kernel that takes eight rows per pass (ops/narrow.py, or the tensor-core
-            # mat-vec of 4-bit weights), and RoPE + the KV append follow as their own small kernel on its fp32 sums
-            if self.fuse_rope and not (nb >= 2 and (lw.wqkv.kind == W_Q4 or D._several(nb, lw.wqkv, h, lw.norm1))):
+            # projected apart, RoPE + the KV append follow as their own small kernel on the fp32 sums
+            if self.fuse_rope and not D.projects_apart(nb, lw.wqkv, h, lw.norm1):
                 D.rms_qkv_rope(h, lw.wqkv, lw.norm1, eps, q, self.cache.k[li], self.cache.v[li],
                                block_table, positions, m.cos, m.sin, m.hq, m.hkv,
                                traditional=cfg.rope_traditional, pdl=pdl)
@@ -317,7 +315,7 @@ class CachedDecode(DecodeEngineBase):
                 D.moe_router(h2, lw.router, lw.norm2, eps, k, lw.expert_bias,
                              self.router_scratch, idx, wts, pdl=pdl)
                 if self.expert_scratch is not None and narrow.pays_shared(lw.experts_gate_up, nb, k) and \
-                        D._several(nb, lw.experts_gate_up, h2, lw.norm2):
+                        D._several(nb, lw.experts_gate_up, h2, lw.norm2, swiglu=True):
                     narrow.expert_ffn(h2, idx, wts, lw.experts_gate_up, lw.experts_down, lw.norm2, eps, residual=h2,
                                       out=h, scratch=self.expert_scratch, pdl=pdl)
                     continue

@@ -15,7 +15,7 @@ import torch
 
 from .. import _lib
 from . import narrow
-from .weights import LinearWeight, W_Q4
+from .weights import LinearWeight, W_BF16, W_Q4
 
 _MAXB = 4
 _Q4_PATH = os.environ.get("RMLX_Q4_PATH", "auto")
@@ -108,15 +108,48 @@ def set_q4_path(path: str) -> None:
     _Q4_PATH = path
 
 
-def _several(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[torch.Tensor] = None) -> bool:
+def _several(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[torch.Tensor] = None, swiglu: bool = False) -> bool:
     """Several rows: the weight-streaming kernel of ``ops/narrow.py``, which multiplies eight rows for the price of one
     (4-bit 9216 x 4096 at 8 rows: 11 us, 39 on the tensor-core mat-vec, 30 on the streaming kernel), unless the weight is so
-    small that its fixed part exceeds two or three passes of the per-row kernels. ``q4_path`` and the streaming switch away
-    from their defaults keep the kernels that they name."""
+    small that its fixed part exceeds two or three passes of the per-row kernels, or bf16 and so large that two or three rows
+    stream at the copy bandwidth anyway. ``q4_path`` and the streaming switch away from their defaults keep the kernels that they
+    name."""
     # two rows of 4-bit weights: a 16384 x 2048 projection 9 us against 11, a 3072 x 2048 one 6 against 5
     least = 0 if b >= 4 else 1 << 24 if b == 2 and w.kind == W_Q4 else 1 << 20
     return (b >= 2 and _STREAM and q4_path() == "auto" and w.n * w.k >= least and narrow.supported(w) and
-            x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and (norm_w is None or norm_w.data_ptr() % 16 == 0))
+            x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and (norm_w is None or norm_w.data_ptr() % 16 == 0) and
+            not (b <= 3 and w.kind == W_BF16 and not swiglu and _rows_stream(b, w.n * w.k, w.k, norm_w is not None)))
+
+
+def _rows_stream(b: int, entries: int, k: int, norm: bool) -> bool:
+    """Whether the per-row kernel reads a bf16 projection as fast for two or three rows as the weight-streaming one does.
+
+    It holds the rows of x in shared memory in fp32, which up to about 120 KB leaves it the copy bandwidth. Measured (us,
+    weight-streaming / per-row). Two rows with a norm, whose product takes two tiles: 16384 x 2048 17 / 18, 32768 x 2048 28 / 28,
+    28672 x 4096 49 / 45, 4096 x 8192 27 / 19, 151936 x 4096 233 / 197, 50000 x 8192 290 / 132; without: 16384 x 2048 14 / 16, 4096 x
+    8192 16 / 18, 28672 x 4096 44 / 42, 4096 x 14336 29 / 24, 151936 x 4096 221 / 195, 8192 x 28672 87 / 148. Three rows with a norm:
+    28672 x 4096 50 / 53, 65536 x 4096 103 / 103, 100000 x 4096 157 / 148, 151936 x 4096 244 / 220, 4096 x 14336 50 / 54."""
+    if b * k > 30720:
+        return False
+    if b == 2:
+        return k > 2048 or entries > 1 << 27 if norm else k > 8192 or entries > 1 << 26
+    return entries > 1 << 28
+
+
+def projects_apart(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[torch.Tensor] = None) -> bool:
+    """Whether several rows' merged QKV projection runs on its own, on a kernel that takes eight rows per pass (``_several``, or the
+    tensor-core mat-vec of 4-bit weights), with the rotation and the append as a launch after it, rather than in one launch per
+    four rows with both in its epilogue (``rms_qkv_rope``).
+
+    Measured on whole steps of four layers (us, apart / one launch), bf16: 3072 x 2048 258 / 244 at 2 rows, 264 / 252 at 3,
+    296 / 285 at 4; 6144 x 4096 552 / 518, 556 / 541, 567 / 592; 9216 x 4096 (two layers) 618 / 612, 743 / 745, 894 / 897. From five
+    rows on the one launch is two. 8-bit: 3072 x 2048 245 / 238 at 2 rows, 245 / 252 at 3; 9216 x 4096 (two layers) 460 / 466 at 2:
+    always apart, where the sums are fp32 (the per-row kernel adds 8-bit products in fp16)."""
+    if b < 2 or w.kind == W_Q4:
+        return b >= 2
+    if w.kind == W_BF16 and b <= (4 if w.n * w.k <= 1 << 23 else 3):
+        return False
+    return _several(b, w, x, norm_w)
 
 
 def _copied_whole(w: LinearWeight) -> bool:
@@ -197,7 +230,7 @@ def rms_gate_up_swiglu(x: torch.Tensor, w: LinearWeight, norm_w: Optional[torch.
     i = w.n // 2
     if out is None:
         out = torch.empty(b, i, dtype=torch.bfloat16, device=x.device)
-    if w.n % 32 == 0 and _several(b, w, x, norm_w):
+    if w.n % 32 == 0 and _several(b, w, x, norm_w, swiglu=True):
         return narrow.narrow_gemm(x, w, norm_w, eps, out=out, swiglu=True, pdl=pdl)
     lib, st = _lib.cuda(), _lib.stream_ptr()
     if _stream("gate_up", w):

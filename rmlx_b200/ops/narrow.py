@@ -39,16 +39,20 @@ def pays(w: LinearWeight, rows: int) -> bool:
 
     Measured (us, this kernel / the tiles). 4-bit, 9216 x 4096: 16 / 28 at 16 rows, 30 / 28 at 32, 40 / 29 at 64; 28672 x 4096:
     31 / 47, 55 / 47, 106 / 45; 4096 x 8192: 21 / 53, 48 / 54, 62 / 57: up to 16 rows, and up to 32 where a few rows of W leave
-    the tiles less than half of the SMs. 8-bit weights would be expanded first (53 us for 28672 x 4096). bf16, 9216 x 4096:
-    20 / 28 at 16 rows; 28672 x 4096: 46 / 45: eight rows, and 16 for up to 16384 rows of W. Weights of less than a million
-    entries take a tile's time anyway."""
-    n = w.n
-    if rows < 1 or rows > 64 or n * w.k < 1 << 20:
+    the tiles less than half of the SMs; above eight rows of a K that x does not fit into its buffer for, the tiles catch up on
+    large weights (28672 x 8192 59 / 72 at 12 rows, 57344 x 8192 156 / 139, 128256 x 8192 249 / 275; 151936 x 4096 146 / 195).
+    8-bit weights would be expanded first (53 us for 28672 x 4096). bf16, 9216 x 4096: 20 / 28 at 16 rows; 28672 x 4096: 46 / 45:
+    eight rows, and 16 for up to 16384 rows of W; large weights stream at the copy bandwidth on the tiles too (at 5 rows
+    28672 x 8192 89 / 119, 65536 x 4096 101 / 103, 151936 x 4096 227 / 214; at 8 rows 32768 x 4096 53 / 72, 28672 x 8192 89 / 84,
+    65536 x 4096 101 / 100). Weights of less than a million entries take a tile's time anyway."""
+    n, k = w.n, w.k
+    entries = n * k
+    if rows < 1 or rows > 64 or entries < 1 << 20:
         return False
     if w.kind == W_BF16:
-        ok = rows <= 8 or (rows <= 16 and n <= 16384)
+        ok = (rows <= 8 and entries <= (1 << 27 if rows > 5 else 1 << 28)) or (rows <= 16 and n <= 16384)
     elif w.kind == W_Q4:
-        ok = rows <= 16 or (rows <= 32 and n <= 4096)
+        ok = rows <= 8 or (rows <= 16 and (k <= 4096 or entries <= 1 << 28)) or (rows <= 32 and n <= 4096)
     else:
         ok = rows <= 16 or (rows <= 32 and n >= 8192)
     return ok and supported(w)

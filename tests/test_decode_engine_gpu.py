@@ -321,14 +321,14 @@ def test_decode_with_8bit_kv_cache(dev, use_graph):
             eng.set_next_tokens([toks[i + 1]])
 
 
-@pytest.mark.parametrize("quant", [None, "q8", "q4"])
+@pytest.mark.parametrize("quant,rows", [(None, 3), (None, 4), (None, 5), ("q8", 5), ("q4", 3), ("q4", 5)])
 @pytest.mark.parametrize("traditional", [False, True])
-def test_several_rows_round_keys_once(dev, quant, traditional):
-    """Several rows project with one kernel and rotate with the next: keys and queries are rounded to bf16 once, after the
+def test_several_rows_round_keys_once(dev, quant, rows, traditional):
+    """Several rows project with one kernel and rotate with the next, or in one launch (bf16, up to four): keys and queries are rounded to bf16 once, after the
     rotation. Per element: that rounding (2^-8 of the value at most) and the projection's own error, for 4-bit and 8-bit weights the
     fp16 rounding of x times the norm's weight (2^-11 per term at most, so 2.1e-4 of the root mean square; five times that),
     for bf16 weights fp32 sums (2e-5). A second rounding before the rotation moves an element by up to 2^-8 of its pair's other half."""
-    rows, at = 5, 3
+    at = 3
     cfg = TransformerConfig(hidden_size=512, num_heads=8, num_kv_heads=4, head_dim=64, num_layers=1, vocab_size=256,
                             max_seq_len=64, rope_theta=1e4, rope_traditional=traditional,
                             ff_type=FeedForwardType.gated(512), name="one-layer").validate()
@@ -339,7 +339,7 @@ def test_several_rows_round_keys_once(dev, quant, traditional):
         cache.reserve(s, at)
         cache.commit(s, at)
     eng = CachedDecode(model, cache, max_batch=rows)
-    tokens = [3, 50, 71, 9, 200]
+    tokens = [3, 50, 71, 9, 200][:rows]
     eng.bind(range(rows), tokens)
     eng.reserve(1)
     eng.step()

@@ -240,3 +240,17 @@ def test_sums_of_bf16_weights(dev, k, norm):
     want = (xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double() if norm else xd) @ wd.t()
     for shares in (0, 1):
         assert _rel(narrow.narrow_gemm(x, w, nw, 1e-6, out_dtype=torch.float32, shares=shares), want) < 5e-7
+
+
+@pytest.mark.parametrize("rows", [2, 3, 4])
+@pytest.mark.parametrize("n,k,norm", [(1024, 2048, True), (1024, 4096, True), (1024, 8192, False), (512, 9216, False), (640, 15424, False)])
+def test_bf16_rows_on_either_side_of_the_rule(dev, rows, n, k, norm):
+    """Two and three rows of bf16 weights stay on the per-row kernels where those stream as fast: both add in fp32, so the error does
+    not tell which one ran (random walk of K / 64 additions; the per-row kernels add K / 32 per lane and the lanes in a tree)."""
+    from rmlx_b200.ops import decode as D
+    w, wd, x, g = _case(dev, None, n, k, rows, seed=13)
+    nw = (torch.rand(k, device=dev, generator=g) + 0.5).to(torch.bfloat16) if norm else None
+    xd = x.double()
+    want = (xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double() if norm else xd) @ wd.t()
+    assert D._several(rows, w, x, nw) == (rows == 4 or rows * k > 30720 or (rows == 2 and not (k > (2048 if norm else 8192))) or rows == 3)
+    assert _rel(D.rms_gemv(x, w, nw, 1e-6, out_dtype=torch.float32), want) < 1e-6
