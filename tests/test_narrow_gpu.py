@@ -254,3 +254,36 @@ def test_bf16_rows_on_either_side_of_the_rule(dev, rows, n, k, norm):
     want = (xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double() if norm else xd) @ wd.t()
     assert D._several(rows, w, x, nw) == (rows == 4 or rows * k > 30720 or (rows == 2 and not (k > (2048 if norm else 8192))) or rows == 3)
     assert _rel(D.rms_gemv(x, w, nw, 1e-6, out_dtype=torch.float32), want) < 1e-6
+
+
+# the even split: clusters of which every block takes a ragged share of K, more tiles per cluster than fit its sums at once
+#, rows of W beyond what a cluster's buffers hold, experts on clusters
+@pytest.mark.parametrize("kind,n,k,rows,shares", [("q4", 80, 2560, 16, 4), ("q8", 208, 3584, 11, 2), ("q4", 72000, 4096, 16, 2),
+                                                  ("q8", 64, 33280, 3, 0), ("q4", 32, 32768, 12, 0)])
+def test_clusters(dev, kind, n, k, rows, shares):
+    from rmlx_b200.ops import narrow
+    w, _, x, g = _case(dev, kind, min(n, 8000), k, rows, seed=7)
+    if n > 8000:                                         # the reference of 8000 rows nine times over
+        w = type(w)(w.kind, *(t.repeat(n // 8000, 1) for t in (w.w, w.scales, w.biases)))
+    want = (x.double() @ w.dequantized()[:8000].double().t()).repeat(1, max(1, n // 8000))
+    got = [narrow.narrow_gemm(x, w, out_dtype=torch.float32, shares=shares) for _ in range(3)]
+    assert _rel(got[0], want) < 2e-5 and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("kind", ["q4", "q8"])
+@pytest.mark.parametrize("k,tiles,shares", [(8192, 1, 0), (3072, 2, 2), (512, 1, 1)])
+def test_experts_on_clusters(dev, kind, k, tiles, shares):
+    """No rows, one row and several passes of rows per expert."""
+    from rmlx_b200.ops import narrow
+    counts = [0, 1, 8, 0, 19, 3, 33, 0]
+    rows = sum(counts)
+    w, wd, x, g = _case(dev, kind, 112, k, rows, experts=len(counts), seed=8)
+    offsets = torch.tensor([0] + counts, device=dev).cumsum(0).to(torch.int32)
+    order = torch.randperm(rows, device=dev, generator=g).to(torch.int32)
+    got = narrow.narrow_gemm(x, w, out_dtype=torch.float32, offsets=offsets, order=order, rows=rows, tiles=tiles, shares=shares)
+    at = 0
+    for e, c in enumerate(counts):
+        r = order[at:at + c].long()
+        at += c
+        if c:
+            assert _rel(got[r], x[r].double() @ wd[e].t()) < 2e-5
