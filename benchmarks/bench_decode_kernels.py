@@ -142,7 +142,7 @@ def main():
     fsc = D.FlashDecodeScratch(B, HQ, HKV, HD, splits, dev)
     fcl = D.FlashDecodeScratch(B, HQ, HKV, HD, splits, dev, max_len=ctx)
     if fcl.clusters > 0:
-        add(f"flash_decode ctx{ctx} clusters {fcl.clusters & 0xff}x{fcl.clusters >> 8}",
+        add(f"flash_decode ctx{ctx} clusters {fcl.clusters & 0xffff}x{fcl.clusters >> 16}",
             [(lambda i=i: D.flash_decode_paged(q, kcs[i], vcs[i], bt, sl, None, None, fcl, out=ao))
              for i in range(ncp)], B * ctx * HKV * HD * 2 * 2)
     add(f"flash_decode ctx{ctx} splits{splits}",

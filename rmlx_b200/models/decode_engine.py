@@ -302,7 +302,7 @@ class CachedDecode(DecodeEngineBase):
                                 traditional=cfg.rope_traditional, pdl=pdl, **self.cache.sb(li))
             D.flash_decode_paged(q, self.cache.k[li], self.cache.v[li], block_table,
                                  seq_lens, m.scale, splits, fd_scratch,
-                                 cfg.sliding_window, out=attn, pdl=pdl, **self.cache.sb(li))
+                                 cfg.sliding_window, out=attn, pdl=pdl, settled=True, **self.cache.sb(li))
             a2 = attn.view(nb, -1)
             if tp:
                 self.comm.gemv_allreduce(a2, lw.wo, residual=h, out=h2, pdl=pdl)

@@ -247,7 +247,8 @@ class BatchedDecode:
             sp = self._splits_arg or D.default_splits(
                 nb, m.hkv, _lib.cuda().rmlx_flash_decode_gtiles(m.hq, m.hkv),
                 self.cache.max_blocks_per_seq * 16)
-            self._fd[nb] = (sp, D.FlashDecodeScratch(nb, m.hq, m.hkv, cfg.head_dim, sp, m.device))
+            self._fd[nb] = (sp, D.FlashDecodeScratch(nb, m.hq, m.hkv, cfg.head_dim, sp, m.device, max_len=None if self._splits_arg
+                                                     else self.cache.max_blocks_per_seq * 16))
         return self._fd[nb]
 
     def bucket(self) -> int:

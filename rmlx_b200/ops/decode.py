@@ -400,10 +400,8 @@ def moe_down(act: torch.Tensor, w: LinearWeight, idx: torch.Tensor, wts: torch.T
 
 
 _lib.register_cuda_sigs({
-    "rmlx_flash_decode_cluster_plan": ("iii", "i"),
-    "rmlx_flash_decode_cluster_part_o_elems": ("iii", "q"),
-    "rmlx_flash_decode_cluster_part_ml_elems": ("ii", "q"),
-    "rmlx_flash_decode_cluster": ("pppppppppiiiiiiifip", "i"),
+    "rmlx_flash_decode_cluster_plan": ("iiiii", "i"),
+    "rmlx_flash_decode_cluster": ("ppppppppiiiiiiifiip", "i"),
 })
 _FD_CLUSTER = os.environ.get("RMLX_FLASH_DECODE_CLUSTER", "1") != "0"
 
@@ -411,10 +409,10 @@ _FD_CLUSTER = os.environ.get("RMLX_FLASH_DECODE_CLUSTER", "1") != "0"
 class FlashDecodeScratch:
     """Split-KV scratch: partial outputs, (max, sum) pairs and the per-tile ticket counters.
 
-    With ``max_len`` given, the scratch also plans the cluster kernel (flash_decode_cluster.cu:
-    thread-block clusters merging through distributed shared memory), which takes over when a
-    few sequences have to fill the machine; ``clusters`` is then its plan
-    ((cluster size << 8) | clusters per tile)."""
+    With ``max_len`` given, the scratch also plans the cluster kernel (flash_decode_cluster.cu: a
+    thread-block cluster per tile, merging through distributed shared memory), which takes over unless
+    ``RMLX_FLASH_DECODE_CLUSTER=0``; ``clusters`` and, for the 8-bit cache, ``clusters_q8`` are its
+    plans ((cluster size << 16) | clusters; 0: not a shape of it)."""
 
     def __init__(self, batch: int, hq: int, hkv: int, head_dim: int, splits: int, device,
                  max_len: Optional[int] = None):
@@ -426,19 +424,12 @@ class FlashDecodeScratch:
                                    dtype=torch.float32, device=device)
         self.tickets = torch.zeros(lib.rmlx_flash_decode_ticket_elems(batch, hq, hkv),
                                    dtype=torch.int32, device=device)
-        self.clusters = 0
+        self.tiles = batch * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv)
+        self.clusters = self.clusters_q8 = 0
         if max_len is not None and _FD_CLUSTER:
-            tiles = batch * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv)
             with torch.cuda.device(device):
-                self.clusters = int(lib.rmlx_flash_decode_cluster_plan(tiles, int(max_len), head_dim))
-            if (self.clusters & 0xff) > 1:
-                self.c_part_o = torch.empty(
-                    lib.rmlx_flash_decode_cluster_part_o_elems(tiles, self.clusters & 0xff, head_dim),
-                    dtype=torch.float32, device=device)
-                self.c_part_ml = torch.empty(
-                    lib.rmlx_flash_decode_cluster_part_ml_elems(tiles, self.clusters & 0xff),
-                    dtype=torch.float32, device=device)
-                self.c_tickets = torch.zeros(tiles, dtype=torch.int32, device=device)
+                self.clusters, self.clusters_q8 = (int(lib.rmlx_flash_decode_cluster_plan(batch, self.tiles, int(max_len), head_dim, q8))
+                                                   for q8 in (0, 1))
 
 
 def default_splits(batch: int, hkv: int, gtiles: int, max_len: int, sm_count: int = 148) -> int:
@@ -455,11 +446,12 @@ def flash_decode_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
                        scratch: Optional[FlashDecodeScratch] = None, window: int = 0,
                        out: Optional[torch.Tensor] = None, pdl: bool = False,
                        k_sb: Optional[torch.Tensor] = None,
-                       v_sb: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       v_sb: Optional[torch.Tensor] = None, settled: bool = False) -> torch.Tensor:
     """q [B, Hq, D] bf16; caches [blocks, Hkv, 16, D] bf16; block_table int32 [B, max_blocks];
     seq_lens int32 [B] (context length including the current token). With ``k_sb`` / ``v_sb``
     (bf16 [blocks, Hkv, 16, D/64, 2]) the caches are the uint8 codes of the 8-bit format and the
-    kernel expands pages in shared memory."""
+    kernel expands pages in shared memory. ``settled`` (with ``pdl``): no kernel that may still run writes
+    lengths, tables, or pages other than the one of a sequence's last token."""
     _lib.require_cuda_tensor(q, k_cache, v_cache, block_table, seq_lens)
     b, hq, d = q.shape
     hkv, page = k_cache.shape[1], k_cache.shape[2]
@@ -477,6 +469,15 @@ def flash_decode_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
         out = torch.empty_like(q)
     if k_sb is not None:
         assert k_cache.dtype == torch.uint8 and v_sb is not None and k_sb.dtype == torch.bfloat16
+    plan = 0 if scratch is None or splits != scratch.splits else scratch.clusters if k_sb is None else scratch.clusters_q8
+    if plan and b * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv) <= scratch.tiles:
+        rc = lib.rmlx_flash_decode_cluster(
+            q.data_ptr(), k_cache.data_ptr(), _lib.ptr(k_sb), v_cache.data_ptr(), _lib.ptr(v_sb), block_table.data_ptr(),
+            seq_lens.data_ptr(), out.data_ptr(), b, hq, hkv, d, block_table.stride(0), plan, window, scale, int(settled), int(pdl),
+            _lib.stream_ptr())
+        _lib.check(rc, "flash_decode_cluster")
+        return out
+    if k_sb is not None:
         rc = lib.rmlx_flash_decode_paged_q8(
             q.data_ptr(), k_cache.data_ptr(), k_sb.data_ptr(), v_cache.data_ptr(), v_sb.data_ptr(),
             block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(),
@@ -485,18 +486,6 @@ def flash_decode_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
             None if scratch is None else scratch.tickets.data_ptr(),
             b, hq, hkv, d, block_table.stride(0), splits, window, scale, int(pdl), _lib.stream_ptr())
         _lib.check(rc, "flash_decode_paged_q8")
-        return out
-    if scratch is not None and scratch.clusters > 0 and (splits is None or splits == scratch.splits):
-        nc = scratch.clusters & 0xff
-        rc = lib.rmlx_flash_decode_cluster(
-            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_table.data_ptr(),
-            seq_lens.data_ptr(), out.data_ptr(),
-            scratch.c_part_o.data_ptr() if nc > 1 else None,
-            scratch.c_part_ml.data_ptr() if nc > 1 else None,
-            scratch.c_tickets.data_ptr() if nc > 1 else None,
-            b, hq, hkv, d, block_table.stride(0), scratch.clusters, window, scale, int(pdl),
-            _lib.stream_ptr())
-        _lib.check(rc, "flash_decode_cluster")
         return out
     rc = lib.rmlx_flash_decode_paged(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_table.data_ptr(),
