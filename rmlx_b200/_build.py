@@ -50,7 +50,7 @@ SETS = {
     },
     "post_norm": {
         "cuda": ("kernels/postnorm_rows.cu", "kernels/wkv.cu", "kernels/moe_route.cu",
-                 "kernels/head_gemv.cu", "kernels/gemm_tcgen05.cu", "kernels/xgemm_tcgen05.cu", "kernels/pair_gemm.cu",
+                 "kernels/head_gemv.cu", "kernels/gemm_tcgen05.cu", "kernels/xgemm_tcgen05.cu", "kernels/pair_gemm.cu", "kernels/row_gemm.cu",
                  "kernels/gemm_f32.cu", "kernels/flash_prefill_tc.cu", "kernels/flash_decode_scored.cu",
                  "kernels/attention_any.cu", "kernels/mla_decode.cu", "kernels/parallel_rows.cu", "kernels/postnorm_gemv.cu",
                  "kernels/parallel_gemv.cu", "kernels/misc.cu", "runtime/graph_exec.cu"),
@@ -58,7 +58,7 @@ SETS = {
     },
     "twin_norm": {
         "cuda": ("kernels/twin_norm_rows.cu", "kernels/twin_norm_gemv.cu", "kernels/linear_scan.cu", "kernels/postnorm_rows.cu", "kernels/moe_route.cu",
-                 "kernels/head_gemv.cu", "kernels/gemm_tcgen05.cu", "kernels/xgemm_tcgen05.cu", "kernels/pair_gemm.cu",
+                 "kernels/head_gemv.cu", "kernels/gemm_tcgen05.cu", "kernels/xgemm_tcgen05.cu", "kernels/pair_gemm.cu", "kernels/row_gemm.cu",
                  "kernels/gemm_f32.cu", "kernels/flash_prefill_tc.cu", "kernels/flash_decode_scored.cu",
                  "kernels/attention_any.cu", "kernels/mla_decode.cu", "kernels/parallel_rows.cu", "kernels/postnorm_gemv.cu",
                  "kernels/parallel_gemv.cu", "kernels/misc.cu", "runtime/graph_exec.cu"),
@@ -66,7 +66,8 @@ SETS = {
     },
     "sandwich": {
         "cuda": ("kernels/sandwich_rows.cu", "kernels/sandwich_gemv.cu", "kernels/twin_norm_rows.cu", "kernels/linear_scan.cu",
-                 "kernels/postnorm_rows.cu", "kernels/moe_route.cu", "kernels/gemm_tcgen05.cu", "kernels/xgemm_tcgen05.cu", "kernels/pair_gemm.cu",
+                 "kernels/postnorm_rows.cu", "kernels/moe_route.cu", "kernels/gemm_tcgen05.cu", "kernels/xgemm_tcgen05.cu",
+                 "kernels/pair_gemm.cu", "kernels/row_gemm.cu",
                  "kernels/gemm_f32.cu", "kernels/flash_prefill_tc.cu", "kernels/flash_decode_scored.cu",
                  "kernels/attention_any.cu", "kernels/parallel_rows.cu", "kernels/postnorm_gemv.cu",
                  "kernels/parallel_gemv.cu", "kernels/misc.cu", "runtime/graph_exec.cu"),

@@ -28,7 +28,7 @@ from ..runtime.graph import GraphCache, bucket_for
 from ..ops.attention import flash_prefill_paged
 from ..ops.gemm import GemmStatus, gemm_bf16
 from ..ops.grouped import moe_prefill_ffn
-from ..ops.quantized import pair_pays, qmm, xgemm
+from ..ops.quantized import pair_pays, qmm, row_gemm, row_supported, xgemm
 from ..ops.weights import LinearWeight, W_BF16, W_Q4
 
 
@@ -151,6 +151,9 @@ class _Layers:
             if w.lm_head.kind == W_BF16 and w.lm_head.k % 8 == 0:
                 from ..ops.gemm import gemm_bf16_f32       # accumulator stored unrounded
                 out = gemm_bf16_f32(xn, w.lm_head.w)
+            elif w.lm_head.kind == W_Q4 and r <= 160 and row_supported(
+                    xn, w.lm_head, out := torch.empty(r, w.lm_head.n, dtype=torch.float32, device=m.device)):
+                row_gemm(xn, w.lm_head, out=out)           # fp32, unrounded: 140 us for 151936 x 4096 at 64 rows, 172 and a cast
             else:
                 out = _mm(xn, w.lm_head).float()
         if m.allgather_logits is not None and m.layout.world > 1 and w.lm_head.n != cfg.vocab_size:

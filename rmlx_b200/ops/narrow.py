@@ -38,9 +38,8 @@ def pays(w: LinearWeight, rows: int) -> bool:
     """Whether a plain projection of ``rows`` rows is faster here than on the 128-row tensor-core tiles (and takes this weight).
 
     Measured (us, this kernel / the tiles). 4-bit: 28672 x 4096 25 / 39 at 16 rows, 43 / 39 at 24; 28672 x 8192 44 / 72 at 16, 75 / 72
-    at 24; 9216 x 4096 15 / 26 at 16, 20 / 26 at 32, 31 / 26 at 48; 4096 x 8192 20 / 45 at 32, 36 / 45 at 64; 4096 x 14336 37 / 74, 60 /
-    74; 4096 x 4096 14 / 25, 24 / 25: up to 16 rows, up to 32 for moderate widths, and up to 64 where a few rows of W leave the tiles
-    less than half of the SMs. 8-bit weights would be expanded first (16384 x 2048 at 64 rows 33 / 50, 28672 x 4096 99 / 165, 3072 x
+    at 24; 9216 x 4096 15 / 26 at 16, 20 / 26 at 32, 31 / 26 at 48; 4096 x 8192 20 / 45 at 32; 4096 x 14336 37 / 74: up to 16 rows, and up to
+    32 for moderate widths (from there 9216 x 4096 takes 22 us on the tensor-core tiles of W's rows, 4096 x 14336 25). 8-bit weights would be expanded first (16384 x 2048 at 64 rows 33 / 50, 28672 x 4096 99 / 165, 3072 x
     2048 17 / 17). bf16, 9216 x 4096: 20 / 28 at 16 rows; 28672 x 4096: 46 / 45:
     eight rows, and 16 for up to 16384 rows of W; large weights stream at the copy bandwidth on the tiles too (at 5 rows
     28672 x 8192 89 / 119, 65536 x 4096 101 / 103, 151936 x 4096 227 / 214; at 8 rows 32768 x 4096 53 / 72, 28672 x 8192 89 / 84,
@@ -52,17 +51,19 @@ def pays(w: LinearWeight, rows: int) -> bool:
     if w.kind == W_BF16:
         ok = (rows <= 8 and entries <= (1 << 27 if rows > 5 else 1 << 28)) or (rows <= 16 and n <= 16384)
     elif w.kind == W_Q4:
-        ok = rows <= 16 or (rows <= 32 and n <= 12288) or n <= 4096
+        ok = rows <= 16 or (rows <= 32 and n <= 12288)
     else:
         ok = True
     return ok and supported(w)
 
 
 def pays_grouped(gate_up: LinearWeight, down: LinearWeight, pairs: int) -> bool:
-    """Whether an expert feed-forward of ``pairs`` (row, slot) pairs is faster here: up to sixteen pairs per expert (128 experts
-    of 4096 x 1536, both projections in 4 bits, us, here / on the tiles: 273 / 892 at 512 pairs, 382 / 764 at 1024, 577 / 765 at 2048).
-    bf16 experts are as fast on the tiles (523 + 275 against 549 + 305 at 512 pairs)."""
-    return (gate_up.kind in (W_Q4, W_Q8) and down.kind == gate_up.kind and 0 < pairs <= 16 * gate_up.experts and
+    """Whether an expert feed-forward of ``pairs`` (row, slot) pairs is faster here: up to twelve pairs per expert in 4 bits, sixteen in 8
+    (128 experts of 4096 x 1536, both projections, us, here / on the tiles: 4-bit 382 / 470 at 1024 pairs, 466 / 480 at 1600, 577 / 490 at
+    2048; 8-bit on expanded weights 586 / 815 at 1024, 748 / 894 at 2048). bf16 experts are as fast on the tiles (523 + 275 against 549 + 305
+    at 512 pairs)."""
+    most = 12 if gate_up.kind == W_Q4 else 16
+    return (gate_up.kind in (W_Q4, W_Q8) and down.kind == gate_up.kind and 0 < pairs <= most * gate_up.experts and
             gate_up.n * gate_up.k >= 1 << 20 and supported(gate_up) and supported(down))
 
 

@@ -20,6 +20,8 @@ _lib.register_cuda_sigs({
     "rmlx_xgemm": ("ipppppppiiiiiiiifpip", "i"),
     "rmlx_pair_gemm_supported": ("iiiiii", "i"),
     "rmlx_pair_gemm": ("ipppppppiiiiiiifpip", "i"),
+    "rmlx_row_gemm_supported": ("iiiii", "i"),
+    "rmlx_row_gemm": ("pppppippiiiiiiifipip", "i"),
     "rmlx_moe_scatter_rows": ("pipppppiiiip", "i"),
     "rmlx_moe_combine": ("ppppipiiiip", "i"),
 })
@@ -45,6 +47,9 @@ def xgemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = N
     # the epilogue reads the residual with the result's row stride
     assert residual is None or (residual.dim() == 2 and residual.shape[0] >= m and residual.shape[1] >= n and
                                 residual.stride(1) == 1 and (m == 1 or residual.stride(0) == out.stride(0)))
+    if bn == 0 and w.kind == W_Q4 and row_pays(m, n, k, e) and row_supported(x, w, out, residual, swiglu) and \
+            (residual is None or (e == 0 and not swiglu and residual.stride(0) == out.stride(0))):
+        return row_gemm(x, w, residual, out, offsets, swiglu, gate_limit, pdl)
     if bn == 0 and m > 128 and pair_pays(w.kind, m, n, k, e) and (not swiglu or (n % 256 == 0 and residual is None)) and \
             (residual is None or e == 0) and (w.kind != W_Q4 or not w.scales_f16) and (w.kind != W_Q4 or k % 512 == 0) and \
             k % 8 == 0 and _pair_ready(x, out, residual) and out.dtype == torch.bfloat16:
@@ -55,6 +60,54 @@ def xgemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = N
                                 gate_limit,
                                 GemmStatus.get(x.device).data_ptr(), int(pdl), _lib.stream_ptr())
     _lib.check(rc, "xgemm")
+    return out
+
+
+def row_pays(m: int, n: int, k: int, experts: int = 0) -> bool:
+    """Whether 4-bit weights go to the kernel whose 128 product rows are rows of W and whose columns are the rows of x that there are
+    (csrc/kernels/row_gemm.cu), rather than to tiles of 128 or 256 rows of x.
+
+    Measured (us, this kernel / the tiles). 128 experts of 4096 x 1536, gate and up + down: 298 + 159 / 552 + 321 at 512 rows in all, 324 +
+    167 / 429 + 242 at 2048, 336 + 186 / 439 + 250 at 8192, 404 + 264 / 637 + 415 at 16384, 750 + 482 / 872 + 644 at 24000, 913 + 544 / 889 +
+    735 at 32768. One weight: 9216 x 4096 20 / 27 at 24 rows, 24 / 27 at 64, 28 / 27 at 96; 28672 x 4096 40 / 47 at 24, 45 / 48 at 96; 4096 x
+    8192 22 / 47 at 64, 26 / 47 at 96; 4096 x 14336 28 / 75 at 64; 151936 x 4096 140 / 172 at 64; 512 rows of 9216 x 4096 44 / 34; 1024 x 256
+    at 16 rows 10 / 9."""
+    return m <= 256 * experts if experts else m <= (96 if n <= 8192 or n > 16384 else 80) and n * k >= 1 << 23
+
+
+def row_supported(x: torch.Tensor, w: LinearWeight, out: torch.Tensor, residual: Optional[torch.Tensor] = None,
+                  swiglu: bool = False) -> bool:
+    """What ``rmlx_row_gemm`` asks of its operands: bf16 scales, 16-byte rows of x, results on 4 bytes."""
+    return (not w.scales_f16 and x.data_ptr() % 16 == 0 and out.data_ptr() % 4 == 0 and out.stride(1) == 1 and
+            (residual is None or (residual.data_ptr() % 4 == 0 and out.dtype == torch.bfloat16)) and
+            (w.w.data_ptr() | w.scales.data_ptr() | w.biases.data_ptr()) % 16 == 0 and
+            w.w.is_contiguous() and w.scales.is_contiguous() and w.biases.is_contiguous() and
+            bool(_lib.cuda().rmlx_row_gemm_supported(w.n, w.k, x.stride(0), out.stride(0), int(swiglu))))
+
+
+def row_gemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+             offsets: Optional[torch.Tensor] = None, swiglu: bool = False, gate_limit: float = 0.0, pdl: bool = False,
+             out_dtype=torch.bfloat16, split: int = 0) -> torch.Tensor:
+    """``xgemm`` with 4-bit weights on csrc/kernels/row_gemm.cu; fp32 results are the accumulators as they are. ``split``: blocks that
+    share K (1, 2, 4, 8; 0: chosen; experts: 1)."""
+    _lib.require_cuda_tensor(x, w.w)
+    assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and w.kind == W_Q4
+    m, k = x.shape
+    n = w.n
+    assert k == w.k
+    e = w.experts if offsets is not None else 0
+    if offsets is not None:
+        assert offsets.dtype == torch.int32 and offsets.numel() == e + 1
+    if out is None:
+        out = torch.empty(m, n // 2 if swiglu else n, dtype=out_dtype, device=x.device)
+    assert out.dtype in (torch.bfloat16, torch.float32) and out.shape[0] >= m and out.shape[1] >= (n // 2 if swiglu else n)
+    assert residual is None or (residual.dtype == torch.bfloat16 and residual.shape[0] >= m and residual.shape[1] >= n and
+                                residual.stride(1) == 1 and (m == 1 or residual.stride(0) == out.stride(0)))
+    rc = _lib.cuda().rmlx_row_gemm(x.data_ptr(), w.w.data_ptr(), w.scales.data_ptr(), w.biases.data_ptr(), out.data_ptr(),
+                                   int(out.dtype == torch.float32), _lib.ptr(residual), _lib.ptr(offsets), e, m, n, k, x.stride(0),
+                                   out.stride(0), int(swiglu), gate_limit, split, GemmStatus.get(x.device).data_ptr(), int(pdl),
+                                   _lib.stream_ptr())
+    _lib.check(rc, "row_gemm")
     return out
 
 
