@@ -328,9 +328,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           sws[i] = x_lds32(scb + i * 8);
           bws[i] = x_lds32(scb + kPairRows * 16 + i * 8);
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(sc_empty + sslot);
-        if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
 #pragma unroll
         for (int k4 = 0; k4 < 2; ++k4) {
           if (!mbar_wait(raw_full + rstage, rphase, abort_flag)) { ok = false; break; }
@@ -360,6 +357,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           stage += kPairGroups;
           if (stage >= STAGES) { stage -= STAGES; phase ^= 1u; }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sc_empty + sslot);     // only once the scales have been used (xgemm_kernel.cuh says why)
+        if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
       }
     }
   }

@@ -385,8 +385,6 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       uint4 w[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) w[c] = x_lds(raw0 + slot * RgSmem::kRaw + ((((i & 1) * 4 + c) ^ (r & 7)) << 4));
-      __syncwarp();
-      if (lane == 0) { mbar_arrive(sc_empty + sc); mbar_arrive(raw_empty + slot); }
       uint32_t o[32];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -407,7 +405,8 @@ row_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(full + group);
+      // what was read is given back only here, where its values have been used (xgemm_kernel.cuh says why)
+      if (lane == 0) { mbar_arrive(full + group); mbar_arrive(sc_empty + sc); mbar_arrive(raw_empty + slot); }
     }
   }
 

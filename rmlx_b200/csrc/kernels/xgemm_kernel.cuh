@@ -685,9 +685,6 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             bws[it][i] = x_lds32(scb + BN * 16 + i * (2 * GROUPS));
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(sc_empty + sslot);       // the slot can be refilled already
-        if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
 #pragma unroll
         for (int i = 0; i < 8 / GROUPS; ++i) {
           if (!mbar_wait(raw_full + rstage, rphase, abort_flag, LIM)) { ok = false; break; }
@@ -729,6 +726,12 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           stage += GROUPS;
           if (stage >= STAGES) { stage -= STAGES; phase ^= 1u; }
         }
+        // Released only now that the values have been used: a load whose result nobody has waited for may still be queued behind other
+        // warps' stores when the release goes out, and the copy engine then writes the slot under it (released right after the loads, 64-column
+        // tiles with a residual took scales of a later block in 2 to 94 of 100 runs).
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sc_empty + sslot);
+        if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
       }
     }
   } else if (WQ4 && !Ro::kDeep && warp < 6 + kDqWarps) {
@@ -754,9 +757,6 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             bv[it] = *reinterpret_cast<const uint4*>(scb + BN * 16 + (item >> 1) * 16);
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(sc_empty + sslot);       // the slot can be refilled already
-        if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           if (!mbar_wait(raw_full + rstage, rphase, abort_flag, LIM)) { ok = false; break; }
@@ -794,6 +794,9 @@ xgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           if (++rstage == RAW) { rstage = 0; rphase ^= 1u; }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sc_empty + sslot);       // only once the scales have been used, as above
+        if (++sslot == 2) { sslot = 0; sphase ^= 1u; }
       }
     }
   }
