@@ -138,6 +138,11 @@ class NativeBlockManager:
         self._lib.rmlx_bm_table(self._h, seq_id, buf, n)
         return list(buf[:n])
 
+    def write_table(self, seq_id: int, row) -> None:
+        """The sequence's blocks into the front of an int32 host row (contiguous) that has room for them."""
+        if self._lib.rmlx_bm_table(self._h, seq_id, ctypes.cast(row.data_ptr(), _IP), row.numel()) < 0:
+            raise KeyError(seq_id)
+
     def seq_len(self, seq_id: int) -> int:
         return self._lib.rmlx_bm_seq_len(self._h, seq_id)
 

@@ -114,6 +114,11 @@ class BlockManager:
             table.append(self._take())
         return copies
 
+    def write_table(self, seq_id: int, row: torch.Tensor) -> None:
+        """The sequence's blocks into the front of an int32 host row that has room for them."""
+        table = self.tables[seq_id]
+        row[:len(table)] = torch.tensor(table, dtype=torch.int32)
+
     def commit(self, seq_id: int, new_tokens: int) -> None:
         self.lengths[seq_id] += new_tokens
 
@@ -242,6 +247,8 @@ class PagedKvCache:
     to no sequence (idle batch rows write there). A state cannot be rolled back or started from cached
     pages: ``trim`` and ``adopt_prefix`` refuse."""
 
+    _HOST_ROWS = 4                         # pinned copies of a sequence's block table
+
     def __init__(self, num_blocks: int, num_layers: int, kv_heads: int, head_dim: int,
                  dtype=torch.bfloat16, device="cpu", max_seqs: int = 64,
                  max_blocks_per_seq: int = 512, block_size: int = PAGE,
@@ -286,14 +293,15 @@ class PagedKvCache:
         self.max_blocks_per_seq = max_blocks_per_seq
         # row r of the device table belongs to the sequence bound to slot r
         self.block_table = torch.zeros(max_seqs, max_blocks_per_seq, dtype=torch.int32, device=device)
-        self._host_table = torch.zeros(max_seqs, max_blocks_per_seq, dtype=torch.int32,
+        self._host_table = torch.zeros(max_seqs, self._HOST_ROWS, max_blocks_per_seq, dtype=torch.int32,
                                        pin_memory=self.device.type == "cuda")
         self.slot_of: Dict[int, int] = {}
         self._free_slots = list(range(max_seqs - 1, -1, -1))
-        # the pinned row of a slot is the source of an asynchronous copy: the event recorded after
-        # the copy is waited for before the row is written again (by a later update of the same
-        # sequence, or by the next sequence that takes the slot)
-        self._row_copied: Dict[int, "torch.cuda.Event"] = {}
+        # a pinned row is the source of an asynchronous copy: the event recorded after the copy is waited for before the row is
+        # written again. A slot's rows take turns, so that an update (a rollback and the reservation after it) does not wait for
+        # the one before, whose copy is queued behind all that the stream still has to do
+        self._row_copied: Dict[tuple, "torch.cuda.Event"] = {}
+        self._last_row: Dict[int, tuple] = {}        # slot -> (row, stream) of its last update
 
     # -------------------------------------------------------------- sequences
     def add_sequence(self, seq_id: int) -> int:
@@ -313,7 +321,9 @@ class PagedKvCache:
     def free_sequence(self, seq_id: int) -> None:
         self.manager.free_sequence(seq_id)
         slot = self.slot_of.pop(seq_id)
-        self._row_idle(slot)
+        for row in range(self._HOST_ROWS):
+            self._row_idle((slot, row))
+        self._last_row.pop(slot, None)
         self._host_table[slot].zero_()
         self._free_slots.append(slot)
 
@@ -336,25 +346,34 @@ class PagedKvCache:
     def seq_len(self, seq_id: int) -> int:
         return self.manager.seq_len(seq_id)
 
-    def _row_idle(self, slot: int) -> None:
-        """Wait until the last queued copy out of the slot's pinned row has run."""
-        ev = self._row_copied.pop(slot, None)
+    def _row_idle(self, row: tuple) -> None:
+        """Wait until the last queued copy out of a pinned row has run."""
+        ev = self._row_copied.pop(row, None)
         if ev is not None:
             ev.synchronize()
 
     def _sync_slot(self, seq_id: int) -> None:
         slot = self.slot_of[seq_id]
-        table = self.manager.block_table(seq_id)
-        if len(table) > self.max_blocks_per_seq:
+        n = self.manager.num_blocks_of(seq_id)
+        if n > self.max_blocks_per_seq:
             raise OutOfBlocks("sequence exceeds max_blocks_per_seq")
-        self._row_idle(slot)
-        row = self._host_table[slot]
-        row[:len(table)] = torch.tensor(table, dtype=torch.int32)
+        last = self._last_row.get(slot)
+        at = 0 if last is None else (last[0] + 1) % self._HOST_ROWS
+        self._row_idle((slot, at))
+        row = self._host_table[slot, at]
+        self.manager.write_table(seq_id, row)
+        if self.device.type != "cuda":
+            self.block_table[slot].copy_(row)
+            self._last_row[slot] = (at, None)
+            return
+        stream = torch.cuda.current_stream(self.device)
+        if last is not None and last[1] != stream and (slot, last[0]) in self._row_copied:
+            stream.wait_event(self._row_copied[slot, last[0]])     # updates reach the device in their order
         self.block_table[slot].copy_(row, non_blocking=True)
-        if self.device.type == "cuda":
-            ev = torch.cuda.Event()
-            ev.record(torch.cuda.current_stream(self.device))
-            self._row_copied[slot] = ev
+        ev = torch.cuda.Event()
+        ev.record(stream)
+        self._row_copied[slot, at] = ev
+        self._last_row[slot] = (at, stream)
 
     def reserve(self, seq_id: int, new_tokens: int) -> None:
         """Ensure blocks exist for ``new_tokens`` more tokens (doing any copy-on-write) and push
@@ -371,7 +390,7 @@ class PagedKvCache:
                 if self.quantized:
                     self.k_sb[l][dst].copy_(self.k_sb[l][src])
                     self.v_sb[l][dst].copy_(self.v_sb[l][src])
-        if copies or len(self.manager.block_table(seq_id)) != before:
+        if copies or self.manager.num_blocks_of(seq_id) != before:
             self._sync_slot(seq_id)
 
     def commit(self, seq_id: int, new_tokens: int) -> None:
