@@ -195,6 +195,12 @@ def launch_count() -> int:
     return _launch_count
 
 
+def count_launches(n: int) -> None:
+    """Launches made by a native call beyond the one that its ``check`` counts."""
+    global _launch_count
+    _launch_count += n
+
+
 def check(rc: int, what: str) -> None:
     global _launch_count
     _launch_count += 1

@@ -42,10 +42,10 @@ struct FcParams {
   const __nv_bfloat16* q;        // [B, Hq, HD]
   const char *k_cache, *v_cache; // [blocks, Hkv, 16, HD] bf16, or uint8 codes with
   const char *k_sb, *v_sb;       // [blocks, Hkv, 16, HD/64] (scale, bias) bf16 pairs
-  const int* block_table;        // [B, max_blocks]
+  const int* block_table;        // [B, max_blocks], rows table_stride apart (0: one row for all)
   const int* seq_lens;           // [B] tokens in the cache including the current one
   __nv_bfloat16* out;            // [B, Hq, HD]
-  int B, max_blocks, Hq, Hkv, G, gtiles, window, early, CS;
+  int B, max_blocks, table_stride, Hq, Hkv, G, gtiles, window, early, CS;
   float scale_log2;              // softmax scale * log2(e)
 };
 
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kFcThreads, FcShape<HD, KVQ>::PER_SM) flash_de
     if (p_tab0 < 0 || at >= p_tab0 + 32) {
       const int len = p.seq_lens[pw.b], pg = first_page(len) + min(at + lane, pw.n - 1);
       p_tab0 = at;
-      p_tab = len > 0 && RB_BOUNDS(pg, p.max_blocks) ? p.block_table[size_t(pw.b) * p.max_blocks + pg] : 0;   // page 0 is reserved
+      p_tab = len > 0 && RB_BOUNDS(pg, p.max_blocks) ? p.block_table[size_t(pw.b) * p.table_stride + pg] : 0;   // page 0 is reserved
     }
     return __shfl_sync(0xffffffffu, p_tab, at - p_tab0);
   };
@@ -656,7 +656,8 @@ extern "C" int rmlx_flash_decode_cluster_plan(int batch, int tiles, int max_len,
 // plan from rmlx_flash_decode_cluster_plan. k_sb null: bf16 cache, else the 8-bit one. `window` > 0: the last `window` tokens only.
 extern "C" int rmlx_flash_decode_cluster(const void* q, const void* k_cache, const void* k_sb, const void* v_cache, const void* v_sb,
                                       const int* block_table, const int* seq_lens, void* out, int B, int Hq, int Hkv, int HD,
-                                      int max_blocks, int plan, int window, float scale, int early, int pdl, cudaStream_t st) {
+                                      int max_blocks, int table_stride, int plan, int window, float scale, int early, int pdl,
+                                      cudaStream_t st) {
   const int cs = plan >> 16, clusters = plan & 0xffff;
   if (B < 1 || B > kFcMaxBatch || Hkv < 1 || Hq % Hkv || clusters < 1 || cs < 1 || cs > kFcMaxCluster || (cs & (cs - 1))) return -2;
   if ((k_sb == nullptr) != (v_sb == nullptr)) return -2;
@@ -666,7 +667,7 @@ extern "C" int rmlx_flash_decode_cluster(const void* q, const void* k_cache, con
   p.k_sb = static_cast<const char*>(k_sb); p.v_sb = static_cast<const char*>(v_sb);
   p.block_table = block_table; p.seq_lens = seq_lens;
   p.out = static_cast<__nv_bfloat16*>(out);
-  p.B = B; p.max_blocks = max_blocks; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.gtiles = (p.G + 15) / 16; p.window = window;
+  p.B = B; p.max_blocks = max_blocks; p.table_stride = table_stride; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.gtiles = (p.G + 15) / 16; p.window = window;
   p.early = early && pdl; p.CS = cs;
   p.scale_log2 = scale * 1.4426950408889634f;
   if (HD == 128) return k_sb ? fc_launch<128, true>(p, clusters, pdl, st) : fc_launch<128, false>(p, clusters, pdl, st);

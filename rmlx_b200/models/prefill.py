@@ -16,6 +16,9 @@ sums go through the injected ``allreduce``.
 """
 from __future__ import annotations
 
+import array
+import ctypes
+import os
 from typing import List, Optional, Sequence
 
 import torch
@@ -25,10 +28,11 @@ from ..kv.paged import PagedKvCache
 from ..ops import decode as D
 from ..ops import narrow
 from ..runtime.graph import GraphCache, bucket_for
-from ..ops.attention import flash_prefill_paged
+from ..ops.attention import few_rows_attention, few_rows_plan, flash_prefill_paged, prefill_kernel_choice
 from ..ops.gemm import GemmStatus, gemm_bf16
+from ..ops import grouped
 from ..ops.grouped import moe_prefill_ffn
-from ..ops.quantized import pair_pays, qmm, row_gemm, row_supported, xgemm
+from ..ops.quantized import pair_pays, qmm, row_gemm, row_supported, row_tables_ready, tiles_route, xgemm
 from ..ops.weights import LinearWeight, W_BF16, W_Q4
 
 
@@ -161,6 +165,151 @@ class _Layers:
         return out
 
 
+_lib.register_cuda_sigs({
+    "rmlx_prompt_sizes": ("p", "i"),
+    "rmlx_prompt_run": ("ppffppp", "i"),
+})
+
+
+class PromptRun:
+    """A prompt portion from one native call (csrc/runtime/prompt_run.cu): the launches of ``_Layers.run`` with the kernels that it
+    would choose, without the interpreter between them. Pointers, sizes and choices are taken from the model and the cache at every call;
+    kept are only the two tables of numbers. ``run`` returns None for what it does not cover (tensor parallelism, shared experts, weights
+    at odd addresses, one launch at a time for debugging): the caller then goes launch by launch."""
+
+    NARROW, ROW, PAIR, TILES, BF16, EXPAND, WITH_NORM, SWIGLU = 1, 2, 3, 4, 5, 6, 16, 32
+
+    def __init__(self, model):
+        self.m = model
+        self._numbers: list = []            # int32 0, 1, 2, ... and zeros on the device; grown ones are kept beside their successors
+
+    def _tables(self, n: int):
+        if not self._numbers or self._numbers[-1][0].numel() < n:
+            size = max(n, 2 * self._numbers[-1][0].numel() if self._numbers else 8192)
+            dev = self.m.device
+            pair = (torch.arange(size, dtype=torch.int32, device=dev), torch.zeros(size, dtype=torch.int32, device=dev))
+            torch.cuda.current_stream(dev).synchronize()    # from here on any stream may read them
+            self._numbers.append(pair)
+        return self._numbers[-1]
+
+    # ------------------------------------------------------------------ routes
+    def _plain(self, w: LinearWeight, t: int) -> int:
+        """What ``_mm`` does with rows on 16 bytes; 0: not covered."""
+        if t <= 64 and narrow.pays(w, t):
+            return self.NARROW
+        if w.kind == W_BF16:
+            if not w.w.is_contiguous() or w.w.dtype != torch.bfloat16:
+                return 0
+            return self.PAIR if t > 128 and pair_pays(W_BF16, t, w.n, w.k) and tiles_route(w, t) == "pair" else self.BF16
+        if w.kind == W_Q4 and not w.scales_f16 and w.k % 512 == 0:
+            return self._tiles(w, t)
+        return self.EXPAND
+
+    def _tiles(self, w: LinearWeight, t: int, experts: int = 0, swiglu: bool = False) -> int:
+        route = tiles_route(w, t, experts, swiglu)
+        if route == "row" and not row_tables_ready(w):
+            route = tiles_route(w, t, experts, swiglu, row=False)
+        return {"row": self.ROW, "pair": self.PAIR, "tiles": self.TILES}[route]
+
+    def _normed(self, w: LinearWeight, t: int, norm: torch.Tensor) -> int:
+        route = self._plain(w, t)
+        return route | self.WITH_NORM if route == self.NARROW and norm.data_ptr() % 16 == 0 and (w.kind != W_BF16 or t <= 8) else route
+
+    def _gate_up(self, w: LinearWeight, t: int, norm: torch.Tensor) -> int:
+        route = self._normed(w, t, norm)
+        if route & 15 == self.NARROW:
+            return route | self.SWIGLU if w.n % 32 == 0 else route & 15
+        if w.n % 256 == 0 and w.k % 8 == 0 and (w.kind == W_BF16 or (w.kind == W_Q4 and not w.scales_f16 and w.k % 512 == 0)):
+            return 0 if not w.w.is_contiguous() else self._tiles(w, t, swiglu=True) | self.SWIGLU
+        return route
+
+    # ------------------------------------------------------------------ the pass
+    def run(self, token_ids: torch.Tensor, cache: PagedKvCache, seq_id: int, pos0: int) -> Optional[torch.Tensor]:
+        m = self.m
+        cfg, mw = m.cfg, m.w
+        t, d, hd, hq, hkv = token_ids.numel(), cfg.hidden_size, cfg.head_dim, m.hq, m.hkv
+        if m.layout.world != 1 or _lib.debug_serialize() or grouped._NARROW_MAX_AVG_ROWS > 0 or d % 64 or cache.block_size != 16 or \
+                token_ids.dtype != torch.int32 or not token_ids.is_contiguous() or not mw.embed.is_contiguous():
+            return None
+        bf16, pages = torch.bfloat16, (pos0 + t + 15) // 16
+        q8 = cache.quantized
+        row = cache.block_table[cache.slot_of[seq_id]]
+        if row.numel() < pages or mw.embed.dtype != bf16:
+            return None
+        recs = array.array("q")
+        mid = act = dense = xs = y = pairs = most = 0
+        for li, lw in enumerate(mw.layers):
+            n1, n2, kc, vc = lw.norm1, lw.norm2, cache.k[li], cache.v[li]
+            if n1.dtype != bf16 or n2.dtype != bf16 or (n1.data_ptr() | n2.data_ptr()) % 16 or not n1.is_contiguous() or not n2.is_contiguous() \
+                    or not kc.is_contiguous() or not vc.is_contiguous() or kc.shape != vc.shape or kc.shape[3] != hd:
+                return None
+            e = k = 0
+            if lw.router is not None:
+                moe, r = cfg.ff_type.moe, lw.router
+                e, k = moe.num_experts, moe.num_experts_per_token
+                up, down, bias = lw.experts_gate_up, lw.experts_down, lw.expert_bias
+                if lw.shared_gate_up is not None or lw.expert_base or up.experts != e or r.dtype != bf16 or not r.is_contiguous() or \
+                        (bias is not None and (bias.dtype != torch.float32 or not bias.is_contiguous())):
+                    return None
+                pairs, most = max(pairs, t * k), max(most, e)
+                if narrow.pays_grouped(up, down, t * k):
+                    r_up = r_down = self.NARROW
+                    y = max(y, t * k * d * 4)
+                else:
+                    up, down = grouped._expanded_if_needed(up), grouped._expanded_if_needed(down)
+                    if not (grouped._grouped_ok(up) and grouped._grouped_ok(down) and up.w.is_contiguous() and down.w.is_contiguous()):
+                        return None
+                    r_up, r_down = self._tiles(up, t * k, e, True), self._tiles(down, t * k, e)
+                    xs, y = max(xs, t * k * d * 2), max(y, t * k * d * 2)
+                act = max(act, t * k * up.n)
+            else:
+                up, down = lw.w_gate_up, lw.w_down
+                r_up, r_down = self._gate_up(up, t, n2), self._plain(down, t)
+                act, mid = max(act, t * up.n), max(mid, 0 if r_up & self.SWIGLU else t * up.n * 2)
+            r_qkv, r_out = self._normed(lw.wqkv, t, n1), self._plain(lw.wo, t)
+            if not (r_qkv and r_out and r_up and r_down):
+                return None
+            recs.extend((n1.data_ptr(), n2.data_ptr(), kc.data_ptr(), vc.data_ptr(), cache.k_sb[li].data_ptr() if q8 else 0,
+                         cache.v_sb[li].data_ptr() if q8 else 0, 0 if not e else lw.router.data_ptr(),
+                         0 if not e or bias is None else bias.data_ptr(), e, k))
+            for w, route in ((lw.wqkv, r_qkv), (lw.wo, r_out), (up, r_up), (down, r_down)):
+                s, b = w.scales, w.biases
+                if s is not None and not (s.is_contiguous() and b.is_contiguous() and w.w.is_contiguous()):
+                    return None
+                if route & 15 == self.EXPAND:
+                    dense = max(dense, w.n * w.k * 2)
+                recs.extend((w.w.data_ptr(), 0 if s is None else s.data_ptr(), 0 if b is None else b.data_ptr(), w.n, w.k,
+                             w.experts if e else 0, w.kind, int(s is not None and w.scales_f16), route))
+        few = few_rows_plan(t, hq, hkv, hd, pos0 + t, q8)
+        kv_bytes = pages * hkv * 16 * hd * 2 if q8 and not few else 0
+        # one block of work space, in pieces at 256-byte addresses
+        at, offs = 0, []
+        for size in (t * d * 2, t * d * 2, t * d * 2, t * (hq + 2 * hkv) * hd * 2, t * hq * hd * 2, t * hq * hd * 2, act, mid, dense,
+                     kv_bytes, kv_bytes, t * most * 4, pairs * 4, pairs * 4, most * 4,
+                     (most + 1) * 4, pairs * 4, most * 4, pairs * 4, xs, y):
+            offs.append(at)
+            at += (size + 255) & ~255
+        ws = torch.empty(at, dtype=torch.uint8, device=m.device)
+        base = ws.data_ptr()
+        iota, zeros = self._tables(pos0 + t + 1)
+        window = int(cfg.sliding_window or 0)
+        head = array.array("q", (
+            len(mw.layers), t, d, hq, hkv, hd, pos0, window, row.numel(), 16, cache.k[0].shape[0], int(cfg.rope_traditional),
+            int(prefill_kernel_choice(hd, window) == "tc"), int(os.environ.get("RMLX_FLASH_PREFILL_LANES", "0")), pages, few, mw.embed.shape[0],
+            mw.embed.data_ptr(), token_ids.data_ptr(), row.data_ptr(), iota.data_ptr() + 4 * pos0, zeros.data_ptr(), iota.data_ptr(),
+            m.cos.data_ptr(), m.sin.data_ptr(), GemmStatus.get(m.device).data_ptr(), *(base + o for o in offs)))
+        lib = _lib.cuda()
+        words = (ctypes.c_int * 2)()
+        lib.rmlx_prompt_sizes(words)
+        assert tuple(words) == (len(head), len(recs) // len(mw.layers)), "the records of csrc/runtime/prompt_run.cu"
+        launches, what = ctypes.c_int(0), ctypes.c_char_p()
+        rc = lib.rmlx_prompt_run(head.buffer_info()[0], recs.buffer_info()[0], cfg.rms_norm_eps, m.scale, ctypes.byref(launches),
+                                 ctypes.byref(what), _lib.stream_ptr())
+        _lib.count_launches(launches.value - 1)
+        _lib.check(rc, (what.value or b"prompt_run").decode())
+        return ws[:t * d * 2].view(bf16).view(t, d)
+
+
 class NativePrefill:
     """Callable ``(token_ids, cache, seq_id) -> last-token logits [1, vocab]`` (fp32); with
     ``all_logits=True`` the logits of every position of the call, ``[T, vocab]`` (what speculative
@@ -170,6 +319,7 @@ class NativePrefill:
         self.m = model
         self.chunk = chunk
         self.layers = _Layers(model)
+        self.at_once = PromptRun(model)
 
     @torch.no_grad()
     def __call__(self, token_ids: torch.Tensor, cache: PagedKvCache, seq_id: int,
@@ -186,6 +336,12 @@ class NativePrefill:
         hd, hq, hkv = cfg.head_dim, m.hq, m.hkv
         pos0 = cache.seq_len(seq_id)
         cache.reserve(seq_id, t)
+        token_ids = token_ids.to(torch.int32)
+        h = self.at_once.run(token_ids, cache, seq_id, pos0)
+        if h is not None:
+            cache.commit(seq_id, t)
+            GemmStatus.check(m.device)
+            return self.layers.logits(h if all_logits else h[t - 1:t])
         row = cache.block_table[cache.slot_of[seq_id]]
         pos = torch.arange(pos0, pos0 + t, dtype=torch.int32, device=m.device)
         seq = torch.zeros(t, dtype=torch.int32, device=m.device)
@@ -193,10 +349,14 @@ class NativePrefill:
 
         npages = (pos0 + t + cache.block_size - 1) // cache.block_size
         ident = torch.arange(npages, dtype=torch.int32, device=m.device) if cache.quantized else None
+        few = few_rows_plan(t, hq, hkv, hd, pos0 + t, cache.quantized)
+        lens = pos + 1 if few else None
 
         def attend(li, qkv):
             D.rope_kv_write(qkv, q, cache.k[li], cache.v[li], row.view(1, -1), pos, m.cos, m.sin,
                             hq, hkv, token_seq=seq, traditional=cfg.rope_traditional, **cache.sb(li))
+            if few:
+                return few_rows_attention(q, cache.k[li], cache.v[li], row, lens, few, m.scale, cfg.sliding_window or 0, **cache.sb(li))
             if cache.quantized:
                 # prompt attention over an 8-bit cache: the sequence's pages are expanded once per
                 # layer into contiguous bf16 pages (amortised over the chunk's tokens)
@@ -206,7 +366,7 @@ class NativePrefill:
             return flash_prefill_paged(q, cache.k[li], cache.v[li], row, pos0, m.scale,
                                        cfg.sliding_window or 0)
 
-        h = self.layers.run(D.embedding(m.w.embed, token_ids.to(torch.int32)), attend)
+        h = self.layers.run(D.embedding(m.w.embed, token_ids), attend)
         cache.commit(seq_id, t)
         GemmStatus.check(m.device)
         return self.layers.logits(h if all_logits else h[t - 1:t])

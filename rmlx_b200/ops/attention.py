@@ -30,6 +30,31 @@ def prefill_kernel_choice(head_dim: int, window: int) -> str:
     return "mma"
 
 
+#: query rows up to which a prompt portion attends on the decode kernel, each row a sequence of its own length over the same pages: five rows
+#: over 1000 keys of 16/4 heads 8 us, 22 on the prompt kernel, whose blocks walk all keys one after another; and an 8-bit cache is read as it is
+FEW_ROWS = 8
+
+
+def few_rows_plan(t: int, hq: int, hkv: int, head_dim: int, tokens: int, q8: bool) -> int:
+    """The cluster plan for ``t`` last rows of a sequence of ``tokens``; 0: the prompt kernels."""
+    if t > FEW_ROWS or head_dim not in (64, 128):
+        return 0
+    lib = _lib.cuda()
+    return int(lib.rmlx_flash_decode_cluster_plan(t, t * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv), tokens, head_dim, int(q8)))
+
+
+def few_rows_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_row: torch.Tensor, lens: torch.Tensor, plan: int,
+                       scale: float, window: int = 0, k_sb: Optional[torch.Tensor] = None, v_sb: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """q [T, Hq, D]: row i attends to the first ``lens[i]`` keys of the one sequence whose pages ``block_row`` lists."""
+    t, hq, d = q.shape
+    out = torch.empty_like(q)
+    rc = _lib.cuda().rmlx_flash_decode_cluster(
+        q.data_ptr(), k_cache.data_ptr(), _lib.ptr(k_sb), v_cache.data_ptr(), _lib.ptr(v_sb), block_row.data_ptr(), lens.data_ptr(),
+        out.data_ptr(), t, hq, k_cache.shape[1], d, block_row.numel(), 0, plan, window, scale, 0, 0, _lib.stream_ptr())
+    _lib.check(rc, "flash_decode_cluster")
+    return out
+
+
 def flash_prefill_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                         block_row: torch.Tensor, pos0: int, scale: Optional[float] = None,
                         window: int = 0, out: Optional[torch.Tensor] = None,

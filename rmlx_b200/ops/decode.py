@@ -401,7 +401,7 @@ def moe_down(act: torch.Tensor, w: LinearWeight, idx: torch.Tensor, wts: torch.T
 
 _lib.register_cuda_sigs({
     "rmlx_flash_decode_cluster_plan": ("iiiii", "i"),
-    "rmlx_flash_decode_cluster": ("ppppppppiiiiiiifiip", "i"),
+    "rmlx_flash_decode_cluster": ("ppppppppiiiiiiiifiip", "i"),
 })
 _FD_CLUSTER = os.environ.get("RMLX_FLASH_DECODE_CLUSTER", "1") != "0"
 
@@ -473,8 +473,8 @@ def flash_decode_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
     if plan and b * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv) <= scratch.tiles:
         rc = lib.rmlx_flash_decode_cluster(
             q.data_ptr(), k_cache.data_ptr(), _lib.ptr(k_sb), v_cache.data_ptr(), _lib.ptr(v_sb), block_table.data_ptr(),
-            seq_lens.data_ptr(), out.data_ptr(), b, hq, hkv, d, block_table.stride(0), plan, window, scale, int(settled), int(pdl),
-            _lib.stream_ptr())
+            seq_lens.data_ptr(), out.data_ptr(), b, hq, hkv, d, block_table.shape[1], block_table.stride(0), plan, window, scale,
+            int(settled), int(pdl), _lib.stream_ptr())
         _lib.check(rc, "flash_decode_cluster")
         return out
     if k_sb is not None:

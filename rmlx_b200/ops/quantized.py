@@ -47,12 +47,12 @@ def xgemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = N
     # the epilogue reads the residual with the result's row stride
     assert residual is None or (residual.dim() == 2 and residual.shape[0] >= m and residual.shape[1] >= n and
                                 residual.stride(1) == 1 and (m == 1 or residual.stride(0) == out.stride(0)))
-    if bn == 0 and w.kind == W_Q4 and row_pays(m, n, k, e) and row_supported(x, w, out, residual, swiglu) and \
+    route = tiles_route(w, m, e, swiglu) if bn == 0 else "tiles"
+    if route == "row" and row_supported(x, w, out, residual, swiglu) and \
             (residual is None or (e == 0 and not swiglu and residual.stride(0) == out.stride(0))):
         return row_gemm(x, w, residual, out, offsets, swiglu, gate_limit, pdl)
-    if bn == 0 and m > 128 and pair_pays(w.kind, m, n, k, e) and (not swiglu or (n % 256 == 0 and residual is None)) and \
-            (residual is None or e == 0) and (w.kind != W_Q4 or not w.scales_f16) and (w.kind != W_Q4 or k % 512 == 0) and \
-            k % 8 == 0 and _pair_ready(x, out, residual) and out.dtype == torch.bfloat16:
+    if bn == 0 and (route == "pair" or tiles_route(w, m, e, swiglu, row=False) == "pair") and (residual is None or (e == 0 and not swiglu)) and \
+            _pair_ready(x, out, residual) and out.dtype == torch.bfloat16:
         return pair_gemm(x, w, residual, out, offsets, swiglu, gate_limit, pdl)
     rc = _lib.cuda().rmlx_xgemm(w.kind, x.data_ptr(), w.w.data_ptr(), _lib.ptr(w.scales),
                                 _lib.ptr(w.biases), out.data_ptr(), _lib.ptr(residual),
@@ -61,6 +61,24 @@ def xgemm(x: torch.Tensor, w: LinearWeight, residual: Optional[torch.Tensor] = N
                                 GemmStatus.get(x.device).data_ptr(), int(pdl), _lib.stream_ptr())
     _lib.check(rc, "xgemm")
     return out
+
+
+def tiles_route(w: LinearWeight, m: int, experts: int = 0, swiglu: bool = False, row: bool = True) -> str:
+    """The kernel that ``xgemm`` prefers for m rows whose operands and results lie on 16-byte rows: "row", "pair" or "tiles"."""
+    n, k = w.n, w.k
+    q4 = w.kind == W_Q4
+    if row and q4 and not w.scales_f16 and row_pays(m, n, k, experts) and n % 128 == 0 and k % 512 == 0:
+        return "row"
+    if m > 128 and pair_pays(w.kind, m, n, k, experts) and (not swiglu or n % 256 == 0) and k % 8 == 0 and \
+            (not q4 or (not w.scales_f16 and k % 512 == 0)):
+        return "pair"
+    return "tiles"
+
+
+def row_tables_ready(w: LinearWeight) -> bool:
+    """Whether the copies of ``rmlx_row_gemm`` can read a 4-bit weight's tables."""
+    return ((w.w.data_ptr() | w.scales.data_ptr() | w.biases.data_ptr()) % 16 == 0 and
+            w.w.is_contiguous() and w.scales.is_contiguous() and w.biases.is_contiguous())
 
 
 def row_pays(m: int, n: int, k: int, experts: int = 0) -> bool:
@@ -80,8 +98,7 @@ def row_supported(x: torch.Tensor, w: LinearWeight, out: torch.Tensor, residual:
     """What ``rmlx_row_gemm`` asks of its operands: bf16 scales, 16-byte rows of x, results on 4 bytes."""
     return (not w.scales_f16 and x.data_ptr() % 16 == 0 and out.data_ptr() % 4 == 0 and out.stride(1) == 1 and
             (residual is None or (residual.data_ptr() % 4 == 0 and out.dtype == torch.bfloat16)) and
-            (w.w.data_ptr() | w.scales.data_ptr() | w.biases.data_ptr()) % 16 == 0 and
-            w.w.is_contiguous() and w.scales.is_contiguous() and w.biases.is_contiguous() and
+            row_tables_ready(w) and
             bool(_lib.cuda().rmlx_row_gemm_supported(w.n, w.k, x.stride(0), out.stride(0), int(swiglu))))
 
 

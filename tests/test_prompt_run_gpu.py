@@ -1,0 +1,93 @@
+"""A prompt portion from one native call (csrc/runtime/prompt_run.cu) against the same launches made one by one: the same kernels on the
+same values, so logits and cache are the same to the bit."""
+import pytest
+import torch
+
+from rmlx_b200.config import FeedForwardType, MoeConfig, TransformerConfig
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    return torch.device("cuda")
+
+
+def _model(dev, experts, quant, window=0, hd=128, bias=False):
+    from rmlx_b200.models.transformer import TransformerModel
+    from rmlx_b200.models.weights import LayerWeights, ModelWeights, ParallelLayout
+    from rmlx_b200.ops.weights import LinearWeight
+    g = torch.Generator(device=dev).manual_seed(1)
+    d, inner, vocab = (1024, 512, 2048) if experts else (2048, 4096, 2048)
+    hq, hkv = d // hd, d // hd // 4
+    ff = FeedForwardType.moe_(MoeConfig(experts, 2, d, inner)) if experts else FeedForwardType.gated(inner)
+    cfg = TransformerConfig(hidden_size=d, num_heads=hq, num_kv_heads=hkv, head_dim=hd, num_layers=2, vocab_size=vocab, max_seq_len=2048,
+                            rope_theta=1e4, ff_type=ff, sliding_window=window, name="prompt-run").validate()
+
+    def lin(n, k, e=0):
+        return LinearWeight.random(n, k, quant, dev, experts=e, generator=g)
+
+    def norm():
+        return (1 + 0.1 * torch.randn(d, device=dev, generator=g)).to(torch.bfloat16)
+
+    layers = []
+    for _ in range(2):
+        ff_w = {"w_gate_up": lin(2 * inner, d), "w_down": lin(d, inner)} if not experts else {
+            "router": torch.randn(experts, d, device=dev, generator=g).mul_(0.1).to(torch.bfloat16),
+            "experts_gate_up": lin(2 * inner, d, experts), "experts_down": lin(d, inner, experts),
+            "expert_bias": torch.randn(experts, device=dev, generator=g) * 0.1 if bias else None}
+        layers.append(LayerWeights(norm1=norm(), wqkv=lin((hq + 2 * hkv) * hd, d), wo=lin(d, hq * hd), norm2=norm(), **ff_w))
+    embed = torch.randn(vocab, d, device=dev, generator=g).to(torch.bfloat16)
+    return TransformerModel(ModelWeights(cfg=cfg, layout=ParallelLayout(), embed=embed, layers=layers, final_norm=norm(), lm_head=lin(vocab, d)))
+
+
+def _prompts(model, lens, kv, at_once):
+    """Portions of one sequence after one another: logits of each, and the cache."""
+    from rmlx_b200.models.prefill import enable_native_prefill
+    assert enable_native_prefill(model)
+    run = model._native_prefill.at_once.run
+    calls = []
+
+    def traced(*args):
+        h = run(*args) if at_once else None
+        calls.append(h is not None)
+        return h
+
+    model._native_prefill.at_once.run = traced
+    cache = model.new_cache(sum(lens) // 16 + 3, max_seqs=1, kv_quant=kv)
+    cache.add_sequence(0)
+    g = torch.Generator().manual_seed(2)
+    out = []
+    for n in lens:
+        ids = torch.randint(0, model.cfg.vocab_size, (n,), generator=g).to(model.device)
+        out.append(model.prefill(ids, cache, 0, all_logits=n <= 40))
+    assert all(c == at_once for c in calls) and cache.seq_len(0) == sum(lens)
+    pools = [*cache.k, *cache.v] + ([*cache.k_sb, *cache.v_sb] if kv else [])
+    return out, [p.clone() for p in pools]
+
+
+@pytest.mark.parametrize("experts", [0, 16])
+@pytest.mark.parametrize("quant", ["q4", "q8", None])
+@pytest.mark.parametrize("kv,window,hd", [(None, 0, 128), ("q8", 300, 128), (None, 0, 64)])
+def test_same_as_launch_by_launch(dev, experts, quant, kv, window, hd):
+    # portions on each side of the lines between the projections' kernels
+    lens = [1, 5, 8, 9, 17, 33, 40, 90, 100, 300, 700, 6]
+    res = [_prompts(_model(dev, experts, quant, window, hd, bias=hd == 64), lens, kv, at_once) for at_once in (False, True)]
+    for a, b in zip(res[0][0] + res[0][1], res[1][0] + res[1][1]):
+        assert torch.equal(a, b)
+
+
+def test_not_covered(dev):
+    """Weights that change between two portions are taken as they are; rows of W apart go launch by launch."""
+    from rmlx_b200.ops.weights import LinearWeight, W_BF16
+    model = _model(dev, 0, None)
+    first = _prompts(model, [40], None, True)[0][0]
+    wide = torch.zeros(model.w.layers[0].wqkv.n, model.cfg.hidden_size + 64, dtype=torch.bfloat16, device=dev)
+    wide[:, :model.cfg.hidden_size] = model.w.layers[0].wqkv.w
+    model.w.layers[0].wqkv = LinearWeight(W_BF16, wide[:, :model.cfg.hidden_size])
+    assert model._native_prefill.at_once._plain(model.w.layers[0].wqkv, 40) == 0
+    assert float((_prompts(model, [40], None, False)[0][0] - first).norm() / first.norm()) < 1e-2
+    model.w.layers[0].wqkv = LinearWeight(W_BF16, wide[:, :model.cfg.hidden_size].contiguous() * 2)
+    assert not torch.equal(_prompts(model, [40], None, True)[0][0], first)
