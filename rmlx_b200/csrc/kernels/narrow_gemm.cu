@@ -1005,37 +1005,91 @@ __global__ void __launch_bounds__(NeShape<KIND, T>::THREADS, 1) narrow_even_kern
 }
 
 
-// Position list of the grouped form: order[offsets[e] ..] are the (row, slot) pairs that chose expert e. One block; pairs
-// of an expert in no particular order (every row of x is a column of its own, so results don't depend on it). A choice outside
-// [0, E) (a row of NaN logits has no largest one: decode_moe.cu) is in no expert's list, and the combination skips it.
+// Pairs by expert in one block: counts, offsets [E + 1] (offsets[E]: all that chose an expert), and the pairs of an expert in their own
+// order: a pair's place decides which pass takes it, and passes add up K in different shares, so that any other order would make
+// results differ in their last bits from run to run. A warp counts a run of the pairs, 32 at a time. A choice outside [0, E) (a row of
+// NaN logits has no largest one: decode_moe.cu) is in no expert's list, and the combination skips it.
 __global__ void __launch_bounds__(1024) narrow_group_kernel(const int* __restrict__ idx, int pairs, int E,
                                                             int* __restrict__ offsets, int* __restrict__ order) {
-  __shared__ int count[kNwMaxExperts], start[kNwMaxExperts + 1];
+  __shared__ int count[32][kNwMaxExperts], start[kNwMaxExperts + 1];   // [warp][expert]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int run = (pairs + 32 * warps - 1) / (32 * warps) * 32, i0 = warp * run, i1 = min(i0 + run, pairs);
   pdl_launch_dependents();
-  for (int i = threadIdx.x; i < E; i += blockDim.x) count[i] = 0;
-  __syncthreads();
+  for (int e = lane; e < E; e += 32) count[warp][e] = 0;
+  __syncwarp();
   pdl_wait();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x)
-    if (const int e = idx[i]; unsigned(e) < unsigned(E)) atomicAdd(count + e, 1);
+  // the lanes of a warp that chose the same expert: from a vote on each bit of its number, a third of __match_any_sync's time
+  auto alike = [&](int e) {
+    unsigned same = __ballot_sync(0xffffffffu, unsigned(e) < unsigned(E));
+#pragma unroll
+    for (int bit = 0; bit < 8; ++bit) {
+      const unsigned set = __ballot_sync(0xffffffffu, e >> bit & 1);
+      same &= e >> bit & 1 ? set : ~set;
+    }
+    return unsigned(e) < unsigned(E) ? same : 0u;
+  };
+  constexpr int kKept = 2;                               // of the first steps is kept what the second pass needs
+  int e_of[kKept];
+  unsigned same_of[kKept];
+#pragma unroll
+  for (int c = 0; c < kKept; ++c) {
+    const int i = i0 + c * 32 + lane;
+    e_of[c] = i < i1 ? idx[i] : -1;
+  }
+#pragma unroll
+  for (int c = 0; c < kKept; ++c) {
+    if (i0 + c * 32 >= i1) break;
+    same_of[c] = alike(e_of[c]);
+    if (same_of[c] && lane == __ffs(same_of[c]) - 1) count[warp][e_of[c]] += __popc(same_of[c]);
+    __syncwarp();
+  }
+  for (int i = i0 + kKept * 32 + lane; i - lane < i1; i += 32) {
+    const int e = i < i1 ? idx[i] : -1;
+    const unsigned same = alike(e);
+    if (same && lane == __ffs(same) - 1) count[warp][e] += __popc(same);
+    __syncwarp();
+  }
   __syncthreads();
-  if (threadIdx.x < 32) {
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {     // the warps' places within an expert
+    int sum = 0;
+#pragma unroll 8
+    for (int w = 0; w < warps; ++w) { const int n = count[w][e]; count[w][e] = sum; sum += n; }
+    start[e] = sum;
+  }
+  __syncthreads();
+  if (warp == 0) {
     int base = 0;
     for (int e0 = 0; e0 < E; e0 += 32) {
-      const int e = e0 + threadIdx.x;
-      const int mine = e < E ? count[e] : 0;
+      const int e = e0 + lane;
+      const int mine = e < E ? start[e] : 0;
       int sum = mine;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (int(threadIdx.x) >= o) sum += v; }
+      for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
       if (e < E) start[e] = base + sum - mine;
       base += __shfl_sync(0xffffffffu, sum, 31);
     }
-    if (threadIdx.x == 0) start[E] = base;
+    if (lane == 0) start[E] = base;
   }
   __syncthreads();
   for (int i = threadIdx.x; i <= E; i += blockDim.x) offsets[i] = start[i];
-  __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x)
-    if (const int e = idx[i]; unsigned(e) < unsigned(E)) order[atomicAdd(start + e, 1)] = i;
+  auto place = [&](int i, int e, unsigned same) {
+    const int at = same ? count[warp][e] : 0;
+    __syncwarp();
+    if (same) {
+      order[start[e] + at + __popc(same & ((1u << lane) - 1u))] = i;
+      if (lane == __ffs(same) - 1) count[warp][e] = at + __popc(same);
+    }
+    __syncwarp();
+  };
+#pragma unroll
+  for (int c = 0; c < kKept; ++c) {
+    if (i0 + c * 32 >= i1) break;
+    place(i0 + c * 32 + lane, e_of[c], same_of[c]);
+  }
+  for (int i = i0 + kKept * 32 + lane; i - lane < i1; i += 32) {
+    const int e = i < i1 ? idx[i] : -1;
+    place(i, e, alike(e));
+  }
 }
 
 // out[t] = residual[t] + sum_s w[t, s] y[t k + s], slots in order, y in fp32; slots whose choice idx[t, s] is no expert are

@@ -287,3 +287,17 @@ def test_experts_on_clusters(dev, kind, k, tiles, shares):
         at += c
         if c:
             assert _rel(got[r], x[r].double() @ wd[e].t()) < 2e-5
+
+
+@pytest.mark.parametrize("rows,top,experts", [(1, 8, 128), (5, 3, 7), (64, 8, 128), (129, 8, 256), (192, 8, 32), (700, 2, 16)])
+def test_pairs_in_order(dev, rows, top, experts):
+    """The pairs of an expert in ascending order, each once, without those that chose none: a pair's place decides how its sums are
+    split, so results would otherwise differ from run to run."""
+    from rmlx_b200.ops import narrow
+    g = torch.Generator(device=dev).manual_seed(rows)
+    idx = torch.randint(-1, experts + 1, (rows, top), device=dev, generator=g, dtype=torch.int32)
+    offsets, order = narrow.group_pairs(idx, experts)
+    flat = idx.flatten().tolist()
+    lists = [[i for i, e in enumerate(flat) if e == x] for x in range(experts)]
+    assert offsets.tolist() == [sum(len(p) for p in lists[:x]) for x in range(experts + 1)]
+    assert order[:sum(map(len, lists))].tolist() == [i for p in lists for i in p]
