@@ -2,8 +2,8 @@
 // device (the reference reads the routing result back to the host on every forward,
 // crates/rmlx-nn/src/moe.rs:600-601).
 //
-//   moe_router        RMSNorm + gate projection + softmax + top-k + renormalise, one launch; the
-//                     last block to finish its logits does the selection
+//   moe_router        RMSNorm + gate projection + softmax + top-k + renormalise, one launch; a
+//                     cluster of blocks takes eight rows and selects their experts
 //                     (reference: moe_topk_route_f32, crates/rmlx-core/src/ops/topk_route.rs:212)
 //   topk_route        the same selection over precomputed logits for many tokens, with the
 //                     per-expert histogram; prefix offsets by moe_prefix_offsets
@@ -21,26 +21,30 @@ namespace rb {
 constexpr int kMaxExperts = 256;
 constexpr int kMaxTopK = 8;
 
-// Softmax over E logits held 8-per-lane, then k rounds of warp arg-max (ties: lowest index wins),
-// weights renormalised to sum 1. Executed by one full warp for one token. NaN logits have no largest one: such a row's choices
-// are numbers outside [0, E), which are not counted and which every user of the choices skips.
-__device__ __forceinline__ void warp_topk(const float* logits, const float* bias, int E, int k,
-                                          int* out_idx, float* out_w, int* counts) {
+// Softmax over E logits held up to 8-per-lane, then k rounds of warp arg-max (ties: lowest index wins), weights renormalised to
+// sum 1. Executed by one full warp for one token. The rounds are a chain: each is two warp reductions of integers (a probability's
+// bits order as it does; 1 is added so that 0 is below all of them) instead of ten shuffles and their comparisons.
+// NaN logits have no largest one: such a row's choices are numbers outside [0, E), which are not counted and which every user of
+// the choices skips.
+template <int V>
+__device__ __forceinline__ void warp_topk_v(const float* logits, const float* bias, int E, int k, int* out_idx, float* out_w, int* counts) {
   const int lane = threadIdx.x & 31;
-  float v[kMaxExperts / 32];
+  float v[V];
   float m = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < kMaxExperts / 32; ++i) {
+  for (int i = 0; i < V; ++i) {
     const int e = i * 32 + lane;
     v[i] = (e < E) ? logits[e] + (bias ? bias[e] : 0.f) : -INFINITY;
     m = fmaxf(m, v[i]);
   }
   m = warp_max(m);
   float s = 0.f;
+  uint32_t key[V];
 #pragma unroll
-  for (int i = 0; i < kMaxExperts / 32; ++i) {
-    v[i] = (i * 32 + lane < E) ? __expf(v[i] - m) : -1.f;  // probabilities are >= 0; -1 = absent
-    s += fmaxf(v[i], 0.f);
+  for (int i = 0; i < V; ++i) {
+    const float p = (i * 32 + lane < E) ? __expf(v[i] - m) : 0.f;
+    s += fmaxf(p, 0.f);
+    key[i] = (i * 32 + lane < E && p >= 0.f) ? __float_as_uint(p) + 1u : 0u;   // neither absent nor NaN
   }
   s = warp_sum(s);
   const float inv = 1.f / s;
@@ -48,24 +52,19 @@ __device__ __forceinline__ void warp_topk(const float* logits, const float* bias
   int sel_e = 0;
   float wsum = 0.f;
   for (int r = 0; r < k; ++r) {
-    float best = -2.f;
-    int best_e = 0x7fffffff;
+    uint32_t best = key[0];
+    int at = 0;
 #pragma unroll
-    for (int i = 0; i < kMaxExperts / 32; ++i) {
-      if (v[i] > best) { best = v[i]; best_e = i * 32 + lane; }
-    }
+    for (int i = 1; i < V; ++i)
+      if (key[i] > best) { best = key[i]; at = i; }
+    const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+    const uint32_t e = __reduce_min_sync(0xffffffffu, best == top && top ? uint32_t(at * 32 + lane) : 0x7fffffffu);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
-#pragma unroll
-    for (int i = 0; i < kMaxExperts / 32; ++i)
-      if (i * 32 + lane == best_e) v[i] = -1.f;
-    const float p = best * inv;
+    for (int i = 0; i < V; ++i)
+      if (uint32_t(i * 32 + lane) == e) key[i] = 0u;
+    const float p = (top ? __uint_as_float(top - 1u) : -2.f) * inv;
     wsum += p;
-    if (lane == r) { sel_w = p; sel_e = best_e; }
+    if (lane == r) { sel_w = p; sel_e = int(e); }
   }
   if (lane < k) {
     out_idx[lane] = sel_e;
@@ -74,9 +73,16 @@ __device__ __forceinline__ void warp_topk(const float* logits, const float* bias
   }
 }
 
+__device__ __forceinline__ void warp_topk(const float* logits, const float* bias, int E, int k, int* out_idx, float* out_w, int* counts) {
+  if (E <= 32) warp_topk_v<1>(logits, bias, E, k, out_idx, out_w, counts);
+  else if (E <= 128) warp_topk_v<4>(logits, bias, E, k, out_idx, out_w, counts);
+  else warp_topk_v<kMaxExperts / 32>(logits, bias, E, k, out_idx, out_w, counts);
+}
+
+// One to four rows, where many blocks read the weights faster than one cluster (rule at the launch).
 template <int B>
 __global__ void __launch_bounds__(kGemvThreads)
-moe_router_kernel(const __nv_bfloat16* __restrict__ gate_w, const __nv_bfloat16* __restrict__ x,
+moe_router_few_kernel(const __nv_bfloat16* __restrict__ gate_w, const __nv_bfloat16* __restrict__ x,
                   int x_stride, const __nv_bfloat16* __restrict__ norm_w, float eps,
                   const float* __restrict__ expert_bias, float* __restrict__ logits,
                   int* __restrict__ topk_idx, float* __restrict__ topk_w, int* __restrict__ counts,
@@ -169,6 +175,167 @@ moe_router_kernel(const __nv_bfloat16* __restrict__ gate_w, const __nv_bfloat16*
     if (threadIdx.x == 0) *ticket = 0u;  // ready for the next launch (graph replay included)
   }
   pdl_launch_dependents();
+}
+
+// The router of any number of rows: a cluster of 8 or 16 blocks per eight rows takes K apart, every warp 32 values at a time for all
+// experts, 16 of them and eight rows to an instruction (mma m16n8k16; both operands come straight from global memory: a lane's 16
+// bytes of a row of W, and the same values of x, are its operands of two instructions, the order of K being free). The sums of the
+// warps, then of the blocks, meet in shared memory, and block r selects the experts of row r.
+//
+// Nothing is rounded on the way to the fp32 sums: x * g is a product of two bf16 numbers and has 16 bits, so a bf16 number and
+// another bf16 remainder hold all of it; each instruction adds 16 products to zero and the sums between instructions are fp32
+// additions. (Root mean square error of the logits of 128 experts of 4096, 64 rows, against 64 bits: 2.6e-8 of the largest; one fused
+// multiply-add per product, as in the kernel above, 3.2e-8.)
+//
+// Bound by latency: 1 MB of weights (128 x 4096), of which a warp requests its first 32 columns before it waits for the rows, then two
+// meetings of the warps and the selection. 128 x 4096, us: 5.7 for 8 rows (19 in two passes of the kernel above, whose every block
+// stages all rows in fp32), 7.4 for 64 (26 as norm, GEMM and selection); 32 x 2048: 4.7 and 5.2 (14 and 19).
+constexpr int kRtWarps = 8, kRtThreads = 32 * kRtWarps, kRtRows = 8, kRtTiles = 8, kRtGroup = 16 * kRtTiles, kRtPad = kRtGroup + 4;
+constexpr int kRtMaxCluster = 16;
+
+__device__ __forceinline__ void rt_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ float rt_remote(uint32_t addr, int rank) {
+  float v;
+  asm volatile("{.reg .u32 a; mapa.shared::cluster.u32 a, %1, %2; ld.shared::cluster.f32 %0, [a];}" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+
+template <int CS>
+__global__ void __launch_bounds__(kRtThreads, 2)
+moe_router_kernel(const __nv_bfloat16* __restrict__ gate_w, const __nv_bfloat16* __restrict__ x, int x_stride,
+                  const __nv_bfloat16* __restrict__ norm_w, float eps, const float* __restrict__ expert_bias,
+                  float* __restrict__ logits, int* __restrict__ topk_idx, float* __restrict__ topk_w, int* __restrict__ counts, int B,
+                  int E, int K, int k) {
+  __shared__ float red[kRtWarps][kRtRows][kRtPad];
+  __shared__ float part[kRtRows][kMaxExperts];           // the block's sums, read by the cluster
+  __shared__ float squares[kRtWarps][kRtRows], square[kRtRows];
+  __shared__ float row_logits[kMaxExperts];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  int rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int row0 = blockIdx.x / CS * kRtRows, chunks = (K + 31) >> 5, chunk0 = rank * kRtWarps + warp;
+  const __nv_bfloat16* const xr = x + size_t(min(row0 + g, B - 1)) * x_stride;
+  const bool have = row0 + g < B;
+
+  uint4 w[2 * kRtTiles];
+  auto load_w = [&](int e0, int chunk) {
+    const int c = chunk * 32 + t * 8;
+#pragma unroll
+    for (int j = 0; j < 2 * kRtTiles; ++j) {
+      const int e = e0 + (j >> 1) * 16 + (j & 1) * 8 + g;
+      w[j] = e < E && c < K ? ldg_stream(gate_w + size_t(e) * K + c) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  load_w(0, chunk0);
+  pdl_launch_dependents();   // let the next kernel start its weight prefetch now; its own wait covers our completion
+  pdl_wait();
+
+  float ssq = 0.f;
+  for (int e0 = 0; e0 < E; e0 += kRtGroup) {
+    float acc[kRtTiles][4];
+#pragma unroll
+    for (int j = 0; j < kRtTiles; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    for (int chunk = chunk0; chunk < chunks; chunk += CS * kRtWarps) {
+      const int c = chunk * 32 + t * 8;
+      const uint4 none = make_uint4(0, 0, 0, 0);
+      const uint4 xv = have && c < K ? __ldcg(reinterpret_cast<const uint4*>(xr + c)) : none;
+      const uint4 gv = norm_w && c < K ? *reinterpret_cast<const uint4*>(norm_w + c) : none;
+      if (e0 != 0 || chunk != chunk0) load_w(e0, chunk);
+      const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, gs[4] = {gv.x, gv.y, gv.z, gv.w};
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float a = bf16lo(xs[i]), b = bf16hi(xs[i]);
+        if (e0 == 0) ssq += a * a + b * b;
+        hi[i] = xs[i]; lo[i] = 0;
+        if (norm_w) {
+          a *= bf16lo(gs[i]); b *= bf16hi(gs[i]);
+          hi[i] = pack_bf16(a, b);
+          // an infinite product has no remainder
+          const float ra = a - bf16lo(hi[i]), rb = b - bf16hi(hi[i]);
+          lo[i] = pack_bf16(isfinite(ra) ? ra : 0.f, isfinite(rb) ? rb : 0.f);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kRtTiles; ++j) {
+        if (e0 + j * 16 >= E) break;
+        const uint4 p = w[2 * j], q = w[2 * j + 1];
+        float d[4], f[4];
+        rt_mma(d, p.x, q.x, p.y, q.y, hi[0], hi[1]);
+        rt_mma(f, p.z, q.z, p.w, q.w, hi[2], hi[3]);
+        if (norm_w) {
+          float u[4], v[4];
+          rt_mma(u, p.x, q.x, p.y, q.y, lo[0], lo[1]);
+          rt_mma(v, p.z, q.z, p.w, q.w, lo[2], lo[3]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { d[i] += u[i]; f[i] += v[i]; }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] += d[i] + f[i];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kRtTiles; ++j) {
+      red[warp][2 * t][j * 16 + g] = acc[j][0]; red[warp][2 * t + 1][j * 16 + g] = acc[j][1];
+      red[warp][2 * t][j * 16 + 8 + g] = acc[j][2]; red[warp][2 * t + 1][j * 16 + 8 + g] = acc[j][3];
+    }
+    if (e0 == 0) {
+      ssq += __shfl_xor_sync(0xffffffffu, ssq, 1);
+      ssq += __shfl_xor_sync(0xffffffffu, ssq, 2);
+      if (t == 0) squares[warp][g] = ssq;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kRtRows * kRtGroup / kRtThreads; ++i) {
+      const int at = i * kRtThreads + threadIdx.x, r = at / kRtGroup, e = at % kRtGroup;
+      float v[kRtWarps];
+#pragma unroll
+      for (int j = 0; j < kRtWarps; ++j) v[j] = red[j][r][e];
+      part[r][e0 + e] = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
+    if (e0 == 0 && threadIdx.x < kRtRows) {
+      float v = 0.f;
+#pragma unroll
+      for (int j = 0; j < kRtWarps; ++j) v += squares[j][threadIdx.x];
+      square[threadIdx.x] = v;
+    }
+    if (e0 + kRtGroup < E) __syncthreads();
+  }
+
+  // block r: row r
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int row = row0 + rank;
+  const bool mine = rank < kRtRows && row < B;
+  if (mine) {
+    const float sq = lane < CS ? rt_remote(smem_u32(&square[rank]), lane) : 0.f;
+    const int e = threadIdx.x;
+    float v[CS];
+    if (e < E) {
+#pragma unroll
+      for (int j = 0; j < CS; ++j) v[j] = rt_remote(smem_u32(&part[rank][e]), j);
+    }
+    const float inv_rms = norm_w ? rsqrtf(warp_sum(sq) / float(K) + eps) : 1.f;
+    if (e < E) {
+#pragma unroll
+      for (int o = CS / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < o; ++j) v[j] += v[j + o];
+      const float l = v[0] * inv_rms;
+      row_logits[e] = l;
+      if (logits) logits[size_t(row) * E + e] = l;
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (mine) {
+    __syncthreads();
+    if (warp == 0) warp_topk(row_logits, expert_bias, E, k, topk_idx + size_t(row) * k, topk_w + size_t(row) * k, counts);
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // nobody leaves while its sums are read
 }
 
 __global__ void __launch_bounds__(256)
@@ -511,31 +678,60 @@ static int launch_moe_down(const void* w, const void* sc, const void* bi, const 
 
 using namespace rb;
 
-// Scratch: `logits` fp32 [B, E] and `ticket` one zero-initialised uint32 (left at zero on return).
-// counts may be null; when given it must be zeroed by the caller and receives the histogram.
-extern "C" int rmlx_moe_router(const void* gate_w, const void* x, int x_stride, const void* norm_w,
-                               float eps, const float* expert_bias, float* logits, int* topk_idx,
-                               float* topk_w, int* counts, unsigned int* ticket, int B, int E, int K,
-                               int k, int pdl, cudaStream_t st) {
-  if (E > kMaxExperts || k > kMaxTopK || k > E || K % 8 || B < 1 || B > 4) return -2;
-  const size_t bstride = (XStage<WBf16>::bytes(K) + 15) & ~size_t(15);
-  int grid = E;
-#define RB_ROUTER(BB)                                                                            \
-  {                                                                                              \
-    auto kern = moe_router_kernel<BB>;                                                           \
-    RB_CHECK(set_max_smem(kern, bstride * BB));                                                  \
-    return launch(kern, dim3(grid), dim3(kGemvThreads), bstride * BB, st, pdl != 0,              \
-                  static_cast<const __nv_bfloat16*>(gate_w), static_cast<const __nv_bfloat16*>(x), \
-                  x_stride, static_cast<const __nv_bfloat16*>(norm_w), eps, expert_bias, logits, \
-                  topk_idx, topk_w, counts, ticket, E, K, k);                                    \
-  }
-  switch (B) {
-    case 1: RB_ROUTER(1)
-    case 2: RB_ROUTER(2)
-    case 3: RB_ROUTER(3)
-    default: RB_ROUTER(4)
-  }
+template <int B>
+static int launch_router_few(const void* gate_w, const void* x, int x_stride, const void* norm_w, float eps, const float* expert_bias,
+                             float* logits, int* topk_idx, float* topk_w, int* counts, unsigned int* ticket, int E, int K, int k, int pdl,
+                             cudaStream_t st) {
+  const size_t smem = ((XStage<WBf16>::bytes(K) + 15) & ~size_t(15)) * B;
+  auto kern = moe_router_few_kernel<B>;
+  RB_CHECK(set_max_smem(kern, smem));
+  return launch(kern, dim3(E), dim3(kGemvThreads), smem, st, pdl != 0, static_cast<const __nv_bfloat16*>(gate_w),
+                static_cast<const __nv_bfloat16*>(x), x_stride, static_cast<const __nv_bfloat16*>(norm_w), eps, expert_bias, logits, topk_idx,
+                topk_w, counts, ticket, E, K, k);
+}
+
+// Scratch: `logits` fp32 [B, E] and `ticket` one zero-initialised uint32 (left at zero on return); either may be null, few rows then
+// take the cluster too. counts may be null; when given it must be zeroed by the caller and receives the histogram. x's rows, norm_w and gate_w at 16-byte
+// addresses.
+extern "C" int rmlx_moe_router(const void* gate_w, const void* x, int x_stride, const void* norm_w, float eps, const float* expert_bias,
+                               float* logits, int* topk_idx, float* topk_w, int* counts, unsigned int* ticket, int B, int E, int K, int k,
+                               int pdl, cudaStream_t st) {
+  if (E > kMaxExperts || k > kMaxTopK || k > E || K % 8 || B < 1) return -2;
+  // One row, and up to four where the cluster goes over the rows twice: a block per expert (us, blocks / cluster: 128 x 4096 4.6 / 5.0
+  // for one row, 5.6 / 5.2 for two; 256 x 4096 6.5 / 9.8 for two, 8.7 / 9.7 for four; 256 x 7168 12 / 19 for four, 25 / 20 for eight,
+  // which are two passes of blocks)
+  if (logits && ticket && (B == 1 || (B <= 4 && E > kRtGroup))) {
+#define RB_ROUTER(BB) return launch_router_few<BB>(gate_w, x, x_stride, norm_w, eps, expert_bias, logits, topk_idx, topk_w, counts, ticket, E, \
+                                                   K, k, pdl, st)
+    switch (B) {
+      case 1: RB_ROUTER(1);
+      case 2: RB_ROUTER(2);
+      case 3: RB_ROUTER(3);
+      default: RB_ROUTER(4);
+    }
 #undef RB_ROUTER
+  }
+  // sixteen blocks for rows of more than 2048: one 32-value step per warp at 4096
+  const int cs = K > 2048 ? 16 : 8;
+  auto kern = cs == 16 ? moe_router_kernel<16> : moe_router_kernel<8>;
+  if (cs > 8) RB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((B + kRtRows - 1) / kRtRows * cs);
+  cfg.blockDim = dim3(kRtThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  if (pdl) prefer_max_shared(kern);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<const __nv_bfloat16*>(gate_w), static_cast<const __nv_bfloat16*>(x), x_stride,
+                                           static_cast<const __nv_bfloat16*>(norm_w), eps, expert_bias, logits, topk_idx, topk_w, counts, B, E,
+                                           K, k);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return static_cast<int>(e);
 }
 
 extern "C" int rmlx_topk_route(const float* logits, const float* expert_bias, int* topk_idx,

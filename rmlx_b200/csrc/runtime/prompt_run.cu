@@ -23,6 +23,8 @@ int rmlx_flash_decode_cluster(const void* q, const void* k_cache, const void* k_
                               float scale, int early, int pdl, cudaStream_t st);
 int rmlx_flash_prefill_tc(const void* q, const void* k_cache, const void* v_cache, const int* block_table, void* out, int T, int Hq, int Hkv,
                           int HD, int num_blocks, int pos0, int window, float scale, int lanes, int* status, int pdl, cudaStream_t st);
+int rmlx_moe_router(const void* gate_w, const void* x, int x_stride, const void* norm_w, float eps, const float* expert_bias, float* logits,
+                    int* topk_idx, float* topk_w, int* counts, unsigned int* ticket, int B, int E, int K, int k, int pdl, cudaStream_t st);
 int rmlx_topk_route(const float* logits, const float* expert_bias, int* topk_idx, float* topk_w, int* counts, int* offsets, int T, int E, int k,
                     cudaStream_t st);
 int rmlx_moe_scatter_rows(const void* x, int x_stride, const int* topk_idx, const int* offsets, int* cursors, void* xs, int* row_of_pair, int T,
@@ -128,13 +130,23 @@ struct Run {
     const int t = int(p.t), d = int(p.d), e = int(l.experts), k = int(l.top_k), pairs = t * k, inner = int(l.up.n / 2);
     int *const idx = at<int>(p.idx), *const offsets = at<int>(p.offsets), *const order = at<int>(p.order), *const row_of = at<int>(p.row_of);
     float* const wts = at<float>(p.wts);
-    if (!done(rmlx_rms_norm(h, nullptr, at(l.norm2), at(p.xn), nullptr, t, d, eps, kPdl, st), "rms_norm") ||
-        !done(rmlx_gemm_bf16_f32(at(p.xn), at(l.router), at(p.logits), t, e, d, d, d, e, at<int>(p.status), kPdl, st), "gemm_bf16_f32") ||
-        !done(rmlx_topk_route(at<float>(p.logits), at<float>(l.router_bias), idx, wts, at<int>(p.counts), offsets, t, e, k, st), "topk_route"))
+    const bool inside = l.up.route & kWithNorm;          // few rows: their norm is taken along by the router and the experts
+    const void* const xn = inside ? h : at(p.xn);
+    const void* const norm = inside ? at(l.norm2) : nullptr;
+    if (inside) {
+      if (!done(rmlx_moe_router(at(l.router), h, d, norm, eps, at<float>(l.router_bias), at<float>(p.logits), idx, wts, nullptr,
+                                nullptr, t, e, d, k, kPdl, st), "moe_router"))
+        return false;
+    } else if (!done(rmlx_rms_norm(h, nullptr, at(l.norm2), at(p.xn), nullptr, t, d, eps, kPdl, st), "rms_norm") ||
+               !done(rmlx_gemm_bf16_f32(at(p.xn), at(l.router), at(p.logits), t, e, d, d, d, e, at<int>(p.status), kPdl, st),
+                     "gemm_bf16_f32") ||
+               !done(rmlx_topk_route(at<float>(p.logits), at<float>(l.router_bias), idx, wts, at<int>(p.counts), offsets, t, e, k, st),
+                     "topk_route")) {
       return false;
+    }
     if ((l.up.route & 15) == kNarrow) {                  // every chosen expert's weights once for all rows that chose it
       return done(rmlx_narrow_group(idx, pairs, e, offsets, order, kPdl, st), "narrow_group") &&
-             done(rmlx_narrow_gemm(int(l.up.kind), at(l.up.w), at(l.up.scales), at(l.up.biases), at(p.xn), d, k, order, offsets, e, nullptr, eps,
+             done(rmlx_narrow_gemm(int(l.up.kind), at(l.up.w), at(l.up.scales), at(l.up.biases), xn, d, k, order, offsets, e, norm, eps,
                                    nullptr, 0, at(p.act), inner, 0, pairs, int(l.up.n), d, 1, 0, 0, kPdl, st), "narrow_gemm") &&
              done(rmlx_narrow_gemm(int(l.down.kind), at(l.down.w), at(l.down.scales), at(l.down.biases), at(p.act), inner, 1, order, offsets, e,
                                    nullptr, eps, nullptr, 0, at(p.y), d, 1, pairs, d, inner, 0, 0, 0, kPdl, st), "narrow_gemm") &&

@@ -90,6 +90,21 @@ def _router_logits(xn: torch.Tensor, router: torch.Tensor) -> torch.Tensor:
     return xn.float() @ router.float().t()
 
 
+# Rows up to which the decode step's router (one launch from the rows before their norm) is faster than a norm, a GEMM and the
+# selection: 128 experts of 4096, us, 7.4 / 26 at 64 rows, 14 / 26 at 128, 16 / 27 at 192, 23 / 27 at 256; 256 experts 26 / 28 at 192,
+# 38 / 28 at 256.
+ROUTER_ROWS = 192
+
+
+def _routed_few(h: torch.Tensor, lw, moe) -> bool:
+    """Whether few rows go to the experts without a normalised copy of them: the router and the weight-streaming kernel take the norm
+    along."""
+    up, r = lw.experts_gate_up, lw.router
+    return (h.shape[0] <= ROUTER_ROWS and up.experts == moe.num_experts and not lw.expert_base and grouped._NARROW_MAX_AVG_ROWS <= 0 and
+            narrow.pays_grouped(up, lw.experts_down, h.shape[0] * moe.num_experts_per_token) and r.dtype == torch.bfloat16 and
+            r.is_contiguous() and h.stride(0) % 8 == 0 and (h.data_ptr() | r.data_ptr() | lw.norm2.data_ptr()) % 16 == 0)
+
+
 def _check_model(model) -> None:
     cfg = model.cfg
     if cfg.head_dim not in (64, 128):
@@ -126,10 +141,14 @@ class _Layers:
             h = self._row_parallel(attn.view(t, hq * hd), lw.wo, h)
             if lw.router is not None:
                 moe = cfg.ff_type.moe
+                single = m.layout.world == 1 and lw.shared_gate_up is None
+                if single and _routed_few(h, lw, moe):
+                    idx, wts = D.moe_router(h, lw.router, lw.norm2, cfg.rms_norm_eps, moe.num_experts_per_token, lw.expert_bias)
+                    h = narrow.expert_ffn(h, idx, wts, lw.experts_gate_up, lw.experts_down, lw.norm2, cfg.rms_norm_eps, residual=h)
+                    continue
                 xn = D.rms_norm(h, lw.norm2, cfg.rms_norm_eps)
                 logits = _router_logits(xn, lw.router)
                 idx, wts, _, offsets = D.topk_route(logits, moe.num_experts_per_token, lw.expert_bias)
-                single = m.layout.world == 1 and lw.shared_gate_up is None
                 y = moe_prefill_ffn(xn, idx, wts, offsets, lw.experts_gate_up, lw.experts_down,
                                     residual=h if single else None, expert_base=lw.expert_base)
                 if lw.shared_gate_up is not None:
@@ -254,6 +273,8 @@ class PromptRun:
                 pairs, most = max(pairs, t * k), max(most, e)
                 if narrow.pays_grouped(up, down, t * k):
                     r_up = r_down = self.NARROW
+                    if t <= ROUTER_ROWS and r.data_ptr() % 16 == 0:
+                        r_up |= self.WITH_NORM
                     y = max(y, t * k * d * 4)
                 else:
                     up, down = grouped._expanded_if_needed(up), grouped._expanded_if_needed(down)

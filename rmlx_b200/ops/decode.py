@@ -295,20 +295,17 @@ def moe_router(x: torch.Tensor, gate_w: torch.Tensor, norm_w: Optional[torch.Ten
     _lib.require_cuda_tensor(x, gate_w)
     b, k = x.shape
     e = gate_w.shape[0]
-    scratch = scratch or RouterScratch(b, e, x.device)
     if idx is None:
         idx = torch.empty(b, top_k, dtype=torch.int32, device=x.device)
     if wts is None:
         wts = torch.empty(b, top_k, dtype=torch.float32, device=x.device)
-    lib, st = _lib.cuda(), _lib.stream_ptr()
-    for b0 in range(0, b, _MAXB):
-        bb = min(_MAXB, b - b0)
-        xs = x[b0:b0 + bb]
-        rc = lib.rmlx_moe_router(gate_w.data_ptr(), xs.data_ptr(), xs.stride(0), _lib.ptr(norm_w),
-                                 eps, _lib.ptr(expert_bias), scratch.logits[b0:].data_ptr(),
-                                 idx[b0:].data_ptr(), wts[b0:].data_ptr(), _lib.ptr(counts),
-                                 scratch.ticket.data_ptr(), bb, e, k, top_k, int(pdl), st)
-        _lib.check(rc, "moe_router")
+    if b == 0:
+        return idx, wts
+    rc = _lib.cuda().rmlx_moe_router(gate_w.data_ptr(), x.data_ptr(), x.stride(0), _lib.ptr(norm_w), eps, _lib.ptr(expert_bias),
+                                     None if scratch is None else scratch.logits.data_ptr(), idx.data_ptr(), wts.data_ptr(),
+                                     _lib.ptr(counts), None if scratch is None else scratch.ticket.data_ptr(), b, e, k, top_k, int(pdl),
+                                     _lib.stream_ptr())
+    _lib.check(rc, "moe_router")
     return idx, wts
 
 
