@@ -109,14 +109,20 @@ def set_q4_path(path: str) -> None:
 
 
 def _several(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[torch.Tensor] = None, swiglu: bool = False) -> bool:
-    """Several rows: the weight-streaming kernel of ``ops/narrow.py``, which multiplies eight rows for the price of one
+    """Several rows, and one of a wide weight: the weight-streaming kernel of ``ops/narrow.py``, which multiplies eight rows for the price of one
     (4-bit 9216 x 4096 at 8 rows: 11 us, 39 on the tensor-core mat-vec, 30 on the streaming kernel), unless the weight is so
     small that its fixed part exceeds two or three passes of the per-row kernels, or bf16 and so large that two or three rows
     stream at the copy bandwidth anyway. ``q4_path`` and the streaming switch away from their defaults keep the kernels that they
     name."""
+    if b == 1:
+        # one row of a wide 4- or 8-bit weight (us, weight-streaming / per-row, 8-bit: streaming). 4-bit: 151936 x 4096 66 / 78, 28672 x 4096
+        # 17 / 21, 32768 x 2048 11 / 15, 16384 x 2048 8.8 / 10.6, but 9 / 8 with SwiGLU; 9216 x 4096 9.0 / 9.2, 6144 x 4096 8.1 / 7.9. 8-bit:
+        # 151936 x 4096 107 / 139, 32768 x 2048 14 / 18, 16384 x 2048 9.5 / 11.5 (SwiGLU 9.5 / 11.7), 2048 x 8192 9.1 / 8.1
+        if w.kind == W_BF16 or w.n < 16384 or w.n * w.k < (1 << 26 if swiglu else 1 << 25):
+            return False
     # two rows of 4-bit weights: a 16384 x 2048 projection 9 us against 11, a 3072 x 2048 one 6 against 5
     least = 0 if b >= 4 else 1 << 24 if b == 2 and w.kind == W_Q4 else 1 << 20
-    return (b >= 2 and _STREAM and q4_path() == "auto" and w.n * w.k >= least and narrow.supported(w) and
+    return (b >= 1 and _STREAM and q4_path() == "auto" and w.n * w.k >= least and narrow.supported(w) and
             x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and (norm_w is None or norm_w.data_ptr() % 16 == 0) and
             not (b <= 3 and w.kind == W_BF16 and not swiglu and _rows_stream(b, w.n * w.k, w.k, norm_w is not None)))
 

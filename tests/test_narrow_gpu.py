@@ -301,3 +301,15 @@ def test_pairs_in_order(dev, rows, top, experts):
     lists = [[i for i, e in enumerate(flat) if e == x] for x in range(experts)]
     assert offsets.tolist() == [sum(len(p) for p in lists[:x]) for x in range(experts + 1)]
     assert order[:sum(map(len, lists))].tolist() == [i for p in lists for i in p]
+
+
+@pytest.mark.parametrize("kind,n,k,wide", [("q4", 16384, 2048, True), ("q8", 16400, 2048, True), ("q4", 16384, 1536, False), ("q8", 8192, 4096, False),
+                                           (None, 16384, 2048, False)])
+def test_one_row_of_a_wide_weight(dev, kind, n, k, wide):
+    from rmlx_b200.ops import decode as D
+    w, wd, x, g = _case(dev, kind, n, k, 1, seed=17)
+    res = torch.randn(1, n, device=dev, generator=g).to(torch.bfloat16)
+    assert D._several(1, w, x) == wide and D._several(1, w, x, swiglu=True) is False
+    # the weight-streaming kernel's sums are fp32; the per-row kernels multiply 4- and 8-bit weights in fp16
+    bound = 1e-5 if wide or kind is None else 2e-3
+    assert _rel(D.rms_gemv(x, w, residual=res, out_dtype=torch.float32), x.double() @ wd.t() + res.double()) < bound
