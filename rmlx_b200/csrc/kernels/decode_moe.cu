@@ -44,7 +44,8 @@ __device__ __forceinline__ void warp_topk_v(const float* logits, const float* bi
   for (int i = 0; i < V; ++i) {
     const float p = (i * 32 + lane < E) ? __expf(v[i] - m) : 0.f;
     s += fmaxf(p, 0.f);
-    key[i] = (i * 32 + lane < E && p >= 0.f) ? __float_as_uint(p) + 1u : 0u;   // neither absent nor NaN
+    const uint32_t bits = __float_as_uint(p);
+    key[i] = (i * 32 + lane < E && bits <= 0x7f800000u) ? bits + 1u : 0u;   // neither absent nor NaN
   }
   s = warp_sum(s);
   const float inv = 1.f / s;

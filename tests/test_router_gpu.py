@@ -61,6 +61,8 @@ def test_ties_nan_and_infinities(dev):
 def test_selection_matches_every_count(dev):
     """The selection over given logits for each number of registers that it is built for, with equal probabilities and zeros."""
     for e in (8, 32, 33, 128, 129, 256):
+        empty = D.topk_route(torch.full((3, e), float("nan"), device=dev), 4)
+        assert all(not 0 <= c < e for r in empty[0].tolist() for c in r) and not empty[2].any()
         logits = torch.randint(0, 4, (50, e), device=dev).float() * 30
         idx, wts, counts, offsets = D.topk_route(logits, 8)
         order = torch.sort(torch.softmax(logits, -1), dim=-1, descending=True, stable=True)
