@@ -15,7 +15,8 @@ int rmlx_rope_kv_write(const void* qkv, int qkv_f32, void* q_out, void* k_cache,
 int rmlx_rope_kv_write_q8(const void* qkv, void* q_out, void* k_q, void* k_sb, void* v_q, void* v_sb, const int* block_table,
                           const int* positions, const int* token_seq, const float* cos_t, const float* sin_t, int T, int Hq, int Hkv, int HD,
                           int max_blocks, int page, int traditional, int pdl, cudaStream_t st);
-int rmlx_kv_dequant_pages(const void* q, const void* sb, const int* table, void* out, int n_pages, int Hkv, int page, int HD, cudaStream_t st);
+int rmlx_kv_dequant_pages(const void* q, const void* sb, const int* table, void* out, int n_pages, int Hkv, int page, int HD, int pdl,
+                          cudaStream_t st);
 int rmlx_flash_prefill_paged(const void* q, const void* k_cache, const void* v_cache, const int* block_table, void* out, int T, int Hq, int Hkv,
                              int HD, int pos0, int window, float scale, int pdl, cudaStream_t st);
 int rmlx_flash_decode_cluster(const void* q, const void* k_cache, const void* k_sb, const void* v_cache, const void* v_sb, const int* block_table,
@@ -174,8 +175,8 @@ struct Run {
                                             int(p.row_blocks), 0, int(p.few), int(p.window), scale, 0, kPdl, st), "flash_decode_cluster");
     if (l.k_sb) {
       // the 8-bit cache's pages are expanded once per layer into contiguous bf16 pages
-      if (!done(rmlx_kv_dequant_pages(at(l.k), at(l.k_sb), row, at(p.kk), int(p.pages), hkv, page, hd, st), "kv_dequant_pages") ||
-          !done(rmlx_kv_dequant_pages(at(l.v), at(l.v_sb), row, at(p.vv), int(p.pages), hkv, page, hd, st), "kv_dequant_pages"))
+      if (!done(rmlx_kv_dequant_pages(at(l.k), at(l.k_sb), row, at(p.kk), int(p.pages), hkv, page, hd, kPdl, st), "kv_dequant_pages") ||
+          !done(rmlx_kv_dequant_pages(at(l.v), at(l.v_sb), row, at(p.vv), int(p.pages), hkv, page, hd, kPdl, st), "kv_dequant_pages"))
         return false;
       k = at(p.kk); v = at(p.vv); table = at<int>(p.iota); blocks = int(p.pages);
     }

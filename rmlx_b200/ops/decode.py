@@ -538,7 +538,7 @@ _lib.register_cuda_sigs({
     "rmlx_rms_qkv_rope": ("ippppipfppppppppiiiiiiiiip", "i"),
     "rmlx_flash_decode_paged_q8": ("pppppppppppiiiiiiifip", "i"),
     "rmlx_rope_kv_write_q8": ("pppppppppppiiiiiiiip", "i"),
-    "rmlx_kv_dequant_pages": ("ppppiiiip", "i"),
+    "rmlx_kv_dequant_pages": ("ppppiiiiip", "i"),
 })
 
 
@@ -552,7 +552,7 @@ def kv_dequant_pages(codes: torch.Tensor, sb: torch.Tensor, table_row: torch.Ten
     if out is None:
         out = torch.empty(n_pages, hkv, page, d, dtype=torch.bfloat16, device=codes.device)
     rc = _lib.cuda().rmlx_kv_dequant_pages(codes.data_ptr(), sb.data_ptr(), table_row.data_ptr(),
-                                           out.data_ptr(), n_pages, hkv, page, d, _lib.stream_ptr())
+                                           out.data_ptr(), n_pages, hkv, page, d, 0, _lib.stream_ptr())
     _lib.check(rc, "kv_dequant_pages")
     return out
 
