@@ -69,6 +69,8 @@ struct NwParams {
   int out_stride, out_f32, res_stride;
   int E, M, N, K, swiglu, RT, KS;
   int CS, cs_log2, RL, xunits;   // even split: blocks of a cluster that share K; tiles per run; units of x
+  const int* choice;         // even split: row i of E = M rows meets expert choice[i] (none outside [0, experts)); null: by offsets
+  int experts;
   int split;                 // bf16 weights and a norm: x times its weight goes in two terms, in two tiles of rows
 };
 
@@ -587,6 +589,8 @@ __global__ void __launch_bounds__(NwShape<KIND, T>::THREADS, 1) narrow_gemm_kern
 //   * the loop has no work but its own: pointers that step, no plan kept in registers, no barrier. 16 warps of 128 registers spill nothing
 //     and stage x with half the barrier's stragglers of 24 warps of 80 (151936 x 4096 at 8 rows 78 us with 24 warps, 71 with 16 and two
 //     stages, 67 with three).
+//   * few (row, slot) pairs need no lists: each is an expert of its own, whose number is read from the choices; x stays where it is from
+//     one expert to the next if all pairs are of one row.
 //   * only rows that exist are staged: a column of B that holds nothing is a column of results that nobody takes.
 // Measured against narrow_gemm_kernel, chained launches, weights out of HBM, 4-bit (us, it / this; their bytes at the copy rate): 8
 // rows, 4096 x 4096 8.5 / 8.4 (1.5), 9216 x 4096 14.1 / 11.8 (3.3), 28672 x 4096 25 / 19 (10), 4096 x 14336 21 / 14 (5), 151936 x 4096 103 /
@@ -641,7 +645,18 @@ __global__ void __launch_bounds__(NeShape<KIND, T>::THREADS, 1) narrow_even_kern
   pdl_launch_dependents();
   if (p.norm && int(threadIdx.x) < gsh) nw_prefetch(p.norm + (k0 * 8 + threadIdx.x) * 64);
 
-  if (p.offsets) {
+  int* const s_map = s_off + kNwMaxExperts / 2;          // the experts of single rows
+  if (p.choice) {
+    pdl_wait();
+    if (warp == 0) {
+      const int c = lane < p.E ? p.choice[lane] : -1;
+      const unsigned is = __ballot_sync(0xffffffffu, unsigned(c) < unsigned(p.experts));
+      s_off[lane] = lane;
+      s_pre[lane] = __popc(is & ((1u << lane) - 1u)) * tiles_n;
+      s_map[lane] = c;
+      if (lane == 31) { s_off[32] = 32; s_pre[32] = __popc(is) * tiles_n; }
+    }
+  } else if (p.offsets) {
     pdl_wait();
     for (int i = threadIdx.x; i <= p.E; i += S::THREADS) {
       const int o = p.offsets[i];
@@ -705,7 +720,7 @@ __global__ void __launch_bounds__(NeShape<KIND, T>::THREADS, 1) narrow_even_kern
       if (u1 > u0) {
         const int tile = u0 / C;
         p_left = u1 - u0; p_c = u0 - tile * C; p_fresh = true;
-        const size_t row = size_t(p_e) * p.N + (tile0 + tile) * per;
+        const size_t row = size_t(p.choice ? s_map[p_e] : p_e) * p.N + (tile0 + tile) * per;
         p_w = p.w + (row + (lane >> 3)) * row_bytes + (k0 * S::PC + p_c) * kNwCB + (lane & 7) * 16;
         p_s = reinterpret_cast<const uint8_t*>((lane < 16 ? p.scales : p.biases) + (row + (lane & 7) + ((lane >> 3) & 1) * half) * groups +
                                                (k0 + p_c / S::PC) * 8);
@@ -739,7 +754,7 @@ __global__ void __launch_bounds__(NeShape<KIND, T>::THREADS, 1) narrow_even_kern
   };
 #pragma unroll 1
   for (int i = 0; i < S::D - 1; ++i) issue();
-  if (!p.offsets) pdl_wait();
+  if (!p.offsets && !p.choice) pdl_wait();
 
   // ---------------------------------------------------------------- x
   auto out_row = [&](int e, int mt, int i) {             // output row of the pass's i-th row of x, -1: none
@@ -846,7 +861,8 @@ __global__ void __launch_bounds__(NeShape<KIND, T>::THREADS, 1) narrow_even_kern
     int mt, tile0;
     const int tiles = run_at(item, e, mt, tile0), u = tiles * C;
     const int u0 = warp * u / S::W, u1 = (warp + 1) * u / S::W;
-    if (e != key_e || mt != key_m) { stage(e, mt); key_e = e; key_m = mt; }
+    // single rows that are all the same row of x stay where they are
+    if (const int x_of = p.choice && p.x_div >= p.M ? 0 : e; x_of != key_e || mt != key_m) { stage(e, mt); key_e = x_of; key_m = mt; }
     if (p.CS > 1) ne_cluster_sync(); else __syncthreads();
 
     float rs[T] = {};                                    // 1 / rms of row lane % 8 of the tile
@@ -1315,6 +1331,30 @@ extern "C" int rmlx_narrow_gemm(int w_kind, const void* w, const void* scales, c
     case 1: return launch_narrow_t<1>(p, T, hint, ks, pdl, st);
     default: return launch_narrow_t<2>(p, T, hint, ks, pdl, st);
   }
+}
+
+// Single (row, slot) pairs, up to 32: output row i is row i / x_div of x through expert choice[i] of w [experts, N, K] (4- or 8-bit);
+// rows whose choice is no expert are not written.
+extern "C" int rmlx_narrow_pairs(int w_kind, const void* w, const void* scales, const void* biases, const void* x, int x_stride, int x_div,
+                                 const int* choice, int experts, const void* norm, float eps, void* out, int out_stride, int out_f32,
+                                 int pairs, int N, int K, int swiglu, int pdl, cudaStream_t st) {
+  if (w_kind < 1 || !rmlx_narrow_supported(w_kind, N, K) || K > 32768 || pairs < 1 || pairs > 32 || experts < 1 || x_stride % 8 || x_div < 1 ||
+      (swiglu && N % 32) || !choice || !scales || !biases)
+    return -2;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(scales) |
+       reinterpret_cast<uintptr_t>(biases) | reinterpret_cast<uintptr_t>(norm)) & 15)
+    return -2;
+  NwParams p = {};
+  p.w = static_cast<const uint8_t*>(w);
+  p.scales = static_cast<const __nv_bfloat16*>(scales);
+  p.biases = static_cast<const __nv_bfloat16*>(biases);
+  p.x = static_cast<const __nv_bfloat16*>(x);
+  p.norm = static_cast<const __nv_bfloat16*>(norm);
+  p.out = out; p.eps = eps; p.x_stride = x_stride; p.x_div = x_div;
+  p.out_stride = out_stride; p.out_f32 = out_f32;
+  p.E = p.M = pairs; p.N = N; p.K = K; p.swiglu = swiglu;
+  p.choice = choice; p.experts = experts;
+  return w_kind == 1 ? launch_even<1, 1>(p, pairs, 0, pdl, st) : launch_even<2, 1>(p, pairs, 0, pdl, st);
 }
 
 extern "C" int rmlx_narrow_group(const int* idx, int pairs, int E, int* offsets, int* order, int pdl, cudaStream_t st) {

@@ -241,10 +241,10 @@ class CachedDecode(DecodeEngineBase):
             self.wts = torch.zeros(B, k, dtype=torch.float32, device=dev)
             self.act = torch.zeros(B * k, i_local, **bf)
             self.router_scratch = D.RouterScratch(B, moe.num_experts, dev)
-            # several rows on one GPU: every chosen expert's weights are read once for all rows (ops/narrow.py)
+            # on one GPU: every chosen expert's weights are read once for all rows, or few pairs one by one (ops/narrow.py)
             self.expert_scratch = None
             routed = [l for l in model.w.layers if l.experts_gate_up is not None]
-            if B > 1 and model.layout.world == 1 and all(
+            if model.layout.world == 1 and all(
                     narrow.supported(l.experts_gate_up) and narrow.supported(l.experts_down) and
                     l.experts_gate_up.n % 32 == 0 and l.experts_gate_up.experts == moe.num_experts for l in routed):
                 l = max(routed, key=lambda l: l.experts_gate_up.n)
@@ -314,6 +314,11 @@ class CachedDecode(DecodeEngineBase):
                 idx, wts, act = self.idx[:nb], self.wts[:nb], self.act[:nb * k]
                 D.moe_router(h2, lw.router, lw.norm2, eps, k, lw.expert_bias,
                              self.router_scratch, idx, wts, pdl=pdl)
+                if self.expert_scratch is not None and D.pairs_apart() and lw.norm2.data_ptr() % 16 == 0 and \
+                        narrow.pays_pairs(lw.experts_gate_up, lw.experts_down, nb, k):
+                    narrow.pairs_ffn(h2, idx, wts, lw.experts_gate_up, lw.experts_down, lw.norm2, eps, residual=h2, out=h,
+                                     scratch=self.expert_scratch, pdl=pdl)
+                    continue
                 if self.expert_scratch is not None and narrow.pays_shared(lw.experts_gate_up, nb, k) and \
                         D._several(nb, lw.experts_gate_up, h2, lw.norm2, swiglu=True):
                     narrow.expert_ffn(h2, idx, wts, lw.experts_gate_up, lw.experts_down, lw.norm2, eps, residual=h2,

@@ -117,14 +117,22 @@ def _several(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[torch.Te
     if b == 1:
         # one row of a wide 4- or 8-bit weight (us, weight-streaming / per-row, 8-bit: streaming). 4-bit: 151936 x 4096 66 / 78, 28672 x 4096
         # 17 / 21, 32768 x 2048 11 / 15, 16384 x 2048 8.8 / 10.6, but 9 / 8 with SwiGLU; 9216 x 4096 9.0 / 9.2, 6144 x 4096 8.1 / 7.9. 8-bit:
-        # 151936 x 4096 107 / 139, 32768 x 2048 14 / 18, 16384 x 2048 9.5 / 11.5 (SwiGLU 9.5 / 11.7), 2048 x 8192 9.1 / 8.1
-        if w.kind == W_BF16 or w.n < 16384 or w.n * w.k < (1 << 26 if swiglu else 1 << 25):
+        # 151936 x 4096 107 / 139, 32768 x 2048 14 / 18, 16384 x 2048 9.5 / 11.5 (SwiGLU 9.5 / 11.7), 2048 x 8192 9.1 / 8.1.
+        # Narrower ones from 2^26 entries on: 8192 x 8192 12.7 / 14.6, 10240 x 8192 14.3 / 19.6, 4096 x 28672 20 / 22; 4096 x 16384 13.6 / 13.3,
+        # in 8 bits 16.8 / 21.1
+        if w.kind == W_BF16 or (w.n * w.k < 1 << 26 and (swiglu or w.n < 16384 or w.n * w.k < 1 << 25)):
             return False
     # two rows of 4-bit weights: a 16384 x 2048 projection 9 us against 11, a 3072 x 2048 one 6 against 5
     least = 0 if b >= 4 else 1 << 24 if b == 2 and w.kind == W_Q4 else 1 << 20
     return (b >= 1 and _STREAM and q4_path() == "auto" and w.n * w.k >= least and narrow.supported(w) and
             x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and (norm_w is None or norm_w.data_ptr() % 16 == 0) and
             not (b <= 3 and w.kind == W_BF16 and not swiglu and _rows_stream(b, w.n * w.k, w.k, norm_w is not None)))
+
+
+def pairs_apart() -> bool:
+    """Whether the switches leave the experts of few rows to ``narrow.pairs_ffn``: like ``_several``, and with both expert
+    projections streaming."""
+    return _STREAM and q4_path() == "auto" and "moe_gate_up" in _STREAM_OPS and "moe_down" in _STREAM_OPS
 
 
 def _rows_stream(b: int, entries: int, k: int, norm: bool) -> bool:
@@ -151,8 +159,11 @@ def projects_apart(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[to
     296 / 285 at 4; 6144 x 4096 552 / 518, 556 / 541, 567 / 592; 9216 x 4096 (two layers) 618 / 612, 743 / 745, 894 / 897. From five
     rows on the one launch is two. 8-bit: 3072 x 2048 245 / 238 at 2 rows, 245 / 252 at 3; 9216 x 4096 (two layers) 460 / 466 at 2:
     always apart, where the sums are fp32 (the per-row kernel adds 8-bit products in fp16)."""
-    if b < 2 or w.kind == W_Q4:
-        return b >= 2
+    if b < 2:
+        # one row, 4-bit: 10240 x 8192 15.9 us apart, 20.8 in one launch; 9216 x 4096 10.6 / 10.0, 6144 x 4096 9.3 / 9.2
+        return b == 1 and w.kind == W_Q4 and w.n * w.k >= 1 << 26 and _several(b, w, x, norm_w)
+    if w.kind == W_Q4:
+        return True
     if w.kind == W_BF16 and b <= (4 if w.n * w.k <= 1 << 23 else 3):
         return False
     return _several(b, w, x, norm_w)

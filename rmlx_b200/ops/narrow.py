@@ -14,6 +14,7 @@ from .weights import LinearWeight, W_BF16, W_Q4, W_Q8
 _lib.register_cuda_sigs({
     "rmlx_narrow_supported": ("iii", "i"),
     "rmlx_narrow_gemm": ("ippppiippipfpipiiiiiiiiip", "i"),
+    "rmlx_narrow_pairs": ("ippppiipipfpiiiiiiip", "i"),
     "rmlx_narrow_group": ("piippip", "i"),
     "rmlx_narrow_combine": ("ppippipiiiiip", "i"),
 })
@@ -171,4 +172,47 @@ def expert_ffn(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, gate_up: L
     offsets, order = group_pairs(idx, gate_up.experts, s.offsets, s.order[:pairs], pdl=pdl)
     act = narrow_gemm(x, gate_up, norm_w, eps, out=s.act[:pairs], swiglu=True, offsets=offsets, order=order, x_div=k, rows=pairs, pdl=pdl)
     y = narrow_gemm(act, down, out=s.y[:pairs], offsets=offsets, order=order, rows=pairs, pdl=pdl)
+    return combine(y, idx, gate_up.experts, wts, residual, out, pdl=pdl)
+
+
+PAIRS = 32       # (row, slot) pairs that ``pairs_ffn`` takes
+
+
+def pays_pairs(gate_up: LinearWeight, down: LinearWeight, rows: int, top_k: int) -> bool:
+    """Whether so few rows' pairs should be multiplied one by one (``pairs_ffn``, three launches): quantised experts, hardly any of which is
+    chosen twice (at random choices a quarter more pairs than experts at most), and enough of them that the even split of the work
+    outweighs its launches. Measured, chained (us: pairs / ``expert_ffn`` / streaming kernels). 4-bit, 128 experts of 4096 x 1536, 8 of
+    them: 37.5 / 51 / 37.2 for one row, 51 / 61 / 60 for two, 79 / 89 / 107 for four; 8 of 4096 x 14336, two of them: 54 / 58 / 69, 93 / 97 /
+    122, three rows 124 / 117 / 175; 64 of 2048 x 1536, six of them: 24 / 33 / 20, 32 / 39 / 31, three rows 38 / 42 / 42. 8-bit, 128 of 2048
+    x 1024, 8 of them: 27 / 38 / 23, 35 / 48 / 36, four rows 50 / 61 / 61; 8 of 4096 x 3584, two of them: 30 / 34 / 35."""
+    pairs, e = rows * top_k, gate_up.experts
+    if gate_up.kind not in (W_Q4, W_Q8) or down.kind != gate_up.kind or not 0 < pairs <= PAIRS or e < 1:
+        return False
+    read = pairs * (gate_up.n * gate_up.k + down.n * down.k) * (0.5625 if gate_up.kind == W_Q4 else 1.0625)
+    distinct = e * (1.0 - (1.0 - min(1.0, top_k / e)) ** rows)
+    return (read >= 90e6 and pairs <= 1.25 * distinct and gate_up.k <= 32768 and down.k <= 32768 and gate_up.n % 32 == 0 and
+            gate_up.scales.dtype == down.scales.dtype == torch.bfloat16 and supported(gate_up) and supported(down))
+
+
+def pairs_gemm(x: torch.Tensor, w: LinearWeight, idx: torch.Tensor, x_div: int, out: torch.Tensor, norm_w: Optional[torch.Tensor] = None,
+               eps: float = 1e-6, swiglu: bool = False, pdl: bool = False) -> torch.Tensor:
+    """out[i] = rmsnorm(x[i // x_div]; norm_w) W_e^T, e = idx[i] of the flattened choices; rows whose choice is no expert stay as they are."""
+    _lib.require_cuda_tensor(x, w.w, idx)
+    n, k, pairs = w.n, w.k, idx.numel()
+    assert x.dtype == torch.bfloat16 and x.stride(1) == 1 and x.shape[1] == k and idx.dtype == torch.int32 and idx.is_contiguous()
+    assert _holds(out, pairs, n // 2 if swiglu else n) and x.shape[0] * x_div >= pairs
+    rc = _lib.cuda().rmlx_narrow_pairs(w.kind, w.w.data_ptr(), w.scales.data_ptr(), w.biases.data_ptr(), x.data_ptr(), x.stride(0), x_div,
+                                       idx.data_ptr(), w.experts, _lib.ptr(norm_w), eps, out.data_ptr(), out.stride(0),
+                                       int(out.dtype == torch.float32), pairs, n, k, int(swiglu), int(pdl), _lib.stream_ptr())
+    _lib.check(rc, "narrow_pairs")
+    return out
+
+
+def pairs_ffn(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, gate_up: LinearWeight, down: LinearWeight, norm_w: torch.Tensor,
+              eps: float, residual: torch.Tensor, out: torch.Tensor, scratch: ExpertScratch, pdl: bool = False) -> torch.Tensor:
+    """``expert_ffn`` of so few rows that hardly any share an expert: every pair by itself, without the lists."""
+    k = idx.shape[1]
+    pairs = idx.numel()
+    act = pairs_gemm(x, gate_up, idx, k, scratch.act[:pairs], norm_w, eps, swiglu=True, pdl=pdl)
+    y = pairs_gemm(act, down, idx, 1, scratch.y[:pairs], pdl=pdl)
     return combine(y, idx, gate_up.experts, wts, residual, out, pdl=pdl)

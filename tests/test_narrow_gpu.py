@@ -313,3 +313,56 @@ def test_one_row_of_a_wide_weight(dev, kind, n, k, wide):
     # the weight-streaming kernel's sums are fp32; the per-row kernels multiply 4- and 8-bit weights in fp16
     bound = 1e-5 if wide or kind is None else 2e-3
     assert _rel(D.rms_gemv(x, w, residual=res, out_dtype=torch.float32), x.double() @ wd.t() + res.double()) < bound
+
+
+@pytest.mark.parametrize("kind", ["q4", "q8"])
+@pytest.mark.parametrize("rows,top,experts,k,n", [(1, 8, 128, 512, 32), (1, 1, 2, 1536, 96), (4, 8, 16, 1024, 64), (3, 5, 7, 4096, 160), (1, 32, 40, 8192, 32)])
+def test_pairs(dev, kind, rows, top, experts, k, n):
+    """Pairs one by one: every expert's rows, choices that are no expert, an expert chosen twice, norm, SwiGLU; then down and combined."""
+    from rmlx_b200.ops import narrow
+    w, wd, x, g = _case(dev, kind, n, k, rows, experts=experts, seed=19)
+    nw = (torch.rand(k, device=dev, generator=g) + 0.5).to(torch.bfloat16)
+    idx = torch.randint(0, experts, (rows, top), device=dev, generator=g, dtype=torch.int32)
+    if rows * top > 1:
+        idx[0, 0] = experts
+        idx[-1, -1] = 0x7fffffff
+    flat = idx.flatten().tolist()
+    real = [i for i, e in enumerate(flat) if e < experts]
+    xd = x.double()
+    xn = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    for norm, src in ((None, xd), (nw, xn)):
+        out = torch.full((rows * top, n), 7.0, device=dev)
+        narrow.pairs_gemm(x, w, idx, top, out, norm)
+        want = torch.stack([src[i // top] @ wd[flat[i]].t() for i in real])
+        # without a norm x is exact in the products; with one it is rounded to fp16, 2^-12 of each value at most, half that on average
+        assert _rel(out[real], want) < (2e-5 if norm is None else 2.0 ** -11)
+        assert all(bool((out[i] == 7.0).all()) for i in range(rows * top) if i not in real)
+    act = torch.zeros(rows * top, n // 2, device=dev, dtype=torch.bfloat16)
+    narrow.pairs_gemm(x, w, idx, top, act, nw, swiglu=True)
+    gate, up = want[:, :n // 2], want[:, n // 2:]
+    assert _rel(act[real], gate * torch.sigmoid(gate) * up) < 6e-3
+    # a row of its own for each pair
+    y = torch.randn(rows * top, k, device=dev, generator=g).to(torch.bfloat16)
+    out = torch.zeros(rows * top, n, device=dev)
+    narrow.pairs_gemm(y, w, idx, 1, out)
+    assert _rel(out[real], torch.stack([y[i].double() @ wd[flat[i]].t() for i in real])) < 2e-5
+
+
+def test_pairs_in_a_decode_step(dev):
+    """Steps of 1 to 4 rows whose experts go pair by pair against the streaming kernels: the same tokens' logits within the latter's
+    rounding (they multiply in fp16, 1e-3 a projection)."""
+    from rmlx_b200.ops import decode as D, narrow
+    from rmlx_b200.ops.weights import LinearWeight
+    g = torch.Generator(device=dev).manual_seed(3)
+    up, down = (LinearWeight.random(a, b, "q4", dev, experts=16, generator=g) for a, b in ((28672, 2048), (2048, 14336)))
+    assert [narrow.pays_pairs(up, down, r, 2) for r in (0, 1, 2, 4, 9, 17)] == [False, True, True, True, False, False] and D.pairs_apart()
+    x = torch.randn(4, 2048, device=dev, generator=g).to(torch.bfloat16)
+    nw = torch.ones(2048, device=dev, dtype=torch.bfloat16)
+    sc = narrow.ExpertScratch(4, 2, up, down)
+    for r in (1, 4):
+        idx = torch.stack([torch.randperm(16, device=dev, generator=g)[:2] for _ in range(r)]).int().contiguous()
+        wts = torch.rand(r, 2, device=dev, generator=g)
+        got = narrow.pairs_ffn(x[:r], idx, wts, up, down, nw, 1e-6, x[:r], torch.empty_like(x[:r]), sc)
+        act = D.moe_gate_up(x[:r], up, nw, 1e-6, idx)
+        want = D.moe_down(act, down, idx, wts, residual=x[:r])
+        assert _rel(got.float() - x[:r].float(), (want.float() - x[:r].float()).double()) < 1e-2
