@@ -253,6 +253,9 @@ class PromptRun:
         bf16, pages = torch.bfloat16, (pos0 + t + 15) // 16
         q8 = cache.quantized
         row = cache.block_table[cache.slot_of[seq_id]]
+        # addresses go to the kernels unseen: host tensors, and ids of another device, are left to the launches one by one, which raise
+        if not mw.embed.is_cuda or not m.cos.is_cuda or not token_ids.device == row.device == mw.embed.device:
+            return None
         if row.numel() < pages or mw.embed.dtype != bf16:
             return None
         recs = array.array("q")
@@ -260,7 +263,8 @@ class PromptRun:
         for li, lw in enumerate(mw.layers):
             n1, n2, kc, vc = lw.norm1, lw.norm2, cache.k[li], cache.v[li]
             if n1.dtype != bf16 or n2.dtype != bf16 or (n1.data_ptr() | n2.data_ptr()) % 16 or not n1.is_contiguous() or not n2.is_contiguous() \
-                    or not kc.is_contiguous() or not vc.is_contiguous() or kc.shape != vc.shape or kc.shape[3] != hd:
+                    or not kc.is_contiguous() or not vc.is_contiguous() or kc.shape != vc.shape or kc.shape[3] != hd or \
+                    not (n1.is_cuda and n2.is_cuda and kc.is_cuda and vc.is_cuda):
                 return None
             e = k = 0
             if lw.router is not None:
@@ -268,7 +272,7 @@ class PromptRun:
                 e, k = moe.num_experts, moe.num_experts_per_token
                 up, down, bias = lw.experts_gate_up, lw.experts_down, lw.expert_bias
                 if lw.shared_gate_up is not None or lw.expert_base or up.experts != e or r.dtype != bf16 or not r.is_contiguous() or \
-                        (bias is not None and (bias.dtype != torch.float32 or not bias.is_contiguous())):
+                        not r.is_cuda or (bias is not None and (not bias.is_cuda or bias.dtype != torch.float32 or not bias.is_contiguous())):
                     return None
                 pairs, most = max(pairs, t * k), max(most, e)
                 if narrow.pays_grouped(up, down, t * k):
@@ -295,7 +299,8 @@ class PromptRun:
                          0 if not e or bias is None else bias.data_ptr(), e, k))
             for w, route in ((lw.wqkv, r_qkv), (lw.wo, r_out), (up, r_up), (down, r_down)):
                 s, b = w.scales, w.biases
-                if s is not None and not (s.is_contiguous() and b.is_contiguous() and w.w.is_contiguous()):
+                if not w.w.is_cuda or (s is not None and not (s.is_cuda and b.is_cuda and s.is_contiguous() and b.is_contiguous() and
+                                                              w.w.is_contiguous())):
                     return None
                 if route & 15 == self.EXPAND:
                     dense = max(dense, w.n * w.k * 2)

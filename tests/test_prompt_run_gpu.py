@@ -91,3 +91,17 @@ def test_not_covered(dev):
     assert float((_prompts(model, [40], None, False)[0][0] - first).norm() / first.norm()) < 1e-2
     model.w.layers[0].wqkv = LinearWeight(W_BF16, wide[:, :model.cfg.hidden_size].contiguous() * 2)
     assert not torch.equal(_prompts(model, [40], None, True)[0][0], first)
+
+
+def test_host_ids_raise(dev):
+    """Ids on the host (the attached path called directly) raise before anything is launched, and the model goes on working."""
+    from rmlx_b200 import _lib
+    from rmlx_b200.models.prefill import NativePrefill
+    model = _model(dev, 0, "q4")
+    native, cache = NativePrefill(model), model.new_cache(8, max_seqs=1)
+    cache.add_sequence(0)
+    ids = torch.arange(20, dtype=torch.int32)
+    assert native.at_once.run(ids, cache, 0, 0) is None
+    with pytest.raises(_lib.NativeError):
+        native(ids, cache, 0)
+    assert torch.isfinite(native(ids.to(dev), cache, 0)).all()
