@@ -151,7 +151,8 @@ def pays_shared(gate_up: LinearWeight, rows: int, top_k: int) -> bool:
 
 
 class ExpertScratch:
-    """Buffers of ``expert_ffn`` for up to ``rows`` rows, for callers whose launches may not allocate."""
+    """Buffers of ``expert_ffn`` and ``pairs_ffn`` for up to ``rows`` rows, for callers whose launches may not allocate. Experts narrower
+    than those it was made for use the first columns of ``act``."""
 
     def __init__(self, rows: int, top_k: int, gate_up: LinearWeight, down: LinearWeight):
         dev, pairs = gate_up.device, rows * top_k
@@ -170,7 +171,8 @@ def expert_ffn(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, gate_up: L
     pairs = t * k
     s = scratch or ExpertScratch(t, k, gate_up, down)
     offsets, order = group_pairs(idx, gate_up.experts, s.offsets, s.order[:pairs], pdl=pdl)
-    act = narrow_gemm(x, gate_up, norm_w, eps, out=s.act[:pairs], swiglu=True, offsets=offsets, order=order, x_div=k, rows=pairs, pdl=pdl)
+    act = narrow_gemm(x, gate_up, norm_w, eps, out=s.act[:pairs, :gate_up.n // 2], swiglu=True, offsets=offsets, order=order, x_div=k,
+                      rows=pairs, pdl=pdl)
     y = narrow_gemm(act, down, out=s.y[:pairs], offsets=offsets, order=order, rows=pairs, pdl=pdl)
     return combine(y, idx, gate_up.experts, wts, residual, out, pdl=pdl)
 
@@ -213,6 +215,6 @@ def pairs_ffn(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, gate_up: Li
     """``expert_ffn`` of so few rows that hardly any share an expert: every pair by itself, without the lists."""
     k = idx.shape[1]
     pairs = idx.numel()
-    act = pairs_gemm(x, gate_up, idx, k, scratch.act[:pairs], norm_w, eps, swiglu=True, pdl=pdl)
+    act = pairs_gemm(x, gate_up, idx, k, scratch.act[:pairs, :gate_up.n // 2], norm_w, eps, swiglu=True, pdl=pdl)
     y = pairs_gemm(act, down, idx, 1, scratch.y[:pairs], pdl=pdl)
     return combine(y, idx, gate_up.experts, wts, residual, out, pdl=pdl)

@@ -63,3 +63,42 @@ def test_launcher_refuses_before_any_launch():
         for name in ("w", "scales", "biases", "x", "norm"):
             assert call(kind, **{name: at[name] + 8}) == -2, name
         assert call(kind, scales=None) == -2 and call(kind, biases=None) == -2
+
+
+@pytest.mark.parametrize("form", ["expert_ffn", "pairs_ffn"])
+def test_experts_narrower_than_the_scratch(monkeypatch, form):
+    """A scratch sized for the widest layer of a model serves its narrower layers too: they take the columns that they fill. The
+    kernels' places are taken by plain products, which hold the operands to the shapes that the kernels' wrappers ask for."""
+    g = torch.Generator().manual_seed(3)
+    rows, top, experts, d = 3, 2, 4, 64
+    layers = [tuple(LinearWeight(W_BF16, 0.1 * torch.randn(experts, n, k, generator=g)) for n, k in ((2 * inner, d), (d, inner)))
+              for inner in (96, 32)]
+
+    def product(x, w, chosen, x_div, out, swiglu):
+        assert x.shape[1] == w.k and out.shape[0] >= len(chosen) and out.shape[1] >= (w.n // 2 if swiglu else w.n)
+        for i, e in enumerate(chosen):
+            y = w.w[e] @ x[i // x_div].float()
+            if swiglu:
+                y = torch.nn.functional.silu(y[:w.n // 2]) * y[w.n // 2:]
+            out[i, :y.numel()] = y
+        return out
+
+    monkeypatch.setattr(narrow, "group_pairs", lambda idx, *a, **kw: (idx, idx))
+    monkeypatch.setattr(narrow, "narrow_gemm", lambda x, w, norm_w=None, eps=0., out=None, swiglu=False, offsets=None, order=None, x_div=1,
+                        rows=None, pdl=False: product(x, w, idx.flatten().tolist(), x_div, out, swiglu))
+    monkeypatch.setattr(narrow, "pairs_gemm", lambda x, w, idx, x_div, out, norm_w=None, eps=0., swiglu=False, pdl=False:
+                        product(x, w, idx.flatten().tolist(), x_div, out, swiglu))
+    monkeypatch.setattr(narrow, "combine", lambda y, idx, experts, wts, residual, out, pdl=False:
+                        residual + (wts[..., None] * y[:, :d].unflatten(0, idx.shape)).sum(1))
+    scratch = narrow.ExpertScratch(rows, top, *layers[0])
+    for up, down in layers:
+        x, idx = torch.randn(rows, d, generator=g), torch.randint(0, experts, (rows, top), generator=g)
+        wts, res = torch.rand(rows, top, generator=g), torch.randn(rows, d, generator=g)
+        got = getattr(narrow, form)(x, idx, wts, up, down, torch.ones(d), 1e-6, residual=res, out=None, scratch=scratch)
+        want = res.clone()
+        for r in range(rows):
+            for s in range(top):
+                gate, value = (up.w[idx[r, s]] @ x[r]).chunk(2)
+                act = (torch.nn.functional.silu(gate) * value).to(torch.bfloat16).float()     # the buffer between the two is bf16
+                want[r] += wts[r, s] * (down.w[idx[r, s]] @ act)
+        assert torch.allclose(got, want, atol=1e-5)

@@ -366,3 +366,22 @@ def test_pairs_in_a_decode_step(dev):
         act = D.moe_gate_up(x[:r], up, nw, 1e-6, idx)
         want = D.moe_down(act, down, idx, wts, residual=x[:r])
         assert _rel(got.float() - x[:r].float(), (want.float() - x[:r].float()).double()) < 1e-2
+
+
+@pytest.mark.parametrize("kind,rows", [("q4", 1), ("q4", 3), ("q8", 2)])
+def test_experts_narrower_than_the_scratch(dev, kind, rows):
+    """A scratch made for wider experts gives the same results to the bit as one of the experts' own width."""
+    from rmlx_b200.ops import narrow
+    from rmlx_b200.ops.weights import LinearWeight
+    g = torch.Generator(device=dev).manual_seed(4)
+    d, top, experts = 1024, 4, 16
+    wide, own = (tuple(LinearWeight.random(a, b, kind, dev, experts=experts, generator=g) for a, b in ((2 * inner, d), (d, inner)))
+                 for inner in (1536, 512))
+    x = torch.randn(rows, d, device=dev, generator=g).to(torch.bfloat16)
+    nw = torch.ones(d, device=dev, dtype=torch.bfloat16)
+    idx = torch.randint(0, experts, (rows, top), device=dev, generator=g, dtype=torch.int32)
+    wts = torch.rand(rows, top, device=dev, generator=g)
+    for ffn in (narrow.expert_ffn, narrow.pairs_ffn):
+        got, want = (ffn(x, idx, wts, *own, nw, 1e-6, residual=x, out=torch.empty_like(x), scratch=narrow.ExpertScratch(rows, top, *of))
+                     for of in (wide, own))
+        assert torch.equal(got, want)
