@@ -12,6 +12,7 @@ from typing import Optional
 import torch
 
 from .. import _lib
+from . import decode
 from .gemm import GemmStatus
 
 _lib.register_cuda_sigs({
@@ -36,8 +37,9 @@ FEW_ROWS = 8
 
 
 def few_rows_plan(t: int, hq: int, hkv: int, head_dim: int, tokens: int, q8: bool) -> int:
-    """The cluster plan for ``t`` last rows of a sequence of ``tokens``; 0: the prompt kernels."""
-    if t > FEW_ROWS or head_dim not in (64, 128):
+    """The cluster plan for ``t`` last rows of a sequence of ``tokens``; 0: the prompt kernels, which also take them where the decode
+    kernel is switched off (``RMLX_FLASH_DECODE_CLUSTER=0``) or ``RMLX_FLASH_PREFILL=mma`` names one of theirs."""
+    if t > FEW_ROWS or head_dim not in (64, 128) or not decode._FD_CLUSTER or os.environ.get("RMLX_FLASH_PREFILL", "tc") == "mma":
         return 0
     lib = _lib.cuda()
     return int(lib.rmlx_flash_decode_cluster_plan(t, t * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv), tokens, head_dim, int(q8)))

@@ -46,3 +46,28 @@ def test_host_tensors_raise_before_any_launch(monkeypatch, ids):
     with pytest.raises(_lib.NativeError):
         native(ids, cache, 0)
     assert not [name for name in lib.called if name in ("rmlx_prompt_run", "rmlx_embedding")]
+
+
+def test_few_rows_follow_the_kernel_switches(monkeypatch):
+    """Portions of up to eight rows attend on the decode kernel, unless the switch of that kernel is off or the one of the prompt kernels
+    names its ``mma.sync`` form."""
+    from rmlx_b200.ops import attention, decode
+
+    class _Plans:
+        rmlx_flash_decode_gtiles = staticmethod(lambda hq, hkv: 1)
+        rmlx_flash_decode_cluster_plan = staticmethod(lambda batch, tiles, tokens, hd, q8: 4 << 16 | tiles)
+
+    monkeypatch.setattr(_lib, "cuda", _Plans)
+    monkeypatch.delenv("RMLX_FLASH_PREFILL", raising=False)
+    monkeypatch.setattr(decode, "_FD_CLUSTER", True)
+
+    def plan(t=5):
+        return attention.few_rows_plan(t, 16, 4, 128, 1000, False)
+
+    assert plan() == 4 << 16 | 20 and plan(8) and plan(9) == 0 and attention.few_rows_plan(5, 16, 4, 96, 1000, False) == 0
+    monkeypatch.setenv("RMLX_FLASH_PREFILL", "mma")
+    assert plan() == 0
+    monkeypatch.setenv("RMLX_FLASH_PREFILL", "tc")
+    assert plan()
+    monkeypatch.setattr(decode, "_FD_CLUSTER", False)
+    assert plan() == 0
