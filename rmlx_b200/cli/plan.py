@@ -342,8 +342,7 @@ def plan(model: str = "moe-a22b", weights: str = "q4", tp: int = 1, batch: int =
     w = weight_bytes_per_gpu(cfg, weights, tp, expert_parallel)
     kv_tok = kv_bytes_per_token_per_gpu(cfg, tp, kv_quant)
     budget = int(HBM_BYTES * budget_fraction)
-    scratch = PrefillPlan(cfg, prefill_chunk, ParallelLayout(0, tp, expert_parallel)).scratch_bytes
-    scratch = scratch() if callable(scratch) else scratch
+    scratch = PrefillPlan(cfg, prefill_chunk, ParallelLayout(0, tp, expert_parallel), weights, kv_quant, ctx).scratch_bytes
     free_for_kv = budget - w["total"] - scratch
     kv_needed = batch * ctx * kv_tok
     return {

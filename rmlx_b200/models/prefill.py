@@ -33,7 +33,8 @@ from ..ops.gemm import GemmStatus, gemm_bf16
 from ..ops import grouped
 from ..ops.grouped import moe_prefill_ffn
 from ..ops.quantized import pair_pays, qmm, row_gemm, row_supported, row_tables_ready, tiles_route, xgemm
-from ..ops.weights import LinearWeight, W_BF16, W_Q4
+from ..ops.weights import LinearWeight, W_BF16, W_Q4, W_Q8
+from .prefill_plan import PIECES, PrefillPlan, prompt_block
 
 
 def _narrow(x: torch.Tensor, w: LinearWeight) -> bool:
@@ -308,14 +309,11 @@ class PromptRun:
                              w.experts if e else 0, w.kind, int(s is not None and w.scales_f16), route))
         few = few_rows_plan(t, hq, hkv, hd, pos0 + t, q8)
         kv_bytes = pages * hkv * 16 * hd * 2 if q8 and not few else 0
-        # one block of work space, in pieces at 256-byte addresses
-        at, offs = 0, []
-        for size in (t * d * 2, t * d * 2, t * d * 2, t * (hq + 2 * hkv) * hd * 2, t * hq * hd * 2, t * hq * hd * 2, act, mid, dense,
-                     kv_bytes, kv_bytes, t * most * 4, pairs * 4, pairs * 4, most * 4,
-                     (most + 1) * 4, pairs * 4, most * 4, pairs * 4, xs, y):
-            offs.append(at)
-            at += (size + 255) & ~255
-        ws = torch.empty(at, dtype=torch.uint8, device=m.device)
+        where, size = prompt_block(dict(
+            h0=t * d * 2, h1=t * d * 2, xn=t * d * 2, qkv=t * (hq + 2 * hkv) * hd * 2, q=t * hq * hd * 2, attn=t * hq * hd * 2, act=act, mid=mid,
+            dense=dense, kk=kv_bytes, vv=kv_bytes, logits=t * most * 4, idx=pairs * 4, wts=pairs * 4, counts=most * 4,
+            offsets=(most + 1) * 4 if most else 0, order=pairs * 4, cursors=most * 4, row_of=pairs * 4, xs=xs, y=y))
+        ws = torch.empty(size, dtype=torch.uint8, device=m.device)
         base = ws.data_ptr()
         iota, zeros = self._tables(pos0 + t + 1)
         window = int(cfg.sliding_window or 0)
@@ -323,7 +321,7 @@ class PromptRun:
             len(mw.layers), t, d, hq, hkv, hd, pos0, window, row.numel(), 16, cache.k[0].shape[0], int(cfg.rope_traditional),
             int(prefill_kernel_choice(hd, window) == "tc"), int(os.environ.get("RMLX_FLASH_PREFILL_LANES", "0")), pages, few, mw.embed.shape[0],
             mw.embed.data_ptr(), token_ids.data_ptr(), row.data_ptr(), iota.data_ptr() + 4 * pos0, zeros.data_ptr(), iota.data_ptr(),
-            m.cos.data_ptr(), m.sin.data_ptr(), GemmStatus.get(m.device).data_ptr(), *(base + o for o in offs)))
+            m.cos.data_ptr(), m.sin.data_ptr(), GemmStatus.get(m.device).data_ptr(), *(base + where[name] for name in PIECES)))
         lib = _lib.cuda()
         words = (ctypes.c_int * 2)()
         lib.rmlx_prompt_sizes(words)
@@ -547,10 +545,13 @@ class BatchedDecode:
 def plan_chunk(model, scratch_limit_bytes: int = 4 << 30, longest: int = 8192) -> int:
     """Largest prompt chunk (a multiple of 128, at most ``longest``) whose per-layer intermediates
     stay within ``scratch_limit_bytes`` according to the layer's static plan
-    (``models.prefill_plan.PrefillPlan``: every launch of a layer with its output size)."""
-    from .prefill_plan import PrefillPlan
+    (``models.prefill_plan.PrefillPlan``, which lays them out as the portion itself does). Not counted, because no chunk makes
+    them fewer: an 8-bit cache's pages, expanded for the whole context, one layer at a time."""
+    kinds = [w for l in getattr(getattr(model, "w", None), "layers", ()) for w in (l.wqkv, l.wo, l.w_gate_up, l.w_down) if w is not None]
+    weights = "q8" if any(w.kind == W_Q8 or (w.kind == W_Q4 and w.scales_f16) for w in kinds) else \
+        "q4" if any(w.kind == W_Q4 for w in kinds) else "bf16"
     chunk = longest
-    while chunk > 128 and PrefillPlan(model.cfg, chunk, model.layout).scratch_bytes > scratch_limit_bytes:
+    while chunk > 128 and PrefillPlan(model.cfg, chunk, model.layout, weights).scratch_bytes > scratch_limit_bytes:
         chunk -= 128
     return chunk
 

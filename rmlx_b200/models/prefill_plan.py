@@ -2,7 +2,8 @@
 
 ``PrefillPlan`` lists, for a sequence length, the launches of one layer with their shapes and the
 scratch each needs (the reference builds the same per-length ``PlanStep`` lists,
-crates/rmlx-nn/src/prefill_plan.rs:16-300); ``PrefillPool`` keeps a few slots of pre-allocated
+crates/rmlx-nn/src/prefill_plan.rs:16-300); ``prompt_block`` lays that scratch out in one block, for the plan and for
+the portion that runs alike; ``PrefillPool`` keeps a few slots of pre-allocated
 intermediates sized for the largest planned length so that chunks of a prompt do not allocate
 (crates/rmlx-nn/src/prefill_pool.rs:33-160, crates/rmlx-nn/src/dynamic.rs:16-104).
 """
@@ -31,8 +32,41 @@ class PlanStep:
         return 2.0 * self.m * self.n * self.k
 
 
+#: The pieces of a portion's work space, in the order of the native call's record (csrc/runtime/prompt_run.cu).
+PIECES = ("h0", "h1", "xn", "qkv", "q", "attn", "act", "mid", "dense", "kk", "vv", "logits", "idx", "wts", "counts", "offsets", "order",
+          "cursors", "row_of", "xs", "y")
+# The residual stream, a weight expanded for one product and the routing's tables have places of their own. The rest belongs to one
+# half of a layer and is dead in the other, so the halves share their memory; and within a half a piece lies where one was
+# that has been read by then (queries on the normed rows, the heads' results on qkv, ...).
+_OWN = ("h0", "h1", "dense", "idx", "wts", "counts", "offsets", "order", "cursors", "row_of")
+_HALVES = ((("xn", "q"), ("qkv", "attn"), ("kk",), ("vv",)), (("xn",), ("logits", "act"), ("mid", "xs", "y")))
+
+
+def prompt_block(sizes: Dict[str, int]) -> Tuple[Dict[str, int], int]:
+    """Where the pieces of a portion's work space lie in one block (bytes from its start, 256-byte addresses), and the block's size.
+    ``sizes``: bytes of each piece of ``PIECES``; those that are left out are empty. A launch writes only after the one before it has
+    finished, so what no later launch reads is free."""
+    size = {name: (sizes.get(name, 0) + 255) & ~255 for name in PIECES}
+    at, start = {}, 0
+    for name in _OWN:
+        at[name] = start
+        start += size[name]
+    total = start
+    for half in _HALVES:
+        end = start
+        for slot in half:
+            at.update((name, end) for name in slot)
+            end += max(size[name] for name in slot)
+        total = max(total, end)
+    return at, total
+
+
 class PrefillPlan:
-    def __init__(self, cfg: TransformerConfig, seq_len: int, layout: Optional[ParallelLayout] = None):
+    """The launches of one layer for ``seq_len`` tokens, and their scratch. ``weights``: "bf16", "q4" or "q8", as the projections are
+    stored; with ``kv_quant`` ("q8") the pages of ``context`` tokens (the portion's own if that is more) are expanded beside them."""
+
+    def __init__(self, cfg: TransformerConfig, seq_len: int, layout: Optional[ParallelLayout] = None, weights: str = "bf16",
+                 kv_quant: Optional[str] = None, context: int = 0):
         layout = layout or ParallelLayout()
         hq, _, hkv, _ = layout.heads(cfg)
         d, hd, t = cfg.hidden_size, cfg.head_dim, seq_len
@@ -62,15 +96,37 @@ class PrefillPlan:
                 PlanStep("down", "gemm+residual", t, d, inter, t * d * 2),
             ]
         self.steps: Tuple[PlanStep, ...] = tuple(steps)
+        # one block holds it all (models/prefill.py: PromptRun); tensor parallelism and shared experts allocate launch by launch
+        moe = cfg.ff_type.moe if cfg.ff_type.kind == "moe" else None
+        self.at_once = layout.world == 1 and not (moe is not None and moe.num_shared_experts)
+
+        def expands(k: int) -> bool:       # products of more than a few rows: 8-bit weights, and 4-bit ones outside the kernels' groups
+            return weights == "q8" or (weights == "q4" and k % 512 != 0)
+
+        pages = -(-max(t, context) // 16) * hkv * 16 * hd * 2 if kv_quant else 0
+        p = self.pieces = dict(h0=t * d * 2, h1=t * d * 2, xn=t * d * 2, qkv=t * (hq + 2 * hkv) * hd * 2, q=t * hq * hd * 2,
+                               attn=t * hq * hd * 2, kk=pages, vv=pages, act=0, mid=0)
+        linear = [((hq + 2 * hkv) * hd, d), (d, hq * hd)]
+        dense = [inter] if moe is None else \
+            [cfg.dense_intermediate_dim // layout.world] if cfg.first_dense_layers and cfg.dense_intermediate_dim else []
+        for i in dense:
+            linear += [(2 * i, d), (d, i)]
+            p["act"] = t * i * 2
+            p["mid"] = t * 2 * i * 2 if expands(d) or 2 * i % 256 else 0
+        p["dense"] = max([n * k * 2 for n, k in linear if expands(k)], default=0)
+        if moe is not None:
+            pairs, e = t * moe.num_experts_per_token, moe.num_experts
+            p["act"] = max(p["act"], pairs * inter * 2)
+            p.update(logits=t * e * 4, idx=pairs * 4, wts=pairs * 4, counts=e * 4, offsets=(e + 1) * 4, order=pairs * 4, cursors=e * 4,
+                     row_of=pairs * 4, xs=pairs * d * 2)
+            # few pairs of quantised experts are added up in fp32, without sorted rows
+            p["y"] = pairs * d * (4 if weights != "bf16" and pairs <= 16 * e else 2)
 
     @property
     def scratch_bytes(self) -> int:
-        """Peak of (a step's output + its input, i.e. the previous step's output)."""
-        peak, prev = 0, 0
-        for s in self.steps:
-            peak = max(peak, prev + s.out_bytes)
-            prev = s.out_bytes
-        return peak
+        """Bytes beside weights and cache: the block of the native call; launch by launch, all intermediates of a layer (each lives until
+        its name is used again)."""
+        return prompt_block(self.pieces)[1] if self.at_once else sum(self.pieces.values())
 
     @property
     def flops(self) -> float:

@@ -105,3 +105,23 @@ def test_host_ids_raise(dev):
     with pytest.raises(_lib.NativeError):
         native(ids, cache, 0)
     assert torch.isfinite(native(ids.to(dev), cache, 0)).all()
+
+
+@pytest.mark.parametrize("experts", [0, 16])
+@pytest.mark.parametrize("quant", ["q4", "q8", None])
+@pytest.mark.parametrize("kv", [None, "q8"])
+def test_block_is_what_the_plan_counts(dev, experts, quant, kv):
+    """The block that a portion allocates is never more than the static plan says, and a long portion's is the plan's to the byte."""
+    from rmlx_b200.models.prefill import NativePrefill
+    from rmlx_b200.models.prefill_plan import PrefillPlan
+    model = _model(dev, experts, quant)
+    native, cache = NativePrefill(model), model.new_cache(80, max_seqs=1, kv_quant=kv)
+    cache.add_sequence(0)
+    for t in (1, 7, 40, 100, 700):
+        at = cache.seq_len(0)
+        cache.reserve(0, t)
+        h = native.at_once.run(torch.zeros(t, dtype=torch.int32, device=dev), cache, 0, at)
+        cache.commit(0, t)
+        plan = PrefillPlan(model.cfg, t, weights=quant or "bf16", kv_quant=kv, context=at + t).scratch_bytes
+        assert h.untyped_storage().nbytes() <= plan
+    assert h.untyped_storage().nbytes() == plan
