@@ -202,10 +202,12 @@ class PromptRun:
     def __init__(self, model):
         self.m = model
         self._numbers: list = []            # int32 0, 1, 2, ... and zeros on the device; grown ones are kept beside their successors
+        if model.layout.world == 1 and model.device.type == "cuda":
+            self._tables(model.cfg.max_seq_len + 1)     # here, not in the first portion that needs them
 
     def _tables(self, n: int):
         if not self._numbers or self._numbers[-1][0].numel() < n:
-            size = max(n, 2 * self._numbers[-1][0].numel() if self._numbers else 8192)
+            size = max(n, 2 * self._numbers[-1][0].numel() if self._numbers else 0)
             dev = self.m.device
             pair = (torch.arange(size, dtype=torch.int32, device=dev), torch.zeros(size, dtype=torch.int32, device=dev))
             torch.cuda.current_stream(dev).synchronize()    # from here on any stream may read them

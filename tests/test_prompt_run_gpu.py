@@ -125,3 +125,17 @@ def test_block_is_what_the_plan_counts(dev, experts, quant, kv):
         plan = PrefillPlan(model.cfg, t, weights=quant or "bf16", kv_quant=kv, context=at + t).scratch_bytes
         assert h.untyped_storage().nbytes() <= plan
     assert h.untyped_storage().nbytes() == plan
+
+
+def test_tables_of_numbers_come_with_the_path(dev):
+    """They are there for every position of the model when the path is attached; no portion within its length makes new ones."""
+    from rmlx_b200.models.prefill import NativePrefill
+    model = _model(dev, 0, "q4")
+    native, cache = NativePrefill(model), model.new_cache(130, max_seqs=1)
+    cache.add_sequence(0)
+    made = list(native.at_once._numbers)
+    assert len(made) == 1 and made[0][0].numel() == model.cfg.max_seq_len + 1
+    for t in (1, model.cfg.max_seq_len - 1):
+        native(torch.zeros(t, dtype=torch.int32, device=dev), cache, 0)
+    assert len(native.at_once._numbers) == 1 and native.at_once._numbers[0] is made[0]
+    assert torch.equal(made[0][0], torch.arange(model.cfg.max_seq_len + 1, dtype=torch.int32, device=dev)) and not made[0][1].any()
