@@ -635,13 +635,17 @@ RB_BOUNDS_REGISTER("flash_decode_cluster.cu")
 
 // Plan for `tiles` (= batch x kv heads x head tiles) tiles of at most `max_len` tokens, (cluster size << 16) | clusters: the size whose rounds
 // of clusters, over the blocks that share a tile, are fewest; the smaller one of equals (a round costs a merge). 0: not a shape of this kernel.
+// One block per tile from one tile per SM on, where clusters only add rounds (us, clusters of 1 / 2 blocks: 148 tiles of 16 heads 9.5 / 13 at 400
+// tokens, 30 / 31 at 2000; 384 tiles of 4 heads 19 / 26 at 400), and where a tile has less than a page for each of sixteen warps (4 tiles of 16
+// heads 6.4 / 8.9 at 150 tokens).
 extern "C" int rmlx_flash_decode_cluster_plan(int batch, int tiles, int max_len, int HD, int kv_quant) {
   if (tiles < 1 || batch < 1 || batch > kFcMaxBatch || (HD != 64 && HD != 128)) return 0;
   const int pages = (max_len + kFcPage - 1) / kFcPage;
   if ((long long)pages * tiles > (1ll << 30)) return 0;
+  const int largest = tiles >= sm_count() || pages < 4 * kFcWarps ? 1 : kFcMaxCluster;
   int best = 0;
   double best_cost = 1e30;
-  for (int cs = 1; cs <= kFcMaxCluster; cs *= 2) {
+  for (int cs = 1; cs <= largest; cs *= 2) {
     if (cs > 1 && pages < cs * kFcWarps / 2) break;      // warps without a page
     const int n = HD == 128 ? (kv_quant ? fc_resident<128, true>(cs) : fc_resident<128, false>(cs))
                             : (kv_quant ? fc_resident<64, true>(cs) : fc_resident<64, false>(cs));

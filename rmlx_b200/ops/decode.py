@@ -420,13 +420,39 @@ _lib.register_cuda_sigs({
 _FD_CLUSTER = os.environ.get("RMLX_FLASH_DECODE_CLUSTER", "1") != "0"
 
 
+def cluster_plan(batch: int, hq: int, hkv: int, head_dim: int, max_len: int, q8: bool) -> int:
+    """(cluster size << 16) | clusters of csrc/kernels/flash_decode_cluster.cu for up to ``max_len`` tokens; 0: not a shape of it."""
+    lib = _lib.cuda()
+    tiles = batch * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv)
+    plan = int(lib.rmlx_flash_decode_cluster_plan(batch, tiles, int(max_len), head_dim, int(q8)))
+    # Sixteen blocks merge a tile's heads into so many parts that with more than eight heads, and more than four tiles, it takes what it
+    # gives: 64 and 4 heads, two sequences, us for 8 / 16 blocks: 7.0 / 9.8 at 17 tokens, 6.8 / 8.3 at 400, 9.1 / 9.5 at 2000, 16.8 / 14.3 at 8000
+    if plan >> 16 > 8 and tiles > 4 and hq > 8 * hkv and not q8:
+        plan = 8 << 16 | tiles
+    return plan
+
+
+def clusters_pay(tiles: int, head_dim: int, max_len: int, q8: bool, sms: int = 148) -> bool:
+    """Whether a cluster per tile is faster than splits of every sequence (csrc/kernels/flash_decode.cu). Up to two tiles per SM, always.
+    Above, blocks take runs of whole tiles: the pages of an 8-bit cache are read in half the time all the same (time against the splits',
+    300 to 2400 tiles of 128: 0.95 to 0.7 at 17 tokens, 0.6 at 2000), those of a bf16 one only if the second round is nearly full (384 tiles 1.28 at
+    400 tokens, 1.18 at 2000; 448 0.95 and 0.97 with 4 heads a tile, 1.02 and 1.10 with 16; 512 0.91 and 0.88) or sequences are short (600 to 2400 tiles 0.8 at 17, 0.95 at 400, 1.07 at 2000).
+    Tiles of 64 are too small for it (1.1 to 1.5; 8-bit 1.2 to 0.9 from 17 to 2000 tokens)."""
+    room = 2 * sms
+    if tiles <= room:
+        return True
+    if head_dim == 64:
+        return False
+    return q8 or (5 * tiles >= 8 * room if tiles <= 2 * room else max_len <= 1024)
+
+
 class FlashDecodeScratch:
     """Split-KV scratch: partial outputs, (max, sum) pairs and the per-tile ticket counters.
 
     With ``max_len`` given, the scratch also plans the cluster kernel (flash_decode_cluster.cu: a
-    thread-block cluster per tile, merging through distributed shared memory), which takes over unless
-    ``RMLX_FLASH_DECODE_CLUSTER=0``; ``clusters`` and, for the 8-bit cache, ``clusters_q8`` are its
-    plans ((cluster size << 16) | clusters; 0: not a shape of it)."""
+    thread-block cluster per tile, merging through distributed shared memory), which takes over where
+    ``clusters_pay`` unless ``RMLX_FLASH_DECODE_CLUSTER=0``; ``clusters`` and, for the 8-bit cache, ``clusters_q8`` are its
+    plans (``cluster_plan``)."""
 
     def __init__(self, batch: int, hq: int, hkv: int, head_dim: int, splits: int, device,
                  max_len: Optional[int] = None):
@@ -438,12 +464,11 @@ class FlashDecodeScratch:
                                    dtype=torch.float32, device=device)
         self.tickets = torch.zeros(lib.rmlx_flash_decode_ticket_elems(batch, hq, hkv),
                                    dtype=torch.int32, device=device)
-        self.tiles = batch * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv)
+        self.tiles, self.max_len = batch * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv), max_len
         self.clusters = self.clusters_q8 = 0
         if max_len is not None and _FD_CLUSTER:
             with torch.cuda.device(device):
-                self.clusters, self.clusters_q8 = (int(lib.rmlx_flash_decode_cluster_plan(batch, self.tiles, int(max_len), head_dim, q8))
-                                                   for q8 in (0, 1))
+                self.clusters, self.clusters_q8 = (cluster_plan(batch, hq, hkv, head_dim, max_len, q8) for q8 in (False, True))
 
 
 def default_splits(batch: int, hkv: int, gtiles: int, max_len: int, sm_count: int = 148) -> int:
@@ -484,7 +509,8 @@ def flash_decode_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
     if k_sb is not None:
         assert k_cache.dtype == torch.uint8 and v_sb is not None and k_sb.dtype == torch.bfloat16
     plan = 0 if scratch is None or splits != scratch.splits else scratch.clusters if k_sb is None else scratch.clusters_q8
-    if plan and b * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv) <= scratch.tiles:
+    tiles = b * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv)
+    if plan and tiles <= scratch.tiles and clusters_pay(tiles, d, scratch.max_len, k_sb is not None):
         rc = lib.rmlx_flash_decode_cluster(
             q.data_ptr(), k_cache.data_ptr(), _lib.ptr(k_sb), v_cache.data_ptr(), _lib.ptr(v_sb), block_table.data_ptr(),
             seq_lens.data_ptr(), out.data_ptr(), b, hq, hkv, d, block_table.shape[1], block_table.stride(0), plan, window, scale,

@@ -102,3 +102,32 @@ def test_settled_cache(dev, q8):
             got.append(D.flash_decode_paged(q, k, v, table, sl, None, None, sc, pdl=pdl, settled=pdl, **sb))
         outs.append(torch.stack(got))
     assert torch.equal(outs[0], outs[1])
+
+
+def test_cluster_sizes(dev):
+    """One block per tile from one tile per SM on and for few pages; several where few tiles have many."""
+    from rmlx_b200.ops import decode as D
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    for batch, hq, hkv, max_len, q8, one in [(sms // 4, 64, 4, 8192, False, True), (sms, 8, 1, 8192, True, True), (48, 32, 8, 8192, False, True),
+                                             (1, 64, 4, 255, False, False), (1, 64, 4, 240, False, True), (2, 64, 4, 100, True, True),
+                                             (1, 64, 4, 8192, False, False), (16, 32, 8, 8192, True, False)]:
+        assert (D.cluster_plan(batch, hq, hkv, 128, max_len, q8) >> 16 == 1) is one
+
+
+@pytest.mark.parametrize("hkv,lens", [(8, [37] * 90 + [1500]), (4, [15 + 61 * (i % 7) for i in range(150)])])
+def test_runs_of_tiles_bf16(dev, hkv, lens):
+    """More tiles than clusters in a bf16 cache, lengths far apart, whichever kernel the rule prefers there."""
+    from rmlx_b200.ops import decode as D
+    g = torch.Generator(device=dev).manual_seed(5)
+    (k, v, _, _), vals, table, sl = _cache(dev, g, lens, hkv, 128, False)
+    q = torch.randn(len(lens), 4 * hkv, 128, device=dev, generator=g).to(torch.bfloat16)
+    want = _want(q, vals, table, lens, 0)
+    sc = D.FlashDecodeScratch(len(lens), 4 * hkv, hkv, 128, 1, dev, max_len=max(lens))
+    real, got = D.clusters_pay, []
+    for use in (True, False):
+        D.clusters_pay = lambda *a: use
+        try:
+            got.append(D.flash_decode_paged(q, k, v, table, sl, scratch=sc))
+        finally:
+            D.clusters_pay = real
+        assert float((got[-1].double() - want).norm() / want.norm()) < 3e-3

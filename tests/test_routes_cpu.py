@@ -1,0 +1,29 @@
+"""Which kernel a call goes to where several take it (host arithmetic): points on both sides of the lines, at sizes that were timed on both
+kernels."""
+import pytest
+import torch
+
+from rmlx_b200.ops import decode as D
+
+
+@pytest.mark.parametrize("tiles,hd,max_len,q8,pays", [
+    (1, 128, 8192, False, True), (148, 128, 8192, False, True), (296, 64, 8192, False, True),
+    (297, 128, 8192, False, False), (384, 128, 8192, False, False), (384, 128, 512, False, False), (448, 128, 8192, False, False),
+    (512, 128, 8192, False, True), (592, 128, 8192, False, True), (640, 128, 8192, False, False), (640, 128, 1024, False, True),
+    (1184, 128, 8192, False, False), (384, 128, 8192, True, True), (2400, 128, 8192, True, True), (384, 64, 8192, False, False),
+    (512, 64, 1024, True, False)])
+def test_decode_attention_tiles(tiles, hd, max_len, q8, pays):
+    assert D.clusters_pay(tiles, hd, max_len, q8) is pays
+
+
+def test_sixteen_blocks_merge_few_heads(monkeypatch):
+    """Tiles of more than eight heads take clusters of up to eight blocks once there are more than four of them."""
+    class _Plans:
+        rmlx_flash_decode_gtiles = staticmethod(lambda hq, hkv: -(-hq // hkv // 16))
+        rmlx_flash_decode_cluster_plan = staticmethod(lambda batch, tiles, max_len, hd, q8: 16 << 16 | tiles)
+
+    monkeypatch.setattr(D._lib, "cuda", _Plans)
+    assert D.cluster_plan(1, 64, 4, 128, 8192, False) == 16 << 16 | 4
+    assert D.cluster_plan(2, 64, 4, 128, 8192, False) == 8 << 16 | 8
+    assert D.cluster_plan(2, 64, 4, 128, 8192, True) == 16 << 16 | 8
+    assert D.cluster_plan(2, 32, 4, 128, 8192, False) == 16 << 16 | 8
