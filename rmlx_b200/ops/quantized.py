@@ -85,12 +85,15 @@ def row_pays(m: int, n: int, k: int, experts: int = 0) -> bool:
     """Whether 4-bit weights go to the kernel whose 128 product rows are rows of W and whose columns are the rows of x that there are
     (csrc/kernels/row_gemm.cu), rather than to tiles of 128 or 256 rows of x.
 
-    Measured (us, this kernel / the tiles). 128 experts of 4096 x 1536, gate and up + down: 298 + 159 / 552 + 321 at 512 rows in all, 324 +
-    167 / 429 + 242 at 2048, 336 + 186 / 439 + 250 at 8192, 404 + 264 / 637 + 415 at 16384, 750 + 482 / 872 + 644 at 24000, 913 + 544 / 889 +
-    735 at 32768. One weight: 9216 x 4096 20 / 27 at 24 rows, 24 / 27 at 64, 28 / 27 at 96; 28672 x 4096 40 / 47 at 24, 45 / 48 at 96; 4096 x
-    8192 22 / 47 at 64, 26 / 47 at 96; 4096 x 14336 28 / 75 at 64; 151936 x 4096 140 / 172 at 64; 512 rows of 9216 x 4096 44 / 34; 1024 x 256
-    at 16 rows 10 / 9."""
-    return m <= 256 * experts if experts else m <= (96 if n <= 8192 or n > 16384 else 80) and n * k >= 1 << 23
+    Experts (time of both projections against the tiles', rows of x per expert): 128 of 4096 x 1536 0.6 to 0.7 from 9 to 64 rows, 0.87 at 96,
+    0.69 at 128, 0.88 at 176; 32 of 2048 x 2048 0.6, 0.87, 1.01, 0.82, 0.97; 64 of 2048 x 1024 0.6, 0.87, 1.0, 0.85, 1.04. From 192 rows on, where
+    a pair of SMs takes the tiles (whole ones of 256 columns), 1.25, 1.39, 1.48. Where all experts together have less than one tile of 128 rows of W per SM twice over,
+    blocks stand idle: 16 of 1024 x 512 0.94 at 32 rows and 1.4 at 160, 8 of 512 x 512 0.99 and 1.1.
+    One weight, up to 96 rows, 4096 x 4096 20 / 25, 12288 x 4096 25 / 46, 4096 x 8192 22 / 47, 4096 x 14336 28 / 75, 512 rows of 9216 x 4096 44 / 34;
+    1024 x 256 at 16 rows 10 / 9."""
+    if experts:
+        return (m < 192 * experts or (n % 256 != 0 and m <= 256 * experts)) and (m <= 32 * experts or experts * n >= 1 << 15)
+    return m <= (96 if n <= 8192 or n > 16384 else 80) and n * k >= 1 << 23
 
 
 def row_supported(x: torch.Tensor, w: LinearWeight, out: torch.Tensor, residual: Optional[torch.Tensor] = None,
