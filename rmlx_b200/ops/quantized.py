@@ -89,11 +89,28 @@ def row_pays(m: int, n: int, k: int, experts: int = 0) -> bool:
     0.69 at 128, 0.88 at 176; 32 of 2048 x 2048 0.6, 0.87, 1.01, 0.82, 0.97; 64 of 2048 x 1024 0.6, 0.87, 1.0, 0.85, 1.04. From 192 rows on, where
     a pair of SMs takes the tiles (whole ones of 256 columns), 1.25, 1.39, 1.48. Where all experts together have less than one tile of 128 rows of W per SM twice over,
     blocks stand idle: 16 of 1024 x 512 0.94 at 32 rows and 1.4 at 160, 8 of 512 x 512 0.99 and 1.1.
-    One weight, up to 96 rows, 4096 x 4096 20 / 25, 12288 x 4096 25 / 46, 4096 x 8192 22 / 47, 4096 x 14336 28 / 75, 512 rows of 9216 x 4096 44 / 34;
-    1024 x 256 at 16 rows 10 / 9."""
+    One weight (us, this kernel / the tiles, at 33, 64 and 96 rows). Up to 9472 rows of W the tiles of x's rows are one round of the SMs and their
+    time is K's, while this kernel shares K between blocks at a cost that grows with the rows: 8192 x 2048 16 / 15, 19 / 15, 22 / 15; 8192 x 3072 18 /
+    20, 21 / 20, 25 / 20; 8192 x 4096 20 / 25, 23 / 25, 27 / 25; 8192 x 5120 22 / 30, 25 / 30, 29 / 30; half as wide it has twice the blocks: 4096 x 2048
+    13 / 14, 14 / 14, 16 / 14, 4096 x 3072 15 / 19, 16 / 19, 19 / 20. Then the tiles take two rounds: 9728 x 1024 11 / 15, 11 / 14, 13 / 14; 12288 x
+    4096 23 / 45, 24 / 45, 25 / 46. From 14336 on they are twice as wide: 16384 x 1024 12 / 13, 13 / 12, 14 / 12; x 1536 14 / 17, 14 / 15, 16 / 15; x
+    2048 16 / 18, 16 / 18, 18 / 18; and from 28672 on both read at the memory's rate, or for small K write at it: 32768 x 1024 16 / 16, 17 / 16, 20 /
+    16; x 2048 24 / 23, 25 / 24, 26 / 24; x 3072 32 / 32, 32 / 32, 34 / 33; x 4096 39 / 40, 40 / 41, 42 / 42; 65536 x 4096 69 / 74, 71 / 75, 73 / 77."""
     if experts:
         return (m < 192 * experts or (n % 256 != 0 and m <= 256 * experts)) and (m <= 32 * experts or experts * n >= 1 << 15)
-    return m <= (96 if n <= 8192 or n > 16384 else 80) and n * k >= 1 << 23
+    if n * k < 1 << 23:
+        return False
+    if n <= 4096:
+        most = 72 if k < 3072 else 96
+    elif n <= 9472:
+        most = 3 * k // 128 - 24
+    elif n < 14336:
+        most = 96
+    elif n <= 24576:
+        most = 0 if k < 1024 else 32 if k < 1536 else 64 if k < 2048 else 96
+    else:
+        most = 0 if k < 1024 else 32 if k < 2560 else 64 if k < 4096 else 96
+    return m <= min(most, 96)
 
 
 def row_supported(x: torch.Tensor, w: LinearWeight, out: torch.Tensor, residual: Optional[torch.Tensor] = None,

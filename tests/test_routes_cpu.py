@@ -36,3 +36,12 @@ def test_sixteen_blocks_merge_few_heads(monkeypatch):
 def test_experts_in_4_bits(rows, experts, n, k, row):
     """``rows`` of x for each expert: on tiles of W's rows, or of x's."""
     assert Q.row_pays(rows * experts, n, k, experts) is row
+
+
+@pytest.mark.parametrize("n,k,most", [
+    (4096, 2048, 72), (3072, 4096, 96), (8192, 1024, 0), (8192, 2048, 24), (6144, 2560, 36), (9472, 3072, 48), (8192, 4096, 72), (6144, 5120, 96),
+    (8192, 14336, 96), (9600, 1024, 96), (12288, 4096, 96), (14336, 1024, 32), (16384, 1536, 64), (16384, 2048, 96), (24576, 512, 0),
+    (32768, 512, 0), (32768, 1024, 32), (28672, 3072, 64), (28672, 4096, 96), (151936, 4096, 96), (2048, 2048, 0)])
+def test_rows_of_4_bit_weights(n, k, most):
+    """Up to ``most`` rows on tiles of W's rows."""
+    assert [m for m in range(1, 160) if Q.row_pays(m, n, k)] == list(range(1, most + 1))
