@@ -38,10 +38,13 @@ def supported(w: LinearWeight) -> bool:
 def pays(w: LinearWeight, rows: int) -> bool:
     """Whether a plain projection of ``rows`` rows is faster here than on the 128-row tensor-core tiles (and takes this weight).
 
-    Measured (us, this kernel / the tiles). 4-bit: 28672 x 4096 25 / 39 at 16 rows, 43 / 39 at 24; 28672 x 8192 44 / 72 at 16, 75 / 72
-    at 24; 9216 x 4096 15 / 26 at 16, 20 / 26 at 32, 31 / 26 at 48; 4096 x 8192 20 / 45 at 32; 4096 x 14336 37 / 74: up to 16 rows, and up to
-    32 for moderate widths (from there 9216 x 4096 takes 22 us on the tensor-core tiles of W's rows, 4096 x 14336 25). 8-bit weights would be expanded first (16384 x 2048 at 64 rows 33 / 50, 28672 x 4096 99 / 165, 3072 x
-    2048 17 / 17). bf16, 9216 x 4096: 20 / 28 at 16 rows; 28672 x 4096: 46 / 45:
+    Measured (us, this kernel / the tiles of 128 rows of x). 4-bit: 28672 x 4096 25 / 39 at 16 rows, 43 / 39 at 24; 28672 x 8192 44 / 72 at 16, 75 /
+    72 at 24; 9216 x 4096 15 / 26 at 16; 4096 x 8192 20 / 45 at 32; 4096 x 14336 37 / 74: up to 16 rows, and up to 32 for moderate widths, except
+    where the tiles are one round of the SMs and K is short: at 17 to 24 rows 8192 x 512 9 / 8, 8192 x 1024 12 / 11, 6144 x 1024 7 / 10, 8192 x 2048
+    15 / 19; at 32 rows, two passes of two tiles, 6144 x 512 11 / 7, 8192 x 2048 19 / 15, 8192 x 2560 23 / 18, 8192 x 4096 25 / 25; 12288 wide
+    512 12 / 10, 1024 14 / 16. 8-bit weights would be expanded first: up to 32 rows; above, short small ones take longer here (at 64 rows 2048 x
+    1024 14 / 9, 2048 x 3072 21 / 19, 4096 x 2048 20 / 19, 4096 x 2560 25 / 22, 8192 x 512 13 / 12; 16384 x 2048 33 / 50, 28672 x 4096
+    99 / 165). bf16, 9216 x 4096: 20 / 28 at 16 rows; 28672 x 4096: 46 / 45:
     eight rows, and 16 for up to 16384 rows of W; large weights stream at the copy bandwidth on the tiles too (at 5 rows
     28672 x 8192 89 / 119, 65536 x 4096 101 / 103, 151936 x 4096 227 / 214; at 8 rows 32768 x 4096 53 / 72, 28672 x 8192 89 / 84,
     65536 x 4096 101 / 100). Weights of less than a million entries take a tile's time anyway."""
@@ -52,9 +55,10 @@ def pays(w: LinearWeight, rows: int) -> bool:
     if w.kind == W_BF16:
         ok = (rows <= 8 and entries <= (1 << 27 if rows > 5 else 1 << 28)) or (rows <= 16 and n <= 16384)
     elif w.kind == W_Q4:
-        ok = rows <= 16 or (rows <= 32 and n <= 12288)
+        ok = rows <= 16 or (rows <= 32 and n <= 12288 and (
+            n <= 4096 or (rows <= 24 and (n <= 6144 or n > 9472 or k >= 1536)) or k >= (1024 if n > 9472 else 3072)))
     else:
-        ok = True
+        ok = rows <= 32 or k >= 4096 or entries >= 12 << 20 or (n >= 6144 and k >= 1024)
     return ok and supported(w)
 
 

@@ -3,7 +3,20 @@ kernels."""
 import pytest
 import torch
 
-from rmlx_b200.ops import decode as D, quantized as Q
+from rmlx_b200.ops import decode as D, narrow, quantized as Q
+from rmlx_b200.ops.weights import W_BF16, W_Q4, W_Q8
+
+
+class _Weight:
+    """A weight's kind and sizes; every table contiguous and at a 16-byte address."""
+
+    def __init__(self, kind, n, k, experts=0):
+        self.kind, self.n, self.k, self.experts = kind, n, k, experts
+
+
+@pytest.fixture
+def aligned(monkeypatch):
+    monkeypatch.setattr(narrow, "supported", lambda w: True)
 
 
 @pytest.mark.parametrize("tiles,hd,max_len,q8,pays", [
@@ -45,3 +58,14 @@ def test_experts_in_4_bits(rows, experts, n, k, row):
 def test_rows_of_4_bit_weights(n, k, most):
     """Up to ``most`` rows on tiles of W's rows."""
     assert [m for m in range(1, 160) if Q.row_pays(m, n, k)] == list(range(1, most + 1))
+
+
+@pytest.mark.parametrize("kind,n,k,rows", [
+    (W_Q4, 28672, 4096, (16,)), (W_Q4, 4096, 512, (16, 32)), (W_Q4, 6144, 1024, (16, 24)), (W_Q4, 8192, 1024, (16,)), (W_Q4, 8192, 2048, (16, 24)),
+    (W_Q4, 8192, 3072, (16, 24, 32)), (W_Q4, 12288, 512, (16, 24)), (W_Q4, 12288, 1024, (16, 24, 32)), (W_Q4, 16384, 2048, (16,)),
+    (W_Q8, 2048, 1024, (16, 24, 32)), (W_Q8, 4096, 2560, (16, 32)), (W_Q8, 4096, 3072, (32, 64)), (W_Q8, 2048, 4096, (32, 64)),
+    (W_Q8, 8192, 512, (32,)), (W_Q8, 8192, 1024, (33, 64)), (W_Q8, 28672, 4096, (64,))])
+def test_rows_on_the_weight_streaming_kernel(aligned, kind, n, k, rows):
+    """Rows of 16, 17, 24, 25, 32, 33 and 64 that go there: all up to the largest of ``rows``."""
+    w = _Weight(kind, n, k)
+    assert [m for m in (1, 16, 17, 24, 25, 32, 33, 64, 65) if narrow.pays(w, m)] == [m for m in (1, 16, 17, 24, 25, 32, 33, 64) if m <= max(rows)]
