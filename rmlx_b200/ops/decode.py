@@ -118,9 +118,12 @@ def _several(b: int, w: LinearWeight, x: torch.Tensor, norm_w: Optional[torch.Te
         # one row of a wide 4- or 8-bit weight (us, weight-streaming / per-row, 8-bit: streaming). 4-bit: 151936 x 4096 66 / 78, 28672 x 4096
         # 17 / 21, 32768 x 2048 11 / 15, 16384 x 2048 8.8 / 10.6, but 9 / 8 with SwiGLU; 9216 x 4096 9.0 / 9.2, 6144 x 4096 8.1 / 7.9. 8-bit:
         # 151936 x 4096 107 / 139, 32768 x 2048 14 / 18, 16384 x 2048 9.5 / 11.5 (SwiGLU 9.5 / 11.7), 2048 x 8192 9.1 / 8.1.
-        # Narrower ones from 2^26 entries on: 8192 x 8192 12.7 / 14.6, 10240 x 8192 14.3 / 19.6, 4096 x 28672 20 / 22; 4096 x 16384 13.6 / 13.3,
-        # in 8 bits 16.8 / 21.1
-        if w.kind == W_BF16 or (w.n * w.k < 1 << 26 and (swiglu or w.n < 16384 or w.n * w.k < 1 << 25)):
+        # Narrower ones from 2^26 entries on: 8192 x 8192 12.7 / 14.6, 10240 x 8192 14.3 / 19.6, 3584 x 20480 15.5 / 16.4, 4096 x 28672 20 / 22; in 8
+        # bits 4096 x 16384 16.8 / 21.1. But not in 4 bits where the per-row kernel's blocks of 32 rows are one round of nearly all SMs, unless K is
+        # long: 4096 x 17408 16.9 / 14.8, x 20480 17.1 / 16.6, x 24576 18.9 / 19.4; 4608 x 20480 18.0 / 16.9, x 24576 21.4 / 20.4; and not beyond
+        # the K that the even split takes (4096 x 36864 67 / 29)
+        if w.kind == W_BF16 or w.k > 32768 or (w.n * w.k < 1 << 26 and (swiglu or w.n < 16384 or w.n * w.k < 1 << 25)) or \
+                (w.kind == W_Q4 and 3584 < w.n <= 4736 and w.k < 6 * w.n - 1024):
             return False
     # two rows of 4-bit weights: a 16384 x 2048 projection 9 us against 11, a 3072 x 2048 one 6 against 5
     least = 0 if b >= 4 else 1 << 24 if b == 2 and w.kind == W_Q4 else 1 << 20

@@ -69,3 +69,14 @@ def test_rows_on_the_weight_streaming_kernel(aligned, kind, n, k, rows):
     """Rows of 16, 17, 24, 25, 32, 33 and 64 that go there: all up to the largest of ``rows``."""
     w = _Weight(kind, n, k)
     assert [m for m in (1, 16, 17, 24, 25, 32, 33, 64, 65) if narrow.pays(w, m)] == [m for m in (1, 16, 17, 24, 25, 32, 33, 64) if m <= max(rows)]
+
+
+@pytest.mark.parametrize("kind,n,k,streams", [
+    (W_Q4, 16384, 2048, True), (W_Q4, 16384, 1024, False), (W_Q4, 8192, 8192, True), (W_Q4, 3584, 20480, True), (W_Q4, 3840, 18432, False),
+    (W_Q4, 4096, 16384, False), (W_Q4, 4096, 20480, False), (W_Q4, 4096, 24576, True), (W_Q4, 4608, 24576, False), (W_Q4, 4608, 28672, True),
+    (W_Q4, 5120, 16384, True), (W_Q8, 4096, 16384, True), (W_Q4, 2048, 32768, True), (W_Q4, 2048, 36864, False), (W_Q8, 4096, 36864, False)])
+def test_one_row(aligned, kind, n, k, streams):
+    """One row of a large quantised weight: the even split, or a block per 32 rows of W."""
+    x = torch.zeros(1, 8, dtype=torch.bfloat16)
+    assert D._several(1, _Weight(kind, n, k), x) is streams
+    assert D._several(2, _Weight(kind, n, k), x) is True
