@@ -87,8 +87,9 @@ def row_pays(m: int, n: int, k: int, experts: int = 0) -> bool:
 
     Experts (time of both projections against the tiles', rows of x per expert): 128 of 4096 x 1536 0.6 to 0.7 from 9 to 64 rows, 0.87 at 96,
     0.69 at 128, 0.88 at 176; 32 of 2048 x 2048 0.6, 0.87, 1.01, 0.82, 0.97; 64 of 2048 x 1024 0.6, 0.87, 1.0, 0.85, 1.04. From 192 rows on, where
-    a pair of SMs takes the tiles (whole ones of 256 columns), 1.25, 1.39, 1.48. Where all experts together have less than one tile of 128 rows of W per SM twice over,
-    blocks stand idle: 16 of 1024 x 512 0.94 at 32 rows and 1.4 at 160, 8 of 512 x 512 0.99 and 1.1.
+    a pair of SMs takes the tiles (whole ones of 256 columns), 1.25, 1.39, 1.48. Small experts have too few tiles of W to keep all SMs busy: 16 of
+    1024 x 512 0.94 at 32 rows and 1.4 at 160, 16 of 1024 x 1024 1.1 at 96 and 1.16 at 176, 32 of 1024 x 512 1.27 and 1.28; but not those of long K, 8 of
+    4096 x 7168 0.69 and 0.82.
     One weight (us, this kernel / the tiles, at 33, 64 and 96 rows). Up to 9472 rows of W the tiles of x's rows are one round of the SMs and their
     time is K's, while this kernel shares K between blocks at a cost that grows with the rows: 8192 x 2048 16 / 15, 19 / 15, 22 / 15; 8192 x 3072 18 /
     20, 21 / 20, 25 / 20; 8192 x 4096 20 / 25, 23 / 25, 27 / 25; 8192 x 5120 22 / 30, 25 / 30, 29 / 30; half as wide it has twice the blocks: 4096 x 2048
@@ -97,7 +98,7 @@ def row_pays(m: int, n: int, k: int, experts: int = 0) -> bool:
     2048 16 / 18, 16 / 18, 18 / 18; and from 28672 on both read at the memory's rate, or for small K write at it: 32768 x 1024 16 / 16, 17 / 16, 20 /
     16; x 2048 24 / 23, 25 / 24, 26 / 24; x 3072 32 / 32, 32 / 32, 34 / 33; x 4096 39 / 40, 40 / 41, 42 / 42; 65536 x 4096 69 / 74, 71 / 75, 73 / 77."""
     if experts:
-        return (m < 192 * experts or (n % 256 != 0 and m <= 256 * experts)) and (m <= 32 * experts or experts * n >= 1 << 15)
+        return (m < 192 * experts or (n % 256 != 0 and m <= 256 * experts)) and (m <= 32 * experts or experts * n * k >= 1 << 26)
     if n * k < 1 << 23:
         return False
     if n <= 4096:

@@ -45,7 +45,8 @@ def test_sixteen_blocks_merge_few_heads(monkeypatch):
 @pytest.mark.parametrize("rows,experts,n,k,row", [
     (9, 128, 3072, 4096, True), (128, 128, 3072, 4096, True), (191, 128, 3072, 4096, True), (192, 128, 3072, 4096, False),
     (256, 128, 4096, 1536, False), (176, 32, 4096, 2048, True), (224, 64, 2048, 2048, False), (224, 64, 2176, 2048, True), (32, 16, 1024, 1024, True),
-    (33, 16, 1024, 1024, False), (33, 8, 512, 512, False), (33, 16, 2048, 1024, True)])
+    (33, 16, 1024, 1024, False), (33, 8, 512, 512, False), (33, 16, 2048, 1024, False), (33, 32, 1024, 1024, False),
+    (191, 8, 4096, 7168, True), (33, 32, 2048, 1024, True)])
 def test_experts_in_4_bits(rows, experts, n, k, row):
     """``rows`` of x for each expert: on tiles of W's rows, or of x's."""
     assert Q.row_pays(rows * experts, n, k, experts) is row
