@@ -63,11 +63,12 @@ def pays(w: LinearWeight, rows: int) -> bool:
 
 
 def pays_grouped(gate_up: LinearWeight, down: LinearWeight, pairs: int) -> bool:
-    """Whether an expert feed-forward of ``pairs`` (row, slot) pairs is faster here: up to twelve pairs per expert in 4 bits, sixteen in 8
+    """Whether an expert feed-forward of ``pairs`` (row, slot) pairs is faster here: up to twelve pairs per expert in 4 bits, fourteen in 8
     (128 experts of 4096 x 1536, both projections, us, here / on the tiles: 4-bit 382 / 470 at 1024 pairs, 466 / 480 at 1600, 577 / 490 at
-    2048; 8-bit on expanded weights 586 / 815 at 1024, 748 / 894 at 2048). bf16 experts are as fast on the tiles (523 + 275 against 549 + 305
-    at 512 pairs)."""
-    most = 12 if gate_up.kind == W_Q4 else 16
+    2048; 8-bit on expanded weights 586 / 815 at 1024, 748 / 894 at 2048; at 14 and 16 pairs per expert 32 of 2048 x 2048 0.89 and 1.06 of their
+    time, 64 of 2048 x 1024 0.94 and 1.07), eight where the experts are few and small (16 of 1024 x 512 at 10: 4-bit 35 / 33, 8-bit 34 / 27). bf16
+    experts are as fast on the tiles (523 + 275 against 549 + 305 at 512 pairs)."""
+    most = 8 if gate_up.experts * gate_up.n * gate_up.k < 1 << 27 else 12 if gate_up.kind == W_Q4 else 14
     return (gate_up.kind in (W_Q4, W_Q8) and down.kind == gate_up.kind and 0 < pairs <= most * gate_up.experts and
             gate_up.n * gate_up.k >= 1 << 20 and supported(gate_up) and supported(down))
 

@@ -81,3 +81,11 @@ def test_one_row(aligned, kind, n, k, streams):
     x = torch.zeros(1, 8, dtype=torch.bfloat16)
     assert D._several(1, _Weight(kind, n, k), x) is streams
     assert D._several(2, _Weight(kind, n, k), x) is True
+
+
+@pytest.mark.parametrize("kind,experts,n,k,most", [
+    (W_Q4, 128, 3072, 4096, 12), (W_Q8, 128, 3072, 4096, 14), (W_Q8, 32, 4096, 2048, 14), (W_Q4, 64, 2048, 2048, 12), (W_Q4, 16, 1024, 1024, 8),
+    (W_Q8, 16, 1024, 1024, 8), (W_Q8, 32, 2048, 1024, 8), (W_BF16, 128, 3072, 4096, 0)])
+def test_pairs_of_experts_on_the_weight_streaming_kernel(aligned, kind, experts, n, k, most):
+    up, down = _Weight(kind, n, k, experts), _Weight(kind, k, n // 2, experts)
+    assert [p for p in range(1, 20) if narrow.pays_grouped(up, down, p * experts)] == list(range(1, most + 1))
