@@ -15,14 +15,14 @@ def dev():
     return torch.device("cuda")
 
 
-def _model(dev, experts, quant, window=0, hd=128, bias=False):
+def _model(dev, experts, quant, window=0, hd=128, bias=False, expert=(1024, 512), top=2):
     from rmlx_b200.models.transformer import TransformerModel
     from rmlx_b200.models.weights import LayerWeights, ModelWeights, ParallelLayout
     from rmlx_b200.ops.weights import LinearWeight
     g = torch.Generator(device=dev).manual_seed(1)
-    d, inner, vocab = (1024, 512, 2048) if experts else (2048, 4096, 2048)
+    d, inner, vocab = (*expert, 2048) if experts else (2048, 4096, 2048)
     hq, hkv = d // hd, d // hd // 4
-    ff = FeedForwardType.moe_(MoeConfig(experts, 2, d, inner)) if experts else FeedForwardType.gated(inner)
+    ff = FeedForwardType.moe_(MoeConfig(experts, top, d, inner)) if experts else FeedForwardType.gated(inner)
     cfg = TransformerConfig(hidden_size=d, num_heads=hq, num_kv_heads=hkv, head_dim=hd, num_layers=2, vocab_size=vocab, max_seq_len=2048,
                             rope_theta=1e4, ff_type=ff, sliding_window=window, name="prompt-run").validate()
 
@@ -77,6 +77,36 @@ def test_same_as_launch_by_launch(dev, experts, quant, kv, window, hd):
     res = [_prompts(_model(dev, experts, quant, window, hd, bias=hd == 64), lens, kv, at_once) for at_once in (False, True)]
     for a, b in zip(res[0][0] + res[0][1], res[1][0] + res[1][1]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("quant,top,lens", [("q8", 1, [193, 256, 448]), ("q8", 2, [192, 193, 224]), ("q4", 1, [193, 384])])
+def test_few_rows_per_expert_of_a_longer_portion(dev, quant, top, lens):
+    """More rows than the router takes along and few for each expert: norm, logits and selection as launches of their own, then the experts
+    on the weight-streaming kernel."""
+    from rmlx_b200.models.prefill import ROUTER_ROWS
+    from rmlx_b200.ops import narrow
+    res = []
+    for at_once in (False, True):
+        model = _model(dev, 32, quant, expert=(2048, 1024), top=top)
+        up, down = model.w.layers[0].experts_gate_up, model.w.layers[0].experts_down
+        assert max(lens) > ROUTER_ROWS and all(narrow.pays_grouped(up, down, t * top) for t in lens)
+        res.append(_prompts(model, lens, None, at_once))
+    for a, b in zip(res[0][0] + res[0][1], res[1][0] + res[1][1]):
+        assert torch.equal(a, b)
+
+
+def test_router_at_an_odd_address(dev):
+    """A router that no kernel reads raises from the native call as it does launch by launch."""
+    from rmlx_b200 import _lib
+    for at_once in (False, True):
+        model = _model(dev, 16, "q4")
+        r = model.w.layers[1].router
+        odd = torch.empty(r.numel() + 1, dtype=r.dtype, device=dev)[1:].view_as(r)
+        odd.copy_(r)
+        model.w.layers[1].router = odd
+        for n in (5, 300):
+            with pytest.raises(_lib.NativeError):
+                _prompts(model, [n], None, at_once)
 
 
 def test_not_covered(dev):
