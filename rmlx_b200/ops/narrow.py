@@ -191,13 +191,19 @@ def pays_pairs(gate_up: LinearWeight, down: LinearWeight, rows: int, top_k: int)
     outweighs its launches. Measured, chained (us: pairs / ``expert_ffn`` / streaming kernels). 4-bit, 128 experts of 4096 x 1536, 8 of
     them: 37.5 / 51 / 37.2 for one row, 51 / 61 / 60 for two, 79 / 89 / 107 for four; 8 of 4096 x 14336, two of them: 54 / 58 / 69, 93 / 97 /
     122, three rows 124 / 117 / 175; 64 of 2048 x 1536, six of them: 24 / 33 / 20, 32 / 39 / 31, three rows 38 / 42 / 42. 8-bit, 128 of 2048
-    x 1024, 8 of them: 27 / 38 / 23, 35 / 48 / 36, four rows 50 / 61 / 61; 8 of 4096 x 3584, two of them: 30 / 34 / 35."""
+    x 1024, 8 of them: 27 / 38 / 23, 35 / 48 / 36, four rows 50 / 61 / 61; 8 of 4096 x 3584, two of them: 30 / 34 / 35. 32 small pairs
+    in 4 bits stream faster (2048 x 1024 among 64 experts 42 / 46 / 40, among 128 42 / 54 / 40; 30 of them 41 / 45 / 43), and beyond 2^27
+    entries that are read for a second time sharing wins (16 of 8192 x 4096, two of them, four rows 100 / 88 / 135, in 8 bits 145 / 134 / 217;
+    three rows 80 / 78 / 107; one of them, eight rows 99 / 90 / 138)."""
     pairs, e = rows * top_k, gate_up.experts
     if gate_up.kind not in (W_Q4, W_Q8) or down.kind != gate_up.kind or not 0 < pairs <= PAIRS or e < 1:
         return False
-    read = pairs * (gate_up.n * gate_up.k + down.n * down.k) * (0.5625 if gate_up.kind == W_Q4 else 1.0625)
+    entries = gate_up.n * gate_up.k + down.n * down.k
+    read = pairs * entries * (0.5625 if gate_up.kind == W_Q4 else 1.0625)
     distinct = e * (1.0 - (1.0 - min(1.0, top_k / e)) ** rows)
-    return (read >= 90e6 and pairs <= 1.25 * distinct and gate_up.k <= 32768 and down.k <= 32768 and gate_up.n % 32 == 0 and
+    least = 150e6 if gate_up.kind == W_Q4 and pairs > 30 else 90e6
+    return (read >= least and pairs <= 1.25 * distinct and (pairs - distinct) * entries <= 1 << 27 and gate_up.k <= 32768 and
+            down.k <= 32768 and gate_up.n % 32 == 0 and
             gate_up.scales.dtype == down.scales.dtype == torch.bfloat16 and supported(gate_up) and supported(down))
 
 

@@ -89,3 +89,14 @@ def test_one_row(aligned, kind, n, k, streams):
 def test_pairs_of_experts_on_the_weight_streaming_kernel(aligned, kind, experts, n, k, most):
     up, down = _Weight(kind, n, k, experts), _Weight(kind, k, n // 2, experts)
     assert [p for p in range(1, 20) if narrow.pays_grouped(up, down, p * experts)] == list(range(1, most + 1))
+
+
+@pytest.mark.parametrize("kind,experts,d,inner,top,rows", [
+    (W_Q4, 128, 4096, 1536, 8, (2, 3, 4)), (W_Q4, 128, 2048, 1024, 8, ()), (W_Q4, 64, 2048, 1024, 8, ()), (W_Q4, 64, 2048, 1024, 6, (5,)),
+    (W_Q4, 64, 2048, 1536, 6, (3, 4, 5)), (W_Q4, 16, 8192, 4096, 2, (1, 2, 3)), (W_Q4, 16, 8192, 4096, 1, (2, 3, 4, 5, 6, 7)),
+    (W_Q8, 16, 8192, 4096, 2, (1, 2, 3)), (W_Q8, 64, 2048, 1024, 8, (2, 3, 4)), (W_Q8, 64, 5120, 1536, 6, (1, 2, 3, 4, 5))])
+def test_pairs_one_by_one(aligned, kind, experts, d, inner, top, rows):
+    """Rows of a decode step, up to eight, whose pairs are multiplied one by one."""
+    up, down = _Weight(kind, 2 * inner, d, experts), _Weight(kind, d, inner, experts)
+    up.scales = down.scales = torch.zeros(1, dtype=torch.bfloat16)
+    assert tuple(r for r in range(1, 9) if narrow.pays_pairs(up, down, r, top)) == rows
