@@ -97,6 +97,17 @@ def _router_logits(xn: torch.Tensor, router: torch.Tensor) -> torch.Tensor:
 ROUTER_ROWS = 192
 
 
+def _logits_by_rows(w: LinearWeight, rows: int) -> bool:
+    """Whether the logits of several rows come from the kernel whose product rows are the vocabulary's (``row_gemm``, fp32 unrounded), rather
+    than as any projection and then converted.
+
+    Measured (us, there / as a projection), 4-bit: 151936 x 4096 145 / 167 at 64 rows, 190 / 292 at 160; 32000 x 2048 25 / 30, 35 / 46; 50304 x 1024
+    24 / 33, 41 / 49; above, two passes: at 192 rows 32768 x 4096 72 / 69, 128256 x 8192 451 / 429. Small vocabularies, which the tiles
+    hold in one round, and short K up to 64 rows: 8192 x 2048 18 / 19 at 64, 22 / 19 at 96; 2048 x 1024 12.5 / 13.3, 13.7 / 13.5, at 160 17.5 / 13.5;
+    65536 x 512 25 / 27 at 64, 37 / 34 at 112."""
+    return w.kind == W_Q4 and rows <= (160 if w.n >= 16384 and w.k >= 1024 else 64)
+
+
 def _routed_few(h: torch.Tensor, lw, moe) -> bool:
     """Whether few rows go to the experts without a normalised copy of them: the router and the weight-streaming kernel take the norm
     along."""
@@ -175,9 +186,9 @@ class _Layers:
             if w.lm_head.kind == W_BF16 and w.lm_head.k % 8 == 0:
                 from ..ops.gemm import gemm_bf16_f32       # accumulator stored unrounded
                 out = gemm_bf16_f32(xn, w.lm_head.w)
-            elif w.lm_head.kind == W_Q4 and r <= 160 and row_supported(
+            elif _logits_by_rows(w.lm_head, r) and row_supported(
                     xn, w.lm_head, out := torch.empty(r, w.lm_head.n, dtype=torch.float32, device=m.device)):
-                row_gemm(xn, w.lm_head, out=out)           # fp32, unrounded: 140 us for 151936 x 4096 at 64 rows, 172 and a cast
+                row_gemm(xn, w.lm_head, out=out)
             else:
                 out = _mm(xn, w.lm_head).float()
         if m.allgather_logits is not None and m.layout.world > 1 and w.lm_head.n != cfg.vocab_size:

@@ -100,3 +100,10 @@ def test_pairs_one_by_one(aligned, kind, experts, d, inner, top, rows):
     up, down = _Weight(kind, 2 * inner, d, experts), _Weight(kind, d, inner, experts)
     up.scales = down.scales = torch.zeros(1, dtype=torch.bfloat16)
     assert tuple(r for r in range(1, 9) if narrow.pays_pairs(up, down, r, top)) == rows
+
+
+@pytest.mark.parametrize("kind,n,k,most", [(W_Q4, 151936, 4096, 160), (W_Q4, 32000, 2048, 160), (W_Q4, 50304, 1024, 160), (W_Q4, 65536, 512, 64),
+                                           (W_Q4, 8192, 2048, 64), (W_Q4, 2048, 1024, 64), (W_Q8, 151936, 4096, 0)])
+def test_logits_of_several_rows(kind, n, k, most):
+    from rmlx_b200.models.prefill import _logits_by_rows
+    assert max([r for r in range(200) if _logits_by_rows(_Weight(kind, n, k), r)], default=0) == most
