@@ -172,7 +172,7 @@ static int launch_rope_kv(const void* qkv, void* q_out, void* k_cache, void* v_c
   // 8 tokens, 2.2 / 5.4 for 64), but whole steps gain nothing by it (8 rows 868 us / 857, 64 rows 1816 / 1809).
   if (tokens >= 128 && HD % 16 == 0 && HD <= 512 && all % 16 == 0) {
     kern = rope_kv_write_pieces_kernel<T>;
-    threads = 256;
+    threads = H * (HD / 16) < 256 ? (H * (HD / 16) + 31) / 32 * 32 : 256;        // no warps without a head (2048 tokens of 3 heads of 64: 6.4 us with)
     const int heads = threads / (HD / 16) * 3;
     gy = (H + heads - 1) / heads;
   }

@@ -101,3 +101,26 @@ def test_argmax_slices(dev, rows, v):
     torch.manual_seed(v)
     logits = torch.randint(0, 200, (rows, v), device=dev).float()
     assert D.argmax(logits).tolist() == [int((r == r.max()).nonzero()[0]) for r in logits.cpu()]
+
+
+@pytest.mark.parametrize("hq,hkv,hd", [(1, 1, 64), (1, 1, 512), (26, 3, 128), (27, 3, 128), (60, 4, 128)])
+def test_rotation_of_few_and_many_heads(dev, hq, hkv, hd):
+    """130 tokens in pieces, by blocks as wide as their heads need, against the same tokens in two halves, one pair at a time; both round
+    once to bf16."""
+    torch.manual_seed(hd + hq)
+    tokens, page, heads = 130, 16, hq + 2 * hkv
+    qkv = torch.randn(tokens, heads * hd, device=dev).to(torch.bfloat16)
+    pos = torch.arange(tokens, dtype=torch.int32, device=dev)
+    ang = torch.randn(tokens, hd // 2, device=dev)
+    table = torch.arange(9, dtype=torch.int32, device=dev).view(1, -1)
+    res = []
+    for parts in ((slice(0, 130),), (slice(0, 65), slice(65, 130))):
+        q = torch.zeros(tokens, hq, hd, dtype=torch.bfloat16, device=dev)
+        kc, vc = (torch.zeros(9, hkv, page, hd, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        for s in parts:
+            D.rope_kv_write(qkv[s], q[s], kc, vc, table, pos[s], ang.cos(), ang.sin(), hq, hkv, token_seq=torch.zeros_like(pos[s]))
+        res.append((q, kc, vc))
+    size = float(qkv.abs().max())
+    for a, b in zip(*res):
+        assert ((a.double() - b.double()).abs() <= b.double().abs() * 2.0 ** -7 + size * 1e-6).all()
+    assert torch.equal(res[0][2], res[1][2]) and res[0][0].any()
