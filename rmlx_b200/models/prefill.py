@@ -34,7 +34,7 @@ from ..ops import grouped
 from ..ops.grouped import moe_prefill_ffn
 from ..ops.quantized import pair_pays, qmm, row_gemm, row_supported, row_tables_ready, tiles_route, xgemm
 from ..ops.weights import LinearWeight, W_BF16, W_Q4, W_Q8
-from .prefill_plan import PIECES, PrefillPlan, prompt_block
+from .prefill_plan import PrefillPlan, prompt_offsets
 
 
 def _narrow(x: torch.Tensor, w: LinearWeight) -> bool:
@@ -212,6 +212,7 @@ class PromptRun:
 
     def __init__(self, model):
         self.m = model
+        self._words: tuple = ()             # 64-bit words of the native call's two records
         self._numbers: list = []            # int32 0, 1, 2, ... and zeros on the device; grown ones are kept beside their successors
         if model.layout.world == 1 and model.device.type == "cuda":
             self._tables(model.cfg.max_seq_len + 1)     # here, not in the first portion that needs them
@@ -276,7 +277,8 @@ class PromptRun:
         mid = act = dense = xs = y = pairs = most = 0
         for li, lw in enumerate(mw.layers):
             n1, n2, kc, vc = lw.norm1, lw.norm2, cache.k[li], cache.v[li]
-            if n1.dtype != bf16 or n2.dtype != bf16 or (n1.data_ptr() | n2.data_ptr()) % 16 or not n1.is_contiguous() or not n2.is_contiguous() \
+            p1, p2 = n1.data_ptr(), n2.data_ptr()
+            if n1.dtype != bf16 or n2.dtype != bf16 or (p1 | p2) % 16 or not n1.is_contiguous() or not n2.is_contiguous() \
                     or not kc.is_contiguous() or not vc.is_contiguous() or kc.shape != vc.shape or kc.shape[3] != hd or \
                     not (n1.is_cuda and n2.is_cuda and kc.is_cuda and vc.is_cuda):
                 return None
@@ -308,13 +310,15 @@ class PromptRun:
             r_qkv, r_out = self._normed(lw.wqkv, t, n1), self._plain(lw.wo, t)
             if not (r_qkv and r_out and r_up and r_down):
                 return None
-            recs.extend((n1.data_ptr(), n2.data_ptr(), kc.data_ptr(), vc.data_ptr(), cache.k_sb[li].data_ptr() if q8 else 0,
+            recs.extend((p1, p2, kc.data_ptr(), vc.data_ptr(), cache.k_sb[li].data_ptr() if q8 else 0,
                          cache.v_sb[li].data_ptr() if q8 else 0, 0 if not e else lw.router.data_ptr(),
                          0 if not e or bias is None else bias.data_ptr(), e, k))
             for w, route in ((lw.wqkv, r_qkv), (lw.wo, r_out), (up, r_up), (down, r_down)):
                 s, b = w.scales, w.biases
-                if not w.w.is_cuda or (s is not None and not (s.is_cuda and b.is_cuda and s.is_contiguous() and b.is_contiguous() and
-                                                              w.w.is_contiguous())):
+                if not w.w.is_cuda or (s is not None and not (s.is_cuda and b.is_cuda)):
+                    return None
+                # a weight of the weight-streaming kernel has been looked at for it (narrow.supported)
+                if route & 15 != self.NARROW and s is not None and not (s.is_contiguous() and b.is_contiguous() and w.w.is_contiguous()):
                     return None
                 if route & 15 == self.EXPAND:
                     dense = max(dense, w.n * w.k * 2)
@@ -322,23 +326,25 @@ class PromptRun:
                              w.experts if e else 0, w.kind, int(s is not None and w.scales_f16), route))
         few = few_rows_plan(t, hq, hkv, hd, pos0 + t, q8)
         kv_bytes = pages * hkv * 16 * hd * 2 if q8 and not few else 0
-        where, size = prompt_block(dict(
-            h0=t * d * 2, h1=t * d * 2, xn=t * d * 2, qkv=t * (hq + 2 * hkv) * hd * 2, q=t * hq * hd * 2, attn=t * hq * hd * 2, act=act, mid=mid,
-            dense=dense, kk=kv_bytes, vv=kv_bytes, logits=t * most * 4, idx=pairs * 4, wts=pairs * 4, counts=most * 4,
-            offsets=(most + 1) * 4 if most else 0, order=pairs * 4, cursors=most * 4, row_of=pairs * 4, xs=xs, y=y))
+        rows, heads, routes = t * d * 2, t * hq * hd * 2, pairs * 4
+        offsets, size = prompt_offsets((                   # prefill_plan.PIECES
+            rows, rows, rows, t * (hq + 2 * hkv) * hd * 2, heads, heads, act, mid, dense, kv_bytes, kv_bytes, t * most * 4, routes, routes, most * 4,
+            (most + 1) * 4 if most else 0, routes, most * 4, routes, xs, y))
         ws = torch.empty(size, dtype=torch.uint8, device=m.device)
         base = ws.data_ptr()
         iota, zeros = self._tables(pos0 + t + 1)
         window = int(cfg.sliding_window or 0)
         head = array.array("q", (
             len(mw.layers), t, d, hq, hkv, hd, pos0, window, row.numel(), 16, cache.k[0].shape[0], int(cfg.rope_traditional),
-            int(prefill_kernel_choice(hd, window) == "tc"), int(os.environ.get("RMLX_FLASH_PREFILL_LANES", "0")), pages, few, mw.embed.shape[0],
+            int(not few and prefill_kernel_choice(hd, window) == "tc"), int(os.environ.get("RMLX_FLASH_PREFILL_LANES", "0")), pages, few, mw.embed.shape[0],
             mw.embed.data_ptr(), token_ids.data_ptr(), row.data_ptr(), iota.data_ptr() + 4 * pos0, zeros.data_ptr(), iota.data_ptr(),
-            m.cos.data_ptr(), m.sin.data_ptr(), GemmStatus.get(m.device).data_ptr(), *(base + where[name] for name in PIECES)))
+            m.cos.data_ptr(), m.sin.data_ptr(), GemmStatus.get(m.device).data_ptr(), *[base + o for o in offsets]))
         lib = _lib.cuda()
-        words = (ctypes.c_int * 2)()
-        lib.rmlx_prompt_sizes(words)
-        assert tuple(words) == (len(head), len(recs) // len(mw.layers)), "the records of csrc/runtime/prompt_run.cu"
+        if not self._words:
+            words = (ctypes.c_int * 2)()
+            lib.rmlx_prompt_sizes(words)
+            self._words = tuple(words)
+        assert self._words == (len(head), len(recs) // len(mw.layers)), "the records of csrc/runtime/prompt_run.cu"
         launches, what = ctypes.c_int(0), ctypes.c_char_p()
         rc = lib.rmlx_prompt_run(head.buffer_info()[0], recs.buffer_info()[0], cfg.rms_norm_eps, m.scale, ctypes.byref(launches),
                                  ctypes.byref(what), _lib.stream_ptr())

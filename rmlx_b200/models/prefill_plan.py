@@ -2,7 +2,7 @@
 
 ``PrefillPlan`` lists, for a sequence length, the launches of one layer with their shapes and the
 scratch each needs (the reference builds the same per-length ``PlanStep`` lists,
-crates/rmlx-nn/src/prefill_plan.rs:16-300); ``prompt_block`` lays that scratch out in one block, for the plan and for
+crates/rmlx-nn/src/prefill_plan.rs:16-300); ``prompt_offsets`` lays that scratch out in one block, for the plan and for
 the portion that runs alike; ``PrefillPool`` keeps a few slots of pre-allocated
 intermediates sized for the largest planned length so that chunks of a prompt do not allocate
 (crates/rmlx-nn/src/prefill_pool.rs:33-160, crates/rmlx-nn/src/dynamic.rs:16-104).
@@ -10,7 +10,7 @@ intermediates sized for the largest planned length so that chunks of a prompt do
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Dict, List, Optional, Tuple
+from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
@@ -35,30 +35,43 @@ class PlanStep:
 #: The pieces of a portion's work space, in the order of the native call's record (csrc/runtime/prompt_run.cu).
 PIECES = ("h0", "h1", "xn", "qkv", "q", "attn", "act", "mid", "dense", "kk", "vv", "logits", "idx", "wts", "counts", "offsets", "order",
           "cursors", "row_of", "xs", "y")
-# The residual stream, a weight expanded for one product and the routing's tables have places of their own. The rest belongs to one
-# half of a layer and is dead in the other, so the halves share their memory; and within a half a piece lies where one was
-# that has been read by then (queries on the normed rows, the heads' results on qkv, ...).
-_OWN = ("h0", "h1", "dense", "idx", "wts", "counts", "offsets", "order", "cursors", "row_of")
-_HALVES = ((("xn", "q"), ("qkv", "attn"), ("kk",), ("vv",)), (("xn",), ("logits", "act"), ("mid", "xs", "y")))
+
+
+def prompt_offsets(sizes: Sequence[int]) -> Tuple[List[int], int]:
+    """Where the pieces of a portion's work space lie in one block (bytes from its start, 256-byte addresses, in the order of ``PIECES``), and
+    the block's size. ``sizes``: bytes of each piece. A launch writes only after the one before it has finished, so what no later
+    launch reads is free.
+
+    The residual stream, a weight expanded for one product and the routing's tables have places of their own. The rest belongs to one
+    half of a layer and is dead in the other, so the halves share their memory; and within a half a piece lies where one was
+    that has been read by then (queries on the normed rows, the heads' results on qkv, ...). Written out: a portion of a few rows waits for
+    this (3 us, 8 by names)."""
+    h0, h1, xn, qkv, q, attn, act, mid, dense, kk, vv, logits, idx, wts, counts, offsets, order, cursors, row_of, xs, y = \
+        [s + 255 & ~255 for s in sizes]
+    at_dense = h0 + h1
+    at_idx = at_dense + dense
+    at_wts = at_idx + idx
+    at_counts = at_wts + wts
+    at_offsets = at_counts + counts
+    at_order = at_offsets + offsets
+    at_cursors = at_order + order
+    at_row_of = at_cursors + cursors
+    shared = at_row_of + row_of
+    # attention: normed rows, then queries; qkv, then the heads' results; expanded pages
+    at_qkv = shared + (xn if xn > q else q)
+    at_kk = at_qkv + (qkv if qkv > attn else attn)
+    at_vv = at_kk + kk
+    # feed-forward: normed rows; logits, then the gated rows; both halves of the gate, sorted rows or the experts' results
+    at_act = shared + xn
+    at_mid = at_act + (logits if logits > act else act)
+    return [0, h0, shared, at_qkv, shared, at_qkv, at_act, at_mid, at_dense, at_kk, at_vv, at_act, at_idx, at_wts, at_counts, at_offsets, at_order,
+            at_cursors, at_row_of, at_mid, at_mid], max(at_vv + vv, at_mid + max(mid, xs, y))
 
 
 def prompt_block(sizes: Dict[str, int]) -> Tuple[Dict[str, int], int]:
-    """Where the pieces of a portion's work space lie in one block (bytes from its start, 256-byte addresses), and the block's size.
-    ``sizes``: bytes of each piece of ``PIECES``; those that are left out are empty. A launch writes only after the one before it has
-    finished, so what no later launch reads is free."""
-    size = {name: (sizes.get(name, 0) + 255) & ~255 for name in PIECES}
-    at, start = {}, 0
-    for name in _OWN:
-        at[name] = start
-        start += size[name]
-    total = start
-    for half in _HALVES:
-        end = start
-        for slot in half:
-            at.update((name, end) for name in slot)
-            end += max(size[name] for name in slot)
-        total = max(total, end)
-    return at, total
+    """``prompt_offsets`` by name; pieces that are left out are empty."""
+    at, total = prompt_offsets([sizes.get(name, 0) for name in PIECES])
+    return dict(zip(PIECES, at)), total
 
 
 class PrefillPlan:

@@ -45,7 +45,7 @@ def few_rows_plan(t: int, hq: int, hkv: int, head_dim: int, tokens: int, q8: boo
     if head_dim == 64 and tokens <= 128 and not q8:
         return 0
     tiles = t * hkv * _lib.cuda().rmlx_flash_decode_gtiles(hq, hkv)
-    return decode.cluster_plan(t, hq, hkv, head_dim, tokens, q8) if decode.clusters_pay(tiles, head_dim, tokens, q8) else 0
+    return decode.cluster_plan(t, hq, hkv, head_dim, tokens, q8, tiles) if decode.clusters_pay(tiles, head_dim, tokens, q8) else 0
 
 
 def few_rows_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_row: torch.Tensor, lens: torch.Tensor, plan: int,

@@ -423,10 +423,11 @@ _lib.register_cuda_sigs({
 _FD_CLUSTER = os.environ.get("RMLX_FLASH_DECODE_CLUSTER", "1") != "0"
 
 
-def cluster_plan(batch: int, hq: int, hkv: int, head_dim: int, max_len: int, q8: bool) -> int:
-    """(cluster size << 16) | clusters of csrc/kernels/flash_decode_cluster.cu for up to ``max_len`` tokens; 0: not a shape of it."""
+def cluster_plan(batch: int, hq: int, hkv: int, head_dim: int, max_len: int, q8: bool, tiles: int = 0) -> int:
+    """(cluster size << 16) | clusters of csrc/kernels/flash_decode_cluster.cu for up to ``max_len`` tokens (``tiles``: of the batch, if
+    known); 0: not a shape of it."""
     lib = _lib.cuda()
-    tiles = batch * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv)
+    tiles = tiles or batch * hkv * lib.rmlx_flash_decode_gtiles(hq, hkv)
     plan = int(lib.rmlx_flash_decode_cluster_plan(batch, tiles, int(max_len), head_dim, int(q8)))
     # Sixteen blocks merge a tile's heads into so many parts that with more than eight heads, and more than four tiles, it takes what it
     # gives: 64 and 4 heads, two sequences, us for 8 / 16 blocks: 7.0 / 9.8 at 17 tokens, 6.8 / 8.3 at 400, 9.1 / 9.5 at 2000, 16.8 / 14.3 at 8000
