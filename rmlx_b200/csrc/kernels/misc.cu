@@ -125,7 +125,8 @@ rms_norm_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
 // slice to one 64-bit key (order-preserving float bits, then inverted index), merges it with
 // atomicMax, and the last block of a row decodes the winner and clears the scratch for the next
 // launch. keys[rows] and tickets[rows] must be zero on first use. A thread requests four pieces of 16 bytes at a time where rows
-// start at 16-byte addresses and are not short (64 rows of 151936: 6.6 us, 17.8 one value at a time; 256 values 3.8, 3.5 one at a time).
+// start at 16-byte addresses (64 rows of 151936: 6.6 us, 17.8 one value at a time; 1024 values by themselves 3.8, 3.7 one at a time, but a whole
+// step of a small model 34.4, 36.1 one at a time).
 template <bool WIDE>
 __global__ void __launch_bounds__(1024)
 argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int V, int stride,
@@ -305,7 +306,7 @@ extern "C" int rmlx_argmax(const float* logits, int* out, int B, int V, int stri
   if (slices > 64) slices = 64;
   const int fill = B < sm_count() ? sm_count() / B : 1;
   if (slices > fill) slices = fill;
-  const bool wide = V >= 2048 && stride % 4 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0;
+  const bool wide = stride % 4 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0;
   return launch(wide ? argmax_kernel<true> : argmax_kernel<false>, dim3(slices, B), dim3(1024), 0, st, pdl != 0, logits, out, V, stride, keys,
                 tickets);
 }

@@ -97,7 +97,7 @@ def test_argmax(dev, rows, v, odd):
 
 @pytest.mark.parametrize("rows,v", [(1, 2044), (1, 2048), (2, 2052), (74, 20000), (75, 20000), (148, 9001), (149, 12288)])
 def test_argmax_slices(dev, rows, v):
-    """Short rows one value at a time, and rows in as many slices as there are SMs for each."""
+    """Short rows, and rows in as many slices as there are SMs for each."""
     torch.manual_seed(v)
     logits = torch.randint(0, 200, (rows, v), device=dev).float()
     assert D.argmax(logits).tolist() == [int((r == r.max()).nonzero()[0]) for r in logits.cpu()]
